@@ -39,6 +39,7 @@ struct Entry {
   DMNode* d_wnodes = nullptr;     // Mbvh: the same tree, exact nodes
   DTBox* d_tboxes = nullptr;      // Mbvh with q_gates: subtree boxes of d_mnodes (from the triangles)
   uint32_t wcount = 0;
+  bool quads_cover = false;       // Mbvh: every quad slot box contains its triangles grown by 1e-4
   bool q_gates = false;           // Mbvh: escaped triangles are flagged (collapse_entry)
   uint32_t* d_indices = nullptr;
   float4* d_tris = nullptr;       // 3 per index slot
@@ -59,6 +60,7 @@ struct Entry {
     d_tboxes = nullptr;
     wcount = 0;
     q_gates = false;
+    quads_cover = false;
     d_indices = nullptr;
     d_tris = nullptr;
     d_vertices = nullptr;
@@ -119,6 +121,7 @@ ResultCode collapse_entry(Entry& m, cudaStream_t s, DMNode** mnodes, uint32_t* m
   m.d_tboxes = nullptr;
   m.wcount = 0;
   m.q_gates = false;
+  m.quads_cover = false;
   if (m.bvh_node_count == 0) {  // Mbvh::default()
     *mnodes = nullptr;
     *mcount = 0;
@@ -130,6 +133,7 @@ ResultCode collapse_entry(Entry& m, cudaStream_t s, DMNode** mnodes, uint32_t* m
   ResultCode rc;
   if (!tris || m.boxes_cover || m.build_type == 3) {
     if ((rc = build_mbvh(m.d_nodes, m.bvh_node_count, s, mnodes, mcount)) != Ok || !tris) return rc;
+    m.quads_cover = m.boxes_cover;
     return build_wide(m.d_nodes, m.bvh_node_count, check, m.prim_count, s, &m.d_wnodes, &m.d_qnodes, &m.wcount);
   }
   Scratch<DAabb> tb;
@@ -148,6 +152,7 @@ ResultCode collapse_entry(Entry& m, cudaStream_t s, DMNode** mnodes, uint32_t* m
   // boxes recomputed from the triangles nest by construction
   rc = build_wide(tb.ptr, m.bvh_node_count, check, m.prim_count, s, &m.d_wnodes, &m.d_qnodes, &m.wcount, true);
   m.q_gates = escaped != 0 && m.wcount != 0;
+  m.quads_cover = escaped == 0;
   if (!m.q_gates) {  // no ray is handed on for an escape: the subtree boxes would go unused
     pool_free(m.d_tboxes, s);
     m.d_tboxes = nullptr;
@@ -878,6 +883,7 @@ static ResultCode trace_common(uint32_t id, bool mbvh, const float* rays, const 
       a.q_count = e->wcount;
       a.q_gates = e->q_gates;
       a.tboxes = e->q_gates ? e->d_tboxes : nullptr;
+      a.quads_cover = e->quads_cover;
     }
     if (walk_stats && (a.qnodes == nullptr || a.q_count == 0)) return InvalidArgument;
     a.nodes = e->d_nodes;

@@ -211,6 +211,9 @@ struct TraceArgs {
   // over the rays the compact walk hands on also skips slots whose subtree
   // box the ray cannot enter below its current t.
   const DTBox* tboxes = nullptr;
+  // Every slot box of mnodes contains its triangles with the 1e-4 margin:
+  // any-hit walks skip slots wholly behind the ray's origin.
+  bool quads_cover = false;
   // Optional per-ray counts of the compact closest-hit walk (3 per ray:
   // traversal-tree node visits, triangle tests, 1 if handed to the exact walk).
   uint32_t* walk_stats = nullptr;

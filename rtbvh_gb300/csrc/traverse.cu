@@ -109,9 +109,12 @@ __device__ __forceinline__ bool mt_test(const float4* tri, RayState& r, float& h
 // return the same value; at most the sign of a zero differs, which no later
 // comparison can see. So the fast form takes every decision the exact form
 // takes. Rays with a zero or non-finite component use the exact form.
-template <bool FAST>
+//
+// BEHIND (FAST only): slots whose exit t is below exit_min are left out of
+// the mask (0: boxes wholly behind the origin; -inf: none).
+template <bool FAST, bool BEHIND = false>
 __device__ __forceinline__ void quad_intersect(const DMNode* node, const RayState& r, uint32_t& mask, uint32_t& ids,
-                                               int4& children, int4& counts) {
+                                               int4& children, int4& counts, float exit_min = 0.0f) {
   const float* q = reinterpret_cast<const float*>(node);
   float vx[8], vy[8], vz[8], vc[8];
   ld8(q, vx);
@@ -146,7 +149,7 @@ __device__ __forceinline__ void quad_intersect(const DMNode* node, const RayStat
       tx = sse_min(txx, sse_min(tyx, tzx));
     }
     tmin[i] = tn;
-    if ((tx >= tn) && (tn < r.t)) m |= 1u << i;
+    if ((tx >= tn) && (tn < r.t) && (!BEHIND || tx >= exit_min)) m |= 1u << i;
   }
   uint32_t i0 = 0, i1 = 1, i2 = 2, i3 = 3;
   float t0 = tmin[0], t1 = tmin[1], t2 = tmin[2], t3 = tmin[3], tt;
@@ -271,13 +274,21 @@ __device__ __forceinline__ uint32_t subtree_mask(const DTBox* box, const RayStat
 // node/triangle order is the reference's. With ray_count_dev the number of
 // rays is read from the device (the rays the compact kernel deferred).
 //
-// TCULL (closest hit over a binned-SAH tree's quad nodes with a.tboxes):
-// a slot whose subtree box (from the triangles) the ray cannot enter below
-// its current t is skipped. The reference would walk that subtree and
-// accept no hit in it (every triangle lies inside the subtree box), so t
-// and the order of all later tests are unchanged: the hit is the
-// reference's bit for bit (the node counts are not, so STATS never culls).
-template <bool ANY_HIT, bool STATS, bool TCULL = false>
+// CULL: slots that cannot hold a hit are skipped; the reference would walk
+// their subtrees and accept nothing in them, so t and the order of all later
+// tests are unchanged and the hit is the reference's bit for bit (the node
+// counts are not, so STATS never culls).
+//  kCullSubtree (binned-SAH trees with a.tboxes): slots whose subtree box
+//   (from the triangles) the ray cannot enter below its current t.
+//  kCullBehind (any hit over a tree whose slot boxes contain their triangles
+//   with the 1e-4 margin, a.quads_cover): slots wholly behind the origin, by
+//   the exit t the slab test has anyway. What bounds such a walk is the
+//   number of boxes visited: the slab test has no lower bound on t, so a
+//   shadow ray that leaves a surface walks the whole scene behind it too.
+//   4.2M shadow rays over 1M clustered triangles: 10.74 ms without the skip,
+//   3.80 ms with it.
+constexpr int kCullNone = 0, kCullSubtree = 1, kCullBehind = 2;
+template <bool ANY_HIT, bool STATS, int CULL = kCullNone>
 __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int* work) {
   RayState ray;
   float hu = 0.0f, hv = 0.0f;
@@ -305,16 +316,23 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int
     r = a.order ? __ldg(a.order + rr) : rr;
     ray = load_ray(a.rays, r, a.t_max);
     fast = finite_ray(ray);
-    if (TCULL && a.node_count > 0) {
-      // |x| <= bound is false for NaN and infinities. Only rays that start
-      // inside the scene's root box: boxes behind them are most of what the
-      // cull saves; for rays from outside it costs more than it saves
+    if (CULL != kCullNone && a.node_count > 0) {
       const DAabb root = load_aabb(a.nodes);
+      // |x| <= bound is false for NaN and infinities
       cull = fabsf(ray.ox) <= kCompactRange && fabsf(ray.oy) <= kCompactRange && fabsf(ray.oz) <= kCompactRange &&
              fabsf(ray.dx) <= 3.0e38f && fabsf(ray.dy) <= 3.0e38f && fabsf(ray.dz) <= 3.0e38f &&
-             fabsf(ray.ix) <= kQuantRange && fabsf(ray.iy) <= kQuantRange && fabsf(ray.iz) <= kQuantRange &&
-             ray.ox >= root.min[0] && ray.oy >= root.min[1] && ray.oz >= root.min[2] && ray.ox <= root.max[0] &&
-             ray.oy <= root.max[1] && ray.oz <= root.max[2];
+             fabsf(ray.ix) <= kQuantRange && fabsf(ray.iy) <= kQuantRange && fabsf(ray.iz) <= kQuantRange;
+      if (CULL == kCullSubtree) {
+        // Only rays that start inside the scene's root box: boxes behind
+        // them are most of what the cull saves; for rays from outside the
+        // extra box loads cost more than they save
+        cull = cull && ray.ox >= root.min[0] && ray.oy >= root.min[1] && ray.oz >= root.min[2] &&
+               ray.ox <= root.max[0] && ray.oy <= root.max[1] && ray.oz <= root.max[2];
+      } else {
+        // the margin argument needs the boxes within the range too
+        for (int k = 0; k < 3; ++k)
+          cull = cull && root.min[k] >= -kCompactRange && root.max[k] <= kCompactRange;
+      }
     }
     hu = hv = 0.0f;
     prim = -1;
@@ -364,9 +382,11 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int
     uint32_t mask, ids;
     int4 children, counts;
     bool done = false;
-    if (fast) quad_intersect<true>(a.mnodes + current, ray, mask, ids, children, counts);
+    if (fast)
+      quad_intersect<true, CULL == kCullBehind>(a.mnodes + current, ray, mask, ids, children, counts,
+                                                cull ? 0.0f : -__int_as_float(0x7f800000));
     else quad_intersect<false>(a.mnodes + current, ray, mask, ids, children, counts);
-    if (TCULL && cull) mask &= subtree_mask(a.tboxes + current, ray);
+    if (CULL == kCullSubtree && cull) mask &= subtree_mask(a.tboxes + current, ray);
     if (STATS) ++visits;
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
@@ -1060,7 +1080,7 @@ cudaError_t launch_compact(const TraceArgs& a, cudaStream_t s, unsigned int* cou
   // deferred)
   b.ray_batch = 32;
   if (b.tboxes) {
-    auto cull_kern = k_trace_mbvh<false, false, true>;
+    auto cull_kern = k_trace_mbvh<false, false, kCullSubtree>;
     cull_kern<<<persistent_grid(cull_kern, b), kBlock, 0, s>>>(b, counters + 2);
     return cudaGetLastError();
   }
@@ -1100,7 +1120,11 @@ cudaError_t launch_any(const TraceArgs& a0, cudaStream_t s) {
     a.order = order.ptr;
   }
   const bool st = a.stats != nullptr;
-  if (a.any_hit) e = st ? launch3<MBVH, true, true>(a, s, work.ptr) : launch3<MBVH, true, false>(a, s, work.ptr);
+  if (a.any_hit && MBVH && !st && (a.quads_cover || a.tboxes)) {
+    auto kern = a.quads_cover ? k_trace_mbvh<true, false, kCullBehind> : k_trace_mbvh<true, false, kCullSubtree>;
+    kern<<<persistent_grid(kern, a), kBlock, 0, s>>>(a, work.ptr);
+    e = cudaGetLastError();
+  } else if (a.any_hit) e = st ? launch3<MBVH, true, true>(a, s, work.ptr) : launch3<MBVH, true, false>(a, s, work.ptr);
   else if (st) e = launch3<MBVH, false, true>(a, s, work.ptr);
   else if (MBVH && a.qnodes && a.q_count > 0) {
     if ((e = deferred.alloc(a.ray_count, s))) return e;
