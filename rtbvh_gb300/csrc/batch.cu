@@ -8,11 +8,10 @@
 //      every mesh's own MortonEncoder::get_sorted_indices order;
 //   3. the clustering levels (locb.cu): a thread-block cluster per large
 //      mesh, one block per small mesh, the two sets concurrently;
-//   4. parent pointers and quad-subtree counts over the whole forest, then
-//      one block per mesh for the top-down MBVH collapse (mbvh.cu);
-//   5. leaf-ordered triangles, per-mesh closest-hit traversal trees (one
-//      block per mesh, see build_wide) and ONE persistent traversal launch
-//      for all rays, each ray starting at its mesh's root.
+//   4. the MBVH collapse and the closest-hit traversal trees of the whole
+//      forest, one thread per node (mbvh.cu);
+//   5. leaf-ordered triangles and ONE persistent traversal launch for all
+//      rays, each ray starting at its mesh's root.
 // Every buffer is allocated when the plan is created, and the whole
 // pipeline is captured in a CUDA graph that rtbvh_gpu_batch_run replays.
 // Per mesh, the result equals the single-mesh build's, with node, leaf and
@@ -141,13 +140,12 @@ struct Plan {
   const float* t_max = nullptr;
   float* hits = nullptr;
   uint32_t flags = 0;
-  DevBuf<uint32_t> prim_off, ray_off, order, keys, vals, nb, parent, arrive, cnt_e, cnt_o, mbase, status, sort_tmp_u;
+  DevBuf<uint32_t> prim_off, ray_off, order, keys, vals, nb, collapse_words, mbase, qroot, status, sort_tmp_u;
   DevBuf<DAabb> aabbs, worlds, lvl0, lvl1, nodes;
   DevBuf<float4> centers, tris;
   DevBuf<DMNode> mnodes;
-  DevBuf<DMNode> wnodes;  // per-mesh closest-hit traversal trees (exact), mesh m at [off_m, off_m + n_m)
+  DevBuf<DMNode> wnodes;  // the meshes' closest-hit traversal trees (exact), mesh m's root at qroot[m]
   DevBuf<DQNode> qnodes;  // the same, compact
-  DevBuf<uint2> q0, q1;
   DevBuf<char> sort_temp;
   size_t sort_bytes = 0;
   // meshes order[0, big_count) get a thread-block cluster each (locb.cu)
@@ -209,16 +207,13 @@ cudaError_t run_build(Plan& p, cudaStream_t s) {
                                 p.lvl0.ptr, p.lvl1.ptr, p.nodes.ptr, p.nb.ptr, p.status.ptr, mesh_blocks(M),
                                 p.big_count, p.cluster_sums.ptr, p.clusters, s, p.side, p.fork, p.join)))
     return e;
-  if ((e = launch_collapse_segments(p.nodes.ptr, p.node_cap, p.prim_off.ptr, p.order.ptr, M, p.parent.ptr,
-                                    p.arrive.ptr, p.cnt_e.ptr, p.cnt_o.ptr, p.mbase.ptr, p.q0.ptr, p.q1.ptr,
-                                    p.mnodes.ptr, p.node_cap, p.status.ptr, mesh_blocks(M), s)))
+  // traversal trees for the closest hit only (LOCB trees are nested)
+  const bool wide = !(p.flags & (RTBVH_TRACE_ANY_HIT | RTBVH_TRACE_EXACT_NODES));
+  if ((e = launch_collapse_forest(p.nodes.ptr, p.node_cap, p.prim_off.ptr, M, N, p.collapse_words.ptr, p.mbase.ptr,
+                                  p.mnodes.ptr, wide ? p.wnodes.ptr : nullptr, wide ? p.qnodes.ptr : nullptr,
+                                  p.qroot.ptr, p.status.ptr + 2, p.status.ptr, s)))
     return e;
   if ((e = launch_gather_triangles(p.vertices, p.vals.ptr, N, p.tris.ptr, s))) return e;
-  // closest-hit traversal trees (LOCB trees are nested, see build_wide)
-  if (!(p.flags & (RTBVH_TRACE_ANY_HIT | RTBVH_TRACE_EXACT_NODES)) &&
-      (e = launch_wide_segments(p.nodes.ptr, p.node_cap, p.prim_off.ptr, p.order.ptr, M, N, p.wnodes.ptr,
-                                p.qnodes.ptr, p.q0.ptr, p.q1.ptr, p.status.ptr, mesh_blocks(M), s)))
-    return e;
   return cudaGetLastError();
 }
 
@@ -244,7 +239,7 @@ cudaError_t run_trace(Plan& p, cudaStream_t s) {
       a.qnodes = p.qnodes.ptr;
       a.qexact = p.wnodes.ptr;
       a.q_count = N;
-      a.seg_qroot = p.prim_off.ptr;  // mesh m's traversal tree starts at off_m
+      a.seg_qroot = p.qroot.ptr;
     }
     a.blocks_per_sm = p.trace_blocks_per_sm;
     a.ray_batch = p.trace_ray_batch;
@@ -362,13 +357,13 @@ ResultCode rtbvh_gpu_batch_create(const float* vertices, const uint32_t* prim_of
     return cuda_rc(e);
   if ((e = p->prim_off.alloc(mesh_count + 1)) || (e = p->ray_off.alloc(mesh_count + 1)) ||
       (e = p->order.alloc(mesh_count)) || (e = p->keys.alloc(N)) || (e = p->vals.alloc(N)) ||
-      (e = p->nb.alloc(p->node_cap)) || (e = p->parent.alloc(p->node_cap)) || (e = p->arrive.alloc(p->node_cap)) ||
-      (e = p->cnt_e.alloc(p->node_cap)) || (e = p->cnt_o.alloc(p->node_cap)) || (e = p->mbase.alloc(mesh_count + 1)) ||
+      (e = p->nb.alloc(p->node_cap)) || (e = p->collapse_words.alloc(collapse_scratch_words(p->node_cap))) ||
+      (e = p->mbase.alloc(mesh_count + 1)) || (e = p->qroot.alloc(mesh_count)) ||
       (e = p->status.alloc(4)) || (e = p->aabbs.alloc(N)) || (e = p->worlds.alloc(mesh_count)) ||
       (e = p->lvl0.alloc(p->node_cap)) || (e = p->lvl1.alloc(p->node_cap)) || (e = p->nodes.alloc(p->node_cap)) ||
       (e = p->centers.alloc(N)) || (e = p->tris.alloc((size_t)kTriFloat4 * N)) ||
-      (e = p->mnodes.alloc(p->node_cap)) || (e = p->qnodes.alloc(N)) || (e = p->wnodes.alloc(N)) || (e = p->q0.alloc(2 * (size_t)p->node_cap)) ||
-      (e = p->q1.alloc(2 * (size_t)p->node_cap)) || (e = p->sort_temp.alloc(p->sort_bytes)))
+      (e = p->mnodes.alloc(p->node_cap)) || (e = p->qnodes.alloc(N)) || (e = p->wnodes.alloc(N)) ||
+      (e = p->sort_temp.alloc(p->sort_bytes)))
     return cuda_rc(e);
   if ((e = cudaMemcpyAsync(p->prim_off.ptr, prim_offsets, 4 * (size_t)(mesh_count + 1), cudaMemcpyHostToDevice, s)) ||
       (e = cudaMemcpyAsync(p->ray_off.ptr, ray_offsets, 4 * (size_t)(mesh_count + 1), cudaMemcpyHostToDevice, s)) ||

@@ -90,7 +90,7 @@ uint32_t store(std::unique_ptr<Entry> e, bool mbvh) {
   return (uint32_t)(t.size() - 1);
 }
 
-// Indices for build_wide's leaf check: trees of the object-split builders
+// Indices for build_mbvh's leaf check: trees of the object-split builders
 // (LOCB, binned SAH) hold each primitive once by construction and skip it;
 // spatial-split trees and structures of unknown origin are checked.
 const uint32_t* leaf_check(uint32_t build_type, const uint32_t* indices) {
@@ -109,7 +109,7 @@ bool boxes_cover(uint32_t build_type) { return build_type == 1; }
 
 // The quad nodes (*mnodes, *mcount: Mbvh::construct) and the closest-hit
 // traversal tree of Mbvh entry m, from its own BVH2 nodes and triangles:
-// the plain traversal tree (build_wide over m's boxes) when the boxes
+// the plain traversal tree (over m's boxes) when the boxes
 // contain the triangles, else the tree over boxes recomputed from the
 // triangles with escape flags in m's triangle records (build_mbvh with
 // MbvhTriangles; object-split leaves only, spatial-split trees get none);
@@ -129,35 +129,40 @@ ResultCode collapse_entry(Entry& m, cudaStream_t s, DMNode** mnodes, uint32_t* m
   }
   if (!m.d_nodes) return Error;
   const bool tris = m.d_vertices && m.d_tris && !m.vertex_lower_bound;
-  const uint32_t* check = leaf_check(m.build_type, m.d_indices);
-  ResultCode rc;
-  if (!tris || m.boxes_cover || m.build_type == 3) {
-    if ((rc = build_mbvh(m.d_nodes, m.bvh_node_count, s, mnodes, mcount)) != Ok || !tris) return rc;
-    m.quads_cover = m.boxes_cover;
-    return build_wide(m.d_nodes, m.bvh_node_count, check, m.prim_count, s, &m.d_wnodes, &m.d_qnodes, &m.wcount);
-  }
+  MbvhRequest req;
+  MbvhOutput out;
+  req.wide = tris;
+  req.check_indices = leaf_check(m.build_type, m.d_indices);
+  req.index_count = m.prim_count;
   Scratch<DAabb> tb;
-  cudaError_t err;
-  if ((err = tb.alloc(m.bvh_node_count, s))) return cuda_rc(err);
   MbvhTriangles t;
-  t.indices = m.d_indices;
-  t.index_count = m.prim_count;
-  t.vertices = m.d_vertices;
-  t.vertex_count = m.vertex_count;
-  t.tris = m.d_tris;
-  t.tb = tb.ptr;
-  t.tboxes_out = &m.d_tboxes;
-  uint32_t escaped = 0;
-  if ((rc = build_mbvh(m.d_nodes, m.bvh_node_count, s, mnodes, mcount, &t, &escaped)) != Ok) return rc;
-  // boxes recomputed from the triangles nest by construction
-  rc = build_wide(tb.ptr, m.bvh_node_count, check, m.prim_count, s, &m.d_wnodes, &m.d_qnodes, &m.wcount, true);
-  m.q_gates = escaped != 0 && m.wcount != 0;
-  m.quads_cover = escaped == 0;
+  const bool from_triangles = tris && !m.boxes_cover && m.build_type != 3;
+  if (from_triangles) {
+    cudaError_t err;
+    if ((err = tb.alloc(m.bvh_node_count, s))) return cuda_rc(err);
+    t.indices = m.d_indices;
+    t.index_count = m.prim_count;
+    t.vertices = m.d_vertices;
+    t.vertex_count = m.vertex_count;
+    t.tris = m.d_tris;
+    t.tb = tb.ptr;
+    req.tri = &t;
+  }
+  const ResultCode rc = build_mbvh(m.d_nodes, m.bvh_node_count, s, req, &out);
+  if (rc != Ok) return rc;
+  *mnodes = out.mnodes;
+  *mcount = out.mcount;
+  m.d_wnodes = out.wnodes;
+  m.d_qnodes = out.wq;
+  m.wcount = out.wcount;
+  m.d_tboxes = out.tboxes;
+  m.quads_cover = tris && (from_triangles ? out.escaped == 0 : m.boxes_cover);
+  m.q_gates = out.escaped != 0 && m.wcount != 0;
   if (!m.q_gates) {  // no ray is handed on for an escape: the subtree boxes would go unused
     pool_free(m.d_tboxes, s);
     m.d_tboxes = nullptr;
   }
-  return rc;
+  return Ok;
 }
 
 cudaStream_t legacy_stream() {
@@ -1491,7 +1496,10 @@ ResultCode rtbvh_deserialize_mbvh(const uint8_t* buffer, uintptr_t size, uint32_
   ResultCode rc = upload_entry(*e, hn.data(), nn, hi.data(), ni, s);
   // the quad nodes must be the collapse of the BVH2 nodes (Mbvh::construct):
   // collapse again on the device and compare bit for bit
-  if (rc == Ok) rc = build_mbvh(e->d_nodes, e->bvh_node_count, s, &e->d_mnodes, &e->node_count);
+  MbvhOutput collapsed;
+  if (rc == Ok) rc = build_mbvh(e->d_nodes, e->bvh_node_count, s, MbvhRequest(), &collapsed);
+  e->d_mnodes = collapsed.mnodes;
+  e->node_count = collapsed.mcount;
   if (rc == Ok) {
     std::vector<DMNode> check;
     if ((rc = fetch_device(check, e->d_mnodes, e->node_count)) == Ok &&

@@ -109,9 +109,7 @@ ResultCode build_spatial_sah(const DAabb* aabbs, const float4* centers, const fl
 // `indices` (index_count slots), which index `vertices` (vertex_count
 // triangles, 9 floats each); `tris` are the leaf-ordered triangle records
 // (kTriFloat4 float4 per index slot) whose flags word gets kTriEscape or 0;
-// `tb` (node_count entries) receives the traversal boxes; with
-// `tboxes_out`, build_mbvh also allocates the quad nodes' subtree boxes
-// (DTBox per quad node, from `tb`) and stores them there.
+// `tb` (node_count entries) receives the traversal boxes.
 struct MbvhTriangles {
   const uint32_t* indices = nullptr;
   uint32_t index_count = 0;
@@ -119,39 +117,41 @@ struct MbvhTriangles {
   uint32_t vertex_count = 0;
   float4* tris = nullptr;
   DAabb* tb = nullptr;
-  DTBox** tboxes_out = nullptr;
 };
-// Mbvh::construct (src/bvh.rs:381-404). mnodes is allocated here. With
-// `tri` (for BVH2s whose boxes need not contain these triangles: binned-SAH
-// builds, whose left boxes can miss primitives, src/builders/
-// binned_sah.rs:236-256; triangles attached after a build) the same passes
-// also compute every node's box from the triangles into tri->tb (leaf:
-// vertex boxes grown by 1e-4; interior: union of the children) and flag the
-// escaped triangles: those whose grown vertex box does not lie inside every
-// slot box the quad nodes test on the way to them. *escaped receives their
-// number.
-ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, DMNode** mnodes,
-                      uint32_t* mnode_count, const MbvhTriangles* tri = nullptr, uint32_t* escaped = nullptr);
-// The closest-hit traversal tree: a 4-wide collapse of the BVH2 with tight
-// slot boxes (largest-area child opened first), as exact nodes and compact
-// copies; *wcount nodes, root 0. No tree (*wcount 0, Ok) when a node's box
-// does not contain its children's (checked unless `nested` is known), or
-// (indices given) when the leaves do not hold each of the index_count slots
-// and each primitive exactly once -- spatial-split trees, whose leaf boxes
-// bound fragments -- closest hit then reads the exact nodes in the
-// reference's order.
-ResultCode build_wide(const DAabb* nodes, uint32_t node_count, const uint32_t* indices, uint32_t index_count,
-                      cudaStream_t s, DMNode** wnodes, DQNode** wq, uint32_t* wcount, bool nested = false);
-// Traversal trees of a concatenated forest (LOCB meshes): mesh m's tree in
-// nodes [off_m, off_m + n_m) of wnodes (exact) and wq (compact), root off_m;
-// q0/q1 hold total_prims entries each.
-cudaError_t launch_wide_segments(const DAabb* nodes, uint32_t node_count, const uint32_t* prim_off,
-                                 const uint32_t* order, uint32_t mesh_count, uint32_t total_prims, DMNode* wnodes,
-                                 DQNode* wq, uint2* q0, uint2* q1, uint32_t* status, unsigned blocks, cudaStream_t s);
-// Compact (64-byte) copies of quad nodes for the closest-hit traversal;
-// with live_count (device) only the first *live_count of `count` nodes.
-cudaError_t launch_quantize_mbvh(const DMNode* mnodes, uint32_t count, DQNode* qnodes, cudaStream_t s,
-                                 const uint32_t* live_count = nullptr);
+// What build_mbvh makes. `tri` (for BVH2s whose boxes need not contain these
+// triangles: binned-SAH builds, whose left boxes can miss primitives,
+// src/builders/binned_sah.rs:236-256; triangles attached after a build): the
+// same passes also compute every node's box from the triangles into tri->tb
+// (leaf: vertex boxes grown by 1e-4; interior: union of the children), flag
+// the escaped triangles -- those whose grown vertex box does not lie inside
+// every slot box the quad nodes test on the way to them -- and make the quad
+// nodes' subtree boxes (DTBox per quad node). `wide`: the closest-hit
+// traversal tree too, over tri->tb or, without tri, over the BVH2's own
+// boxes: a 4-wide collapse with tight slot boxes (largest-area child opened
+// first), as exact nodes and compact copies, root 0. There is none (wcount
+// 0, Ok) when a node's box does not contain its children's, or (check_indices
+// given) when the leaves do not hold each of the index_count slots and each
+// primitive exactly once -- spatial-split trees, whose leaf boxes bound
+// fragments -- closest hit then reads the exact nodes in the reference's
+// order.
+struct MbvhRequest {
+  const MbvhTriangles* tri = nullptr;
+  bool wide = false;
+  const uint32_t* check_indices = nullptr;
+  uint32_t index_count = 0;
+};
+struct MbvhOutput {
+  DMNode* mnodes = nullptr;  // Mbvh::construct's nodes (library pool, owned by the caller)
+  uint32_t mcount = 0;
+  DTBox* tboxes = nullptr;   // with tri
+  uint32_t escaped = 0;      // with tri: triangles that escape a box
+  DMNode* wnodes = nullptr;  // traversal tree: exact and compact nodes
+  DQNode* wq = nullptr;
+  uint32_t wcount = 0;
+};
+// Mbvh::construct (src/bvh.rs:381-404).
+ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, const MbvhRequest& req,
+                      MbvhOutput* out);
 
 
 // Bvh::refit (src/bvh.rs:176-205) bounds, topology kept. Leaves index
@@ -275,12 +275,16 @@ cudaError_t launch_locb_segments(const DAabb* aabbs, const uint32_t* sorted, uin
                                  DAabb* final_nodes, uint32_t* nb, uint32_t* status, unsigned blocks,
                                  uint32_t big_count, uint32_t* cluster_sums, unsigned clusters, cudaStream_t s,
                                  cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
-// Per-mesh MBVH collapse of a concatenated forest (see mbvh.cu).
-cudaError_t launch_collapse_segments(const DAabb* nodes, uint32_t node_count, const uint32_t* prim_off,
-                                     const uint32_t* order, uint32_t mesh_count, uint32_t* parent, uint32_t* arrive,
-                                     uint32_t* cnt_e, uint32_t* cnt_o, uint32_t* mbase, uint2* q0, uint2* q1,
-                                     DMNode* mnodes, uint32_t m_capacity, uint32_t* status, unsigned blocks,
-                                     cudaStream_t s);
+// MBVH collapse of a concatenated forest (see mbvh.cu): mesh m's quad nodes
+// at [mbase[m], mbase[m + 1]); with wnodes / wq also the traversal trees of
+// all meshes (LOCB: nested boxes), mesh m's root at qroot[m]. mnodes, wnodes
+// and wq hold total_prims nodes or more. scratch:
+// collapse_scratch_words(node_count) words; walloc: one word.
+size_t collapse_scratch_words(size_t node_count);
+cudaError_t launch_collapse_forest(const DAabb* nodes, uint32_t node_count, const uint32_t* prim_off,
+                                   uint32_t mesh_count, uint32_t total_prims, uint32_t* scratch, uint32_t* mbase,
+                                   DMNode* mnodes, DMNode* wnodes, DQNode* wq, uint32_t* qroot, uint32_t* walloc,
+                                   uint32_t* status, cudaStream_t s);
 
 // ------------------------------------------------------------------ backward
 cudaError_t launch_intersect_backward(const float* vertices, size_t prim_count, const float* rays,

@@ -9,9 +9,9 @@
 // for interior c and 0 for leaves. So:
 //   1. parent pointers;
 //   2. cntE/cntO bottom-up (the second child to arrive at a parent computes it);
-//   3. top-down, one quad level per step of a cooperative launch: a quad node
-//      with index mi gives its k-th interior slot the index
-//      mi + 1 + sum of cntE over the interior slots before it.
+//   3. every quad node's index from the counts on its way up (find_place):
+//      no order between levels;
+//   4. the quad nodes, one thread each in index order.
 // The slot contents reproduce merge_nodes line by line, including its quirks
 // (a leaf child keeps the parent's box in its slot; the second slot of that
 // side stays empty with the parent's box).
@@ -62,23 +62,37 @@ __device__ __forceinline__ DAabb grown_triangle_box(const float* __restrict__ ve
   return b;
 }
 
+// Parent word of a node: parent << 1 | 1 for the right child of a pair
+// (kNone: no parent). Node indices that left_first can name are below 2^31.
+__device__ __forceinline__ uint32_t parent_of(uint32_t w) { return w >> 1; }
+
+// cnt / known (may be NULL) start as kNone words: not counted / not placed.
 __global__ void __launch_bounds__(kBlock)
     k_parents(const DAabb* __restrict__ nodes, uint32_t node_count, uint32_t* __restrict__ parent,
-              uint32_t* __restrict__ arrive, uint32_t* __restrict__ status) {
+              uint32_t* __restrict__ arrive, uint2* __restrict__ cnt, uint2* __restrict__ known,
+              uint32_t* __restrict__ status) {
   uint32_t c = blockIdx.x * kBlock + threadIdx.x;
   if (c >= node_count) return;
   arrive[c] = 0;
+  if (cnt) cnt[c] = make_uint2(kNone, kNone);
+  if (known) known[c] = make_uint2(kNone, kNone);
   DAabb nd = load_aabb(nodes + c);
-  if (nd.count < 0 && nd.left_first >= 0) {
+  if (nd.count < 0 && nd.left_first >= 0 && c <= 0x7fffffffu) {
     uint32_t lf = (uint32_t)nd.left_first;
     if (lf + 1 < node_count) {
-      parent[lf] = c;
-      parent[lf + 1] = c;
+      parent[lf] = c << 1;
+      parent[lf + 1] = c << 1 | 1u;
     } else {
       atomicOr(status, kStatusBadIndex);
     }
   }
 }
+
+// Per node {cntE, cntO}. kBadBox in the first word (TRIS): the node's box
+// does not contain its box from the triangles.
+constexpr uint32_t kBadBox = 1u << 31;
+__device__ __forceinline__ uint32_t cnt_e_of(uint2 c) { return c.x & ~kBadBox; }
+__device__ __forceinline__ bool counted(uint2 c) { return c.y != kNone; }
 
 // With TRIS, the same walk also computes every node's traversal box `tb`
 // from the triangles: a leaf's is the union of its triangles' vertex boxes
@@ -88,14 +102,13 @@ __global__ void __launch_bounds__(kBlock)
 template <bool TRIS>
 __global__ void __launch_bounds__(kBlock)
     k_counts_bottom_up(const DAabb* __restrict__ nodes, uint32_t node_count, const uint32_t* __restrict__ parent,
-                       uint32_t* __restrict__ arrive, uint32_t* __restrict__ cnt_e, uint32_t* __restrict__ cnt_o,
-                       MbvhTriangles tri, uint32_t* __restrict__ status) {
+                       uint32_t* __restrict__ arrive, uint2* __restrict__ cnt, MbvhTriangles tri,
+                       uint32_t* __restrict__ status) {
   uint32_t c = blockIdx.x * kBlock + threadIdx.x;
   if (c >= node_count) return;
   DAabb nd = load_aabb(nodes + c);
   if (nd.count < 0) return;  // walks start at leaves
-  cnt_e[c] = 0;
-  cnt_o[c] = 0;
+  cnt[c] = make_uint2(0u, 0u);
   if (TRIS) {
     DAabb box = nd;
     for (int a = 0; a < 3; ++a) { box.min[a] = 1e34f; box.max[a] = -1e34f; }
@@ -116,23 +129,26 @@ __global__ void __launch_bounds__(kBlock)
   }
   uint32_t x = c;
   for (uint32_t steps = 0; steps < node_count; ++steps) {
-    uint32_t p = __ldcg(parent + x);
-    if (p == kNone) break;
+    const uint32_t w = __ldcg(parent + x);
+    if (w == kNone) break;
+    const uint32_t p = parent_of(w);
     if (arrive_acq_rel(arrive + p) == 0u) break;  // first arrival: the sibling finishes p
     DAabb pn = load_aabb(nodes + p);
     uint32_t lf = (uint32_t)pn.left_first;
-    uint32_t e = 1u + __ldcg(cnt_o + lf) + __ldcg(cnt_o + lf + 1);
-    uint32_t o = __ldcg(cnt_e + lf) + __ldcg(cnt_e + lf + 1);
-    cnt_e[p] = e;
-    cnt_o[p] = o;
+    const uint2 cl = __ldcg(cnt + lf), cr = __ldcg(cnt + lf + 1);
+    uint32_t e = 1u + cl.y + cr.y;
+    const uint32_t o = cnt_e_of(cl) + cnt_e_of(cr);
     if (TRIS) {
       const DAabb l = load_aabb_cg(tri.tb + lf), r = load_aabb_cg(tri.tb + lf + 1);
+      DAabb t = pn;
       for (int a = 0; a < 3; ++a) {
-        pn.min[a] = rs_min(l.min[a], r.min[a]);
-        pn.max[a] = rs_max(l.max[a], r.max[a]);
+        t.min[a] = rs_min(l.min[a], r.min[a]);
+        t.max[a] = rs_max(l.max[a], r.max[a]);
       }
-      store_aabb(tri.tb + p, pn);
+      if (!box_contains(pn, t)) e |= kBadBox;
+      store_aabb(tri.tb + p, t);
     }
+    cnt[p] = make_uint2(e, o);
     x = p;
   }
 }
@@ -140,41 +156,102 @@ __global__ void __launch_bounds__(kBlock)
 struct CollapseParams {
   const DAabb* nodes;
   uint32_t node_count;
-  const uint32_t* cnt_e;
+  const uint32_t* parent;  // parent words
+  const uint2* cnt;
+  uint2* known;            // places found so far: {place << 1 | depth parity, nearest bad box}; roots preset
+  uint32_t* quads;         // BVH2 node of every quad node
   DMNode* mnodes;
-  uint32_t m_total;
-  uint2* queue[2];
-  uint32_t* qcount;  // 3 rotating counters
-  GridBarrier* bar;
+  uint32_t m_total;        // capacity of quads / mnodes / tboxes
+  const uint32_t* m_count; // quad nodes (device)
+  bool forest;             // several meshes (k_seg_mbase)
   uint32_t* status;
-  // escape flags only: triangles, per quad node the intersection of the
-  // slot boxes on the way to it, the count of escaped triangles
+  // escape flags only: triangles, the count of escaped triangles
   MbvhTriangles tri;
-  DAabb* ibox;
   uint32_t* escaped;
   DTBox* tboxes;  // optional (TRIS): subtree boxes of every quad node's slots
-  // optional: the quad count, read on the device; m_total then holds the
-  // capacity of mnodes / ibox / tboxes
-  const uint32_t* m_total_dev;
 };
 
-// Warp-aggregated reservation of n consecutive entries from *counter: every
-// lane of the warp calls it (n = 0 for nothing), one atomic per warp; the
-// lane's first entry is returned. The top-down passes append to one queue
-// counter per level, whose atomics would otherwise serialise.
-__device__ __forceinline__ uint32_t warp_reserve(uint32_t* counter, uint32_t n) {
-  const int lane = threadIdx.x & 31;
-  uint32_t incl = n;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
+__device__ __forceinline__ uint2 ld_place(const uint2* p) {
+  const unsigned long long v = __ldcg(reinterpret_cast<const unsigned long long*>(p));
+  return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+}
+__device__ __forceinline__ void st_place(uint2* p, uint2 v) {
+  __stcg(reinterpret_cast<unsigned long long*>(p), (unsigned long long)v.x | ((unsigned long long)v.y << 32));
+}
+
+// Place of interior node x: a node at even depth is a quad node and its
+// place is its quad index; the quad nodes below a node at odd depth start at
+// its place. From parent to child the place grows by
+//   even parent: 1 + (right child: cntO(left sibling))
+//   odd parent:  (right child: cntE(left sibling)).
+// The walk goes up until it meets a node whose place is known (other threads
+// publish theirs as they find them; what is not there yet only makes the
+// walk longer, nothing waits) and keeps the sums for both parities x may
+// have. Only counted nodes are passed: they form trees, so the walk ends.
+// What bounds it is the latency of the walk, one dependent read per level;
+// nodes near the root have low indices and are placed first, so most walks
+// are short. The level-by-level frontier it replaces spent a grid barrier
+// per level (collapse of 200k
+// sphere triangles 172 us; k_place 27 + k_quads 13 us now; refit of them with
+// both trees 824 -> 440 us).
+// bad (TRIS): the nearest quad node at or above x whose box misses
+// triangles below it (kNone: none).
+struct Place {
+  uint32_t pos, parity, bad;
+  bool ok;
+};
+template <bool TRIS>
+__device__ Place find_place(const CollapseParams& p, uint32_t x) {
+  uint32_t even = 0, odd = 0;                 // sums if the current node lies at even / odd depth
+  uint32_t bad_even = kNone, bad_odd = kNone;  // the same for the nearest bad quad node
+  uint32_t cur = x;
+  for (uint32_t k = 0; k < p.node_count; ++k) {
+    const uint2 s = ld_place(p.known + cur);
+    const uint32_t w = __ldg(p.parent + cur);
+    const uint2 own = __ldg(p.cnt + cur);
+    if (s.x != kNone) {
+      const bool is_even = (s.x & 1u) == 0u;
+      Place r;
+      r.pos = (s.x >> 1) + (is_even ? even : odd);
+      r.parity = (s.x & 1u) ^ (k & 1u);
+      r.bad = is_even ? bad_even : bad_odd;
+      if (r.bad == kNone) r.bad = s.y;
+      r.ok = true;
+      return r;
+    }
+    if (w == kNone || !counted(own)) break;
+    if (TRIS && (own.x & kBadBox) && bad_even == kNone) bad_even = cur;
+    uint32_t e = 0, o = 1u;
+    if (w & 1u) {
+      const uint2 sib = __ldg(p.cnt + cur - 1u);
+      e = cnt_e_of(sib);
+      o += sib.y;
+    }
+    // cur at even depth: its parent is odd
+    const uint32_t se = even + e, so = odd + o, be = bad_even, bo = bad_odd;
+    odd = se;
+    even = so;
+    bad_odd = be;
+    bad_even = bo;
+    cur = parent_of(w);
   }
-  const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-  uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(counter, total);
-  base = __shfl_sync(0xffffffffu, base, 31);
-  return base + incl - n;
+  Place r;
+  r.pos = r.parity = 0u;
+  r.bad = kNone;
+  r.ok = false;
+  return r;
+}
+
+// Four 256-bit stores: neighbouring threads write neighbouring 128-byte
+// nodes, so every store fills whole sectors.
+__device__ __forceinline__ void store_node(DMNode* out, const DMNode& m) {
+  const float* f = reinterpret_cast<const float*>(&m);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(reinterpret_cast<float*>(out) + 8 * k),
+                 "f"(f[8 * k]), "f"(f[8 * k + 1]), "f"(f[8 * k + 2]), "f"(f[8 * k + 3]), "f"(f[8 * k + 4]),
+                 "f"(f[8 * k + 5]), "f"(f[8 * k + 6]), "f"(f[8 * k + 7])
+                 : "memory");
 }
 
 __device__ __forceinline__ void set_slot_box(DMNode& m, int i, const DAabb& b) {
@@ -182,36 +259,24 @@ __device__ __forceinline__ void set_slot_box(DMNode& m, int i, const DAabb& b) {
   m.max_x[i] = b.max[0]; m.max_y[i] = b.max[1]; m.max_z[i] = b.max[2];
 }
 
-// Escape flags of quad node mi's slots (TRIS): an interior slot hands its
-// child quad the intersection of the slot boxes on the way to it; a leaf
-// slot's triangles are escaped when their vertex box grown by 1e-4 is not
-// inside that intersection -- the reference's walk tests these boxes
-// before it yields the triangle (src/iter_indices.rs:264-313), so it can
-// miss the triangle's hits. Flags go to the flags word of each leaf-ordered
-// triangle record (kTriEscape).
-__device__ void mark_escapes(const CollapseParams& p, uint32_t mi, const DMNode& m) {
-  const DAabb in = load_aabb_cg(p.ibox + mi);
+// Escape flags of a quad node's leaf slots (TRIS): a leaf slot's triangle is
+// escaped when its vertex box grown by 1e-4 is not inside every slot box on
+// the way to it -- the reference's walk tests these boxes before it yields
+// the triangle (src/iter_indices.rs:264-313), so it can miss the triangle's
+// hits. Those boxes are the leaf's slot box and the boxes of the quad nodes
+// on the way up (but the root's, which is no slot). A quad node's box that
+// contains its box from the triangles contains every triangle below it, so
+// only the others, marked kBadBox, are compared; they are few. Flags go to
+// the flags word of each leaf-ordered triangle record (kTriEscape).
+__device__ void mark_escapes(const CollapseParams& p, const DMNode& m, uint32_t bad) {
   uint32_t n_esc = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int32_t ch = m.children[i], cnt = m.counts[i];
-    if (cnt < 0 && ch < 0) continue;  // empty slot
-    const float smin[3] = {m.min_x[i], m.min_y[i], m.min_z[i]}, smax[3] = {m.max_x[i], m.max_y[i], m.max_z[i]};
-    DAabb box;
-    bool nan = false;
-    for (int a = 0; a < 3; ++a) {
-      nan = nan || !(smin[a] == smin[a]) || !(smax[a] == smax[a]);
-      box.min[a] = fmaxf(in.min[a], smin[a]);
-      box.max[a] = fminf(in.max[a], smax[a]);
-    }
-    if (nan)  // a NaN bound: nothing below counts as inside
-      for (int a = 0; a < 3; ++a) { box.min[a] = 3.0e38f; box.max[a] = -3.0e38f; }
-    box.count = 0;
-    box.left_first = 0;
-    if (cnt < 0) {
-      if ((uint32_t)ch < p.m_total) store_aabb(p.ibox + ch, box);
-      continue;
-    }
+    if (cnt < 0) continue;  // empty or interior slot
+    DAabb slot_box;
+    slot_box.min[0] = m.min_x[i]; slot_box.min[1] = m.min_y[i]; slot_box.min[2] = m.min_z[i];
+    slot_box.max[0] = m.max_x[i]; slot_box.max[1] = m.max_y[i]; slot_box.max[2] = m.max_z[i];
     for (int32_t j = 0; j < cnt; ++j) {
       const uint32_t slot = (uint32_t)ch + (uint32_t)j;
       const uint32_t prim = slot < p.tri.index_count ? __ldg(p.tri.indices + slot) : kNone;
@@ -219,21 +284,27 @@ __device__ void mark_escapes(const CollapseParams& p, uint32_t mi, const DMNode&
         atomicOr(p.status, kStatusBadIndex);
         break;
       }
-      const bool esc = !box_contains(box, grown_triangle_box(p.tri.vertices, prim));
-      reinterpret_cast<float*>(p.tri.tris + (size_t)kTriFloat4 * slot + 1)[3] = __uint_as_float(esc ? kTriEscape : 0u);
-      n_esc += esc ? 1u : 0u;
+      const DAabb t = grown_triangle_box(p.tri.vertices, prim);
+      bool inside = box_contains(slot_box, t);
+      uint32_t b = bad;
+      while (inside && b != kNone) {
+        inside = box_contains(load_aabb(p.nodes + b), t);
+        // the next one above b: its grandparent's (b lies at even depth >= 2)
+        const uint32_t w = __ldg(p.parent + b);
+        const uint32_t gw = w != kNone ? __ldg(p.parent + parent_of(w)) : kNone;
+        b = gw != kNone ? find_place<true>(p, parent_of(gw)).bad : kNone;
+      }
+      reinterpret_cast<float*>(p.tri.tris + (size_t)kTriFloat4 * slot + 1)[3] =
+          __uint_as_float(inside ? 0u : kTriEscape);
+      n_esc += inside ? 0u : 1u;
     }
   }
   if (n_esc) atomicAdd(p.escaped, n_esc);
 }
 
-// merge_nodes(mi, c) without the recursion: fills quad node mi and appends
-// its interior slots (bvh node, quad index) to `next`. AGG: called by all
-// lanes of a warp (`valid` false for lanes without an item), the queue
-// entries reserved once per warp.
-template <bool TRIS, bool AGG>
-__device__ void emit_quad(const CollapseParams& p, uint32_t c, uint32_t mi, uint2* next, uint32_t* next_count,
-                          bool valid = true) {
+// merge_nodes(mi, c) without the recursion: fills quad node mi.
+template <bool TRIS>
+__device__ void emit_quad(const CollapseParams& p, uint32_t c, uint32_t mi, uint32_t bad) {
   const DAabb cur = load_aabb(p.nodes + c);
   DMNode m;
 #pragma unroll
@@ -245,7 +316,13 @@ __device__ void emit_quad(const CollapseParams& p, uint32_t c, uint32_t mi, uint
   int32_t nodes_[4] = {-1, -1, -1, -1};
   int32_t leafs[4] = {-1, -1, -1, -1};
   int32_t sub[4] = {-1, -1, -1, -1};  // BVH2 node under each slot (TRIS: its box from the triangles)
-  if (cur.left_first >= 0) {
+  if (p.forest && cur.count >= 0) {
+    // Root leaf of a mesh: the single-mesh tree has this one node, so
+    // merge_nodes finds only the root itself in slot 0 (its left_first is
+    // no node of this forest).
+    nodes_[0] = cur.left_first;
+    leafs[0] = cur.count;
+  } else if (cur.left_first >= 0) {
     const uint32_t lf = (uint32_t)cur.left_first;
 #pragma unroll
     for (int side = 0; side < 2; ++side) {
@@ -279,14 +356,6 @@ __device__ void emit_quad(const CollapseParams& p, uint32_t c, uint32_t mi, uint
       }
     }
   }
-  uint32_t n_int = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) n_int += (nodes_[i] >= 0 && leafs[i] < 0) ? 1u : 0u;
-  if (!valid) n_int = 0;
-  uint32_t qslot = 0;
-  if (AGG) qslot = warp_reserve(next_count, n_int);
-  else if (n_int) qslot = atomicAdd(next_count, n_int);
-  if (!valid) return;
   uint32_t next_index = mi + 1u;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -300,31 +369,21 @@ __device__ void emit_quad(const CollapseParams& p, uint32_t c, uint32_t mi, uint
       if (node != -1) atomicOr(p.status, kStatusBadIndex);
       continue;
     }
-    const uint32_t g = (uint32_t)node;
-    const uint32_t idx = next_index;
-    next_index += __ldg(p.cnt_e + g);
-    const uint32_t slot = qslot++;
-    if (idx < p.m_total) {
-      m.children[i] = (int32_t)idx;
-      if (slot < p.m_total) next[slot] = make_uint2(g, idx);
-      else atomicOr(p.status, kStatusBadIndex);
-    } else {
-      atomicOr(p.status, kStatusBadIndex);
-    }
+    const uint2 below = __ldg(p.cnt + node);
+    if (next_index < p.m_total && counted(below)) m.children[i] = (int32_t)next_index;
+    else atomicOr(p.status, kStatusBadIndex);
+    next_index += cnt_e_of(below);
   }
   if (mi < p.m_total) {
-    float4* dst = reinterpret_cast<float4*>(p.mnodes + mi);
-    const float4* src = reinterpret_cast<const float4*>(&m);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) dst[k] = src[k];
-    if (TRIS) mark_escapes(p, mi, m);
+    store_node(p.mnodes + mi, m);
+    if (TRIS) mark_escapes(p, m, bad);
     if (TRIS && p.tboxes) {
       DTBox t;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         bool ok = sub[i] >= 0 && (uint32_t)sub[i] < p.node_count;
         DAabb b = cur;
-        if (ok) b = load_aabb_cg(p.tri.tb + sub[i]);
+        if (ok) b = load_aabb(p.tri.tb + sub[i]);
         for (int a = 0; a < 3; ++a)  // false for NaN
           ok = ok && fabsf(b.min[a]) <= kCompactRange && fabsf(b.max[a]) <= kCompactRange;
         const float inf = __int_as_float(0x7f800000);
@@ -343,71 +402,39 @@ __device__ void emit_quad(const CollapseParams& p, uint32_t c, uint32_t mi, uint
 }
 
 template <bool TRIS>
-__global__ void __launch_bounds__(kBlock) k_collapse(CollapseParams p) {
-  if (p.m_total_dev) {
-    // every block reads the same word (written before the launch), so all
-    // of them return here together or none does
-    const uint32_t mt = __ldcg(p.m_total_dev);
-    if (mt == 0 || mt > p.m_total) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(p.status, kStatusBadIndex);
-      return;
-    }
-    p.m_total = mt;
+__global__ void __launch_bounds__(kBlock) k_quads(CollapseParams p) {
+  const uint32_t mi = blockIdx.x * kBlock + threadIdx.x;
+  if (mi >= min(__ldg(p.m_count), p.m_total)) return;
+  const uint32_t c = __ldg(p.quads + mi);
+  if (c >= p.node_count) {  // not placed: only after another error
+    atomicOr(p.status, kStatusBadIndex);
+    return;
   }
-  const uint32_t G = gridDim.x;
-  const uint32_t tid = blockIdx.x * kBlock + threadIdx.x, nthreads = G * kBlock;
-  for (uint32_t level = 0; level < p.m_total + 1; ++level) {
-    uint32_t size = __ldcg(p.qcount + (level % 3));
-    if (size == 0) break;
-    if (size > p.m_total) size = p.m_total;  // only after a kStatusBadIndex
-    const uint2* q = p.queue[level & 1];
-    uint2* next = p.queue[(level + 1) & 1];
-    uint32_t* next_count = p.qcount + ((level + 1) % 3);
-    // warp-uniform loop: every lane takes part in the queue reservation
-    for (uint32_t k0 = tid - (threadIdx.x & 31u); k0 < size; k0 += nthreads) {
-      const uint32_t k = k0 + (threadIdx.x & 31u);
-      const bool valid = k < size;
-      const uint2 item = valid ? __ldcg(q + k) : make_uint2(0u, 0u);
-      emit_quad<TRIS, true>(p, item.x, item.y, next, next_count, valid);
-    }
-    if (tid == 0) p.qcount[(level + 2) % 3] = 0;
-    if (!grid_sync(p.bar, G, p.status)) return;
-  }
+  emit_quad<TRIS>(p, c, mi, TRIS ? p.known[c].y : kNone);
 }
 
-__global__ void k_collapse_init(const uint32_t* cnt_e, const DAabb* nodes, uint2* queue0, uint32_t* qcount,
-                                uint32_t* m_total_out) {
+// The root's place, and the number of quad nodes for the host. A root whose
+// count did not come up (no tree) is an error.
+__global__ void k_root_place(const uint2* cnt, const DAabb* nodes, uint2* known, uint32_t m_cap, uint32_t* m_total,
+                             uint32_t* walloc, uint32_t* status) {
   if (threadIdx.x == 0) {
-    queue0[0] = make_uint2(0u, 0u);
-    qcount[0] = 1;
-    qcount[1] = 0;
-    qcount[2] = 0;
-    DAabb r = *nodes;
-    uint32_t t = r.count < 0 ? cnt_e[0] : 1u;
-    *m_total_out = t;
+    *walloc = 1u;  // traversal node 0 is the root's
+    const uint2 c = *cnt;
+    const uint32_t t = nodes->count < 0 ? cnt_e_of(c) : 1u;
+    if (!counted(c) || t == 0u || t > m_cap) atomicOr(status, kStatusBadIndex);
+    else *known = make_uint2(0u, kNone);
+    *m_total = t;
   }
 }
-
-// The root quad's slots are the first boxes on every way down.
-__global__ void k_ibox_init(DAabb* ibox) {
-  if (threadIdx.x == 0) {
-    DAabb b;
-    for (int a = 0; a < 3; ++a) { b.min[a] = -3.0e38f; b.max[a] = 3.0e38f; }
-    b.count = 0;
-    b.left_first = 0;
-    store_aabb(ibox, b);
-  }
-}
-
 
 // ---------------------------------------------------------------- many meshes
 // A concatenated forest: mesh m's root is BVH2 node 2 off_m - m. Its quad
 // nodes get the contiguous index range [mbase[m], mbase[m+1]) (the
-// single-mesh numbering shifted by mbase[m]), and one block per mesh runs
-// the top-down frontier of k_collapse with block barriers.
-__global__ void __launch_bounds__(1024) k_seg_mbase(const DAabb* __restrict__ nodes, const uint32_t* __restrict__ cnt_e,
+// single-mesh numbering shifted by mbase[m]): its root's place is mbase[m],
+// and k_quads does the rest for all meshes at once.
+__global__ void __launch_bounds__(1024) k_seg_mbase(const DAabb* __restrict__ nodes, const uint2* __restrict__ cnt,
                                                     const uint32_t* __restrict__ prim_off, uint32_t mesh_count,
-                                                    uint32_t* __restrict__ mbase) {
+                                                    uint2* __restrict__ known, uint32_t* __restrict__ mbase) {
   __shared__ uint32_t s_warp[32];
   uint32_t carry = 0;
   for (uint32_t base = 0; base < mesh_count; base += 1024) {
@@ -417,81 +444,18 @@ __global__ void __launch_bounds__(1024) k_seg_mbase(const DAabb* __restrict__ no
       const uint32_t off = prim_off[m], n = prim_off[m + 1] - off;
       if (n > 0) {
         const uint32_t root = 2u * off - m;
-        q = load_aabb(nodes + root).count < 0 ? cnt_e[root] : 1u;
+        if (counted(cnt[root])) q = load_aabb(nodes + root).count < 0 ? cnt_e_of(cnt[root]) : 1u;
       }
     }
     uint32_t total;
     const uint32_t incl = block_inclusive_scan<1024>(q, s_warp, &total);
-    if (m < mesh_count) mbase[m] = carry + incl - q;
+    if (m < mesh_count) {
+      mbase[m] = carry + incl - q;
+      if (q) known[2u * prim_off[m] - m] = make_uint2((carry + incl - q) << 1, kNone);
+    }
     carry += total;
   }
   if (threadIdx.x == 0) mbase[mesh_count] = carry;
-}
-
-struct SegCollapseParams {
-  CollapseParams c;
-  const uint32_t* prim_off;
-  const uint32_t* order;
-  const uint32_t* mbase;
-  uint2* queue[2];
-  uint32_t mesh_count;
-};
-
-__global__ void __launch_bounds__(kBlock) k_collapse_segments(SegCollapseParams p) {
-  __shared__ uint32_t s_count[2];
-  for (uint32_t q = blockIdx.x; q < p.mesh_count; q += gridDim.x) {
-    const uint32_t m = p.order[q];
-    const uint32_t off = p.prim_off[m], n = p.prim_off[m + 1] - off;
-    if (n == 0) continue;
-    const uint32_t base = p.mbase[m];
-    const uint32_t quads = p.mbase[m + 1] - base;
-    const uint32_t root = 2u * off - m;
-    const DAabb rb = load_aabb(p.c.nodes + root);
-    if (rb.count >= 0) {
-      // Root leaf (n <= 2): the single-mesh tree has this one node, so
-      // merge_nodes finds only the root itself in slot 0. emit_quad would
-      // read the next mesh's nodes as the root's second child here.
-      if (threadIdx.x == 0 && quads >= 1) {
-        DMNode q;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          set_slot_box(q, i, rb);
-          q.children[i] = -1;
-          q.counts[i] = -1;
-        }
-        q.children[0] = rb.left_first;
-        q.counts[0] = rb.count;
-        float4* dst = reinterpret_cast<float4*>(p.c.mnodes + base);
-        const float4* src = reinterpret_cast<const float4*>(&q);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) dst[k] = src[k];
-      }
-      continue;
-    }
-    if (threadIdx.x == 0) {
-      p.queue[0][base] = make_uint2(root, base);
-      s_count[0] = 1;
-      s_count[1] = 0;
-    }
-    __syncthreads();
-    int cur = 0;
-    for (uint32_t level = 0; level <= quads; ++level) {
-      uint32_t size = s_count[cur];
-      if (size == 0) break;
-      if (size > quads) size = quads;
-      const uint2* qin = p.queue[cur] + base;
-      uint2* qout = p.queue[cur ^ 1] + base;
-      for (uint32_t k = threadIdx.x; k < size; k += kBlock) {
-        const uint2 item = qin[k];
-        emit_quad<false, false>(p.c, item.x, item.y, qout, &s_count[cur ^ 1]);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) s_count[cur] = 0;
-      __syncthreads();
-      cur ^= 1;
-    }
-    __syncthreads();
-  }
 }
 
 // Bvh::refit (src/bvh.rs:176-205): leaf box = union of its primitives'
@@ -525,8 +489,9 @@ __global__ void __launch_bounds__(kBlock)
   if (nd.left_first < 0) return;
   uint32_t x = c;
   for (uint32_t steps = 0; steps < node_count; ++steps) {
-    uint32_t p = __ldcg(parent + x);
-    if (p == kNone) break;
+    const uint32_t w = __ldcg(parent + x);
+    if (w == kNone) break;
+    const uint32_t p = parent_of(w);
     if (arrive_acq_rel(arrive + p) == 0u) break;
     DAabb pn = load_aabb_cg(nodes + p);
     const uint32_t lf = (uint32_t)pn.left_first;
@@ -544,114 +509,6 @@ __global__ void __launch_bounds__(kBlock)
 
 }  // namespace
 
-ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, DMNode** mnodes_out,
-                      uint32_t* mnode_count, const MbvhTriangles* tri, uint32_t* escaped_out) {
-  *mnodes_out = nullptr;
-  *mnode_count = 0;
-  if (escaped_out) *escaped_out = 0;
-  if (node_count == 0) return Ok;  // Mbvh::default()
-  const bool with_tris = tri != nullptr;
-  if (with_tris && (!tri->indices || !tri->vertices || !tri->tris || !tri->tb)) return Error;
-  cudaError_t e;
-  Scratch<uint32_t> parent, arrive, cnt_e, cnt_o, status, mtot;
-  if ((e = parent.alloc(node_count, s)) || (e = arrive.alloc(node_count, s)) || (e = cnt_e.alloc(node_count, s)) ||
-      (e = cnt_o.alloc(node_count, s)) || (e = status.alloc(4, s)) || (e = mtot.alloc(4, s)))
-    return cuda_rc(e);
-  if ((e = cudaMemsetAsync(parent.ptr, 0xff, (size_t)node_count * 4, s)) ||
-      (e = cudaMemsetAsync(status.ptr, 0, 16, s)))
-    return cuda_rc(e);
-  // unreachable nodes keep an empty leaf box (never read by a collapse)
-  if (with_tris && (e = cudaMemsetAsync(tri->tb, 0, (size_t)node_count * sizeof(DAabb), s))) return cuda_rc(e);
-  const unsigned blocks = (node_count + kBlock - 1) / kBlock;
-  k_parents<<<blocks, kBlock, 0, s>>>(nodes, node_count, parent.ptr, arrive.ptr, status.ptr);
-  const MbvhTriangles none;
-  if (with_tris)
-    k_counts_bottom_up<true><<<blocks, kBlock, 0, s>>>(nodes, node_count, parent.ptr, arrive.ptr, cnt_e.ptr,
-                                                       cnt_o.ptr, *tri, status.ptr);
-  else
-    k_counts_bottom_up<false><<<blocks, kBlock, 0, s>>>(nodes, node_count, parent.ptr, arrive.ptr, cnt_e.ptr,
-                                                        cnt_o.ptr, none, status.ptr);
-  Scratch<uint2> q0, q1;
-  Scratch<uint32_t> qcount;
-  Scratch<GridBarrier> bar;
-  if ((e = qcount.alloc(4, s)) || (e = bar.alloc(1, s))) return cuda_rc(e);
-  if ((e = q0.alloc(node_count, s)) || (e = q1.alloc(node_count, s))) return cuda_rc(e);
-  k_collapse_init<<<1, 32, 0, s>>>(cnt_e.ptr, nodes, q0.ptr, qcount.ptr, mtot.ptr);
-  // The quad count stays on the device (the collapse reads it); arrays are
-  // sized by its bound: quad nodes are interior BVH2 nodes, at most
-  // (node_count - 1) / 2 of a binary tree, or the root leaf.
-  const uint32_t m_cap = (node_count + 1u) / 2u;
-  Scratch<DAabb> ibox;
-  if (with_tris) {
-    if ((e = ibox.alloc(m_cap, s))) return cuda_rc(e);
-    k_ibox_init<<<1, 32, 0, s>>>(ibox.ptr);
-  }
-  DMNode* mnodes = nullptr;
-  DTBox* tboxes = nullptr;
-  if ((e = device_alloc(&mnodes, m_cap, s))) return cuda_rc(e);
-  if (with_tris && tri->tboxes_out && (e = device_alloc(&tboxes, m_cap, s))) {
-    pool_free(mnodes, s);
-    return cuda_rc(e);
-  }
-  auto drop = [&]() {
-    pool_free(mnodes, s);
-    pool_free(tboxes, s);
-  };
-  if ((e = cudaMemsetAsync(bar.ptr, 0, sizeof(GridBarrier), s))) {
-    drop();
-    return cuda_rc(e);
-  }
-  auto kern = with_tris ? k_collapse<true> : k_collapse<false>;
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, 0);
-  if (per_sm < 1) per_sm = 1;
-  unsigned grid = (unsigned)(sm_count() * per_sm);
-  const unsigned useful = (m_cap + kBlock - 1) / kBlock;
-  if (grid > useful) grid = useful;
-  if (grid < 1) grid = 1;
-  CollapseParams p;
-  p.nodes = nodes;
-  p.node_count = node_count;
-  p.cnt_e = cnt_e.ptr;
-  p.mnodes = mnodes;
-  p.m_total = m_cap;
-  p.m_total_dev = mtot.ptr;
-  p.queue[0] = q0.ptr;
-  p.queue[1] = q1.ptr;
-  p.qcount = qcount.ptr;
-  p.bar = bar.ptr;
-  p.status = status.ptr;
-  if (with_tris) p.tri = *tri;
-  p.ibox = ibox.ptr;
-  p.escaped = status.ptr + 2;
-  p.tboxes = tboxes;
-  void* args[] = {&p};
-  if ((e = cudaLaunchCooperativeKernel((void*)kern, dim3(grid), dim3(kBlock), args, 0, s))) {
-    drop();
-    return cuda_rc(e);
-  }
-  uint32_t st[4] = {0, 0, 0, 0};
-  if ((e = cudaMemcpyAsync(st, status.ptr, 12, cudaMemcpyDeviceToHost, s)) ||
-      (e = cudaMemcpyAsync(st + 3, mtot.ptr, 4, cudaMemcpyDeviceToHost, s)) || (e = cudaStreamSynchronize(s))) {
-    drop();
-    return cuda_rc(e);
-  }
-  if (st[0] != 0) {
-    drop();
-    return (st[0] & kStatusTimeout) ? Timeout : Error;
-  }
-  const uint32_t m_total = st[3];  // checked on the device: 1 .. m_cap
-  *mnodes_out = mnodes;
-  *mnode_count = m_total;
-  if (with_tris && tri->tboxes_out) *tri->tboxes_out = tboxes;
-  if (escaped_out) *escaped_out = st[2];
-  return Ok;
-}
-
-}  // namespace rtbvh
-
-namespace rtbvh {
-
 ResultCode refit_bvh(DAabb* nodes, uint32_t node_count, const uint32_t* indices, uint32_t index_count,
                      uint32_t prim_count, const DAabb* aabbs, cudaStream_t s) {
   if (node_count == 0) return Ok;
@@ -663,7 +520,7 @@ ResultCode refit_bvh(DAabb* nodes, uint32_t node_count, const uint32_t* indices,
       (e = cudaMemsetAsync(status.ptr, 0, 16, s)))
     return cuda_rc(e);
   const unsigned blocks = (node_count + kBlock - 1) / kBlock;
-  k_parents<<<blocks, kBlock, 0, s>>>(nodes, node_count, parent.ptr, arrive.ptr, status.ptr);
+  k_parents<<<blocks, kBlock, 0, s>>>(nodes, node_count, parent.ptr, arrive.ptr, nullptr, nullptr, status.ptr);
   k_refit<<<blocks, kBlock, 0, s>>>(nodes, node_count, indices, index_count, prim_count, aabbs, parent.ptr,
                                     arrive.ptr, status.ptr);
   uint32_t st = 0;
@@ -728,52 +585,10 @@ ResultCode refit_bvh_noalloc(DAabb* nodes, uint32_t node_count, const uint32_t* 
   // clean (k_parents zeroes the arrival counters itself).
   if ((e = cudaMemsetAsync(parent, 0xff, (size_t)node_count * 4, s))) return cuda_rc(e);
   const unsigned blocks = (node_count + kBlock - 1) / kBlock;
-  k_parents<<<blocks, kBlock, 0, s>>>(nodes, node_count, parent, arrive, status);
+  k_parents<<<blocks, kBlock, 0, s>>>(nodes, node_count, parent, arrive, nullptr, nullptr, status);
   k_refit<<<blocks, kBlock, 0, s>>>(nodes, node_count, indices, index_count, prim_count, aabbs, parent, arrive,
                                     status);
   return cuda_rc(cudaGetLastError());
-}
-
-}  // namespace rtbvh
-
-namespace rtbvh {
-
-cudaError_t launch_collapse_segments(const DAabb* nodes, uint32_t node_count, const uint32_t* prim_off,
-                                     const uint32_t* order, uint32_t mesh_count, uint32_t* parent, uint32_t* arrive,
-                                     uint32_t* cnt_e, uint32_t* cnt_o, uint32_t* mbase, uint2* q0, uint2* q1,
-                                     DMNode* mnodes, uint32_t m_capacity, uint32_t* status, unsigned blocks,
-                                     cudaStream_t s) {
-  if (node_count == 0 || mesh_count == 0) return cudaSuccess;
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(parent, 0xff, (size_t)node_count * 4, s))) return e;
-  const unsigned nb = (node_count + kBlock - 1) / kBlock;
-  k_parents<<<nb, kBlock, 0, s>>>(nodes, node_count, parent, arrive, status);
-  k_counts_bottom_up<false><<<nb, kBlock, 0, s>>>(nodes, node_count, parent, arrive, cnt_e, cnt_o, MbvhTriangles(),
-                                                  status);
-  k_seg_mbase<<<1, 1024, 0, s>>>(nodes, cnt_e, prim_off, mesh_count, mbase);
-  SegCollapseParams p;
-  p.c.nodes = nodes;
-  p.c.node_count = node_count;
-  p.c.cnt_e = cnt_e;
-  p.c.mnodes = mnodes;
-  p.c.m_total = m_capacity;
-  p.c.queue[0] = q0;
-  p.c.queue[1] = q1;
-  p.c.qcount = nullptr;
-  p.c.bar = nullptr;
-  p.c.status = status;
-  p.c.ibox = nullptr;
-  p.c.escaped = nullptr;
-  p.c.tboxes = nullptr;
-  p.c.m_total_dev = nullptr;
-  p.prim_off = prim_off;
-  p.order = order;
-  p.mbase = mbase;
-  p.queue[0] = q0;
-  p.queue[1] = q1;
-  p.mesh_count = mesh_count;
-  k_collapse_segments<<<blocks, kBlock, 0, s>>>(p);
-  return cudaGetLastError();
 }
 
 }  // namespace rtbvh
@@ -864,12 +679,7 @@ __device__ bool quantize_axis(const float* mn, const float* mx, float* lo_out, u
   return false;
 }
 
-__global__ void __launch_bounds__(kBlock) k_quantize(const DMNode* __restrict__ in, uint32_t count,
-                                                      const uint32_t* __restrict__ live_count,
-                                                      DQNode* __restrict__ out) {
-  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= count || (live_count && i >= __ldg(live_count))) return;
-  const DMNode m = in[i];
+__device__ void quantize_node(const DMNode& m, DQNode* out) {
   DQNode q;
   uint32_t ex = 0, ey = 0, ez = 0;
   bool ok = quantize_axis(m.min_x, m.max_x, &q.lo[0], &ex, &q.qx[0], &q.qx[1]) &&
@@ -895,19 +705,12 @@ __global__ void __launch_bounds__(kBlock) k_quantize(const DMNode* __restrict__ 
   const uint32_t flags = (ok ? 0u : kQFlagExact) | (in_range ? 0u : kQFlagOutOfRange);
   q.exps = ex | (ey << 8) | (ez << 16) | (flags << 24);
   const float4* src = reinterpret_cast<const float4*>(&q);
-  float4* dst = reinterpret_cast<float4*>(out + i);
+  float4* dst = reinterpret_cast<float4*>(out);
 #pragma unroll
   for (int k = 0; k < 4; ++k) dst[k] = src[k];
 }
 
 }  // namespace
-
-cudaError_t launch_quantize_mbvh(const DMNode* mnodes, uint32_t count, DQNode* qnodes, cudaStream_t s,
-                                 const uint32_t* live_count) {
-  if (count == 0) return cudaSuccess;
-  k_quantize<<<(count + kBlock - 1) / kBlock, kBlock, 0, s>>>(mnodes, count, live_count, qnodes);
-  return cudaGetLastError();
-}
 
 }  // namespace rtbvh
 
@@ -938,189 +741,249 @@ namespace rtbvh {
 namespace {
 
 struct WideParams {
-  const DAabb* nodes;
+  const DAabb* nodes;  // boxes the tree is built over (BVH2, or its boxes from the triangles)
   uint32_t node_count;
+  const uint32_t* parent;
+  const uint2* cnt;     // nodes that are not counted are not below a root
+  uint8_t* opened;      // per interior node: which of its descendants its traversal node would open
+  uint32_t* index;      // per node: its traversal node, kNone for none
+  uint32_t* roots;      // BVH2 node of every traversal node
   DMNode* wnodes;
+  DQNode* wq;
   uint32_t capacity;
-  uint32_t* walloc;   // next free traversal-node index
-  uint2* queue[2];
-  uint32_t* qcount;   // 3 rotating counters
-  GridBarrier* bar;
+  uint32_t* walloc;     // next free traversal-node index (starts at 1; node 0 is BVH2 node 0's)
   uint32_t* status;
-  // optional checks run before the launch: the tree is not collapsed when
-  // check[0] != 0 (boxes that do not nest, or duplicate leaf slots) or,
-  // with expect_seen != UINT32_MAX, when check[1] (primitives seen in
-  // leaves) differs from it
-  const uint32_t* check;
+  // optional checks run before: nothing is built when check[0] != 0 (boxes
+  // that do not nest, or duplicate leaf slots) or, with expect_seen != kNone,
+  // when check[1] (primitives seen in leaves) differs from it
+  uint32_t* check;
   uint32_t expect_seen;
+  bool check_nested;
+  // a forest: index of every mesh's root
+  const uint32_t* prim_off;
+  uint32_t mesh_count;
+  uint32_t* qroot;
 };
 
-// Traversal node wi from BVH2 node c. Interior slots get indices from
-// *alloc (below alloc_end) and are appended to `next` (next_cap entries).
-struct WideCtx {
-  const DAabb* nodes;
-  uint32_t node_count;
-  DMNode* wnodes;
-  uint32_t* alloc;
-  uint32_t alloc_end;
-  uint32_t next_cap;
-  uint32_t* status;
-};
+__device__ __forceinline__ bool interior(const DAabb& b) { return b.count < 0 && b.left_first >= 0; }
 
-// AGG: called by all lanes of a warp (`valid` false for lanes without an
-// item), node indices and queue entries reserved once per warp.
-template <bool AGG>
-__device__ void emit_wide(const WideCtx& p, uint32_t c, uint32_t wi, uint2* next, uint32_t* next_count,
-                          bool valid = true) {
+// A traversal node takes the two children of its BVH2 node as slots 0 and 1
+// and opens up to two slots: each time the interior slot of largest half
+// area (the first one of equals) is replaced by its left child, and the
+// right child is appended. The code of a node: bits 0-1 the first opened slot
+// + 1 (0: none), bits 2-3 the second opened slot + 1.
+__device__ __forceinline__ int largest_interior(const DAabb* box, int ns) {
+  int best = -1;
+  float best_area = -1.0f;
+  for (int i = 0; i < ns; ++i) {
+    if (!interior(box[i])) continue;
+    const float a = half_area(box[i].min[0], box[i].min[1], box[i].min[2], box[i].max[0], box[i].max[1],
+                              box[i].max[2]);
+    if (a > best_area) {
+      best_area = a;
+      best = i;
+    }
+  }
+  return best;
+}
+// Whether code c opens its own child `side`.
+__device__ __forceinline__ bool opens_child(uint32_t c, uint32_t side) {
+  const uint32_t first = c & 3u, second = c >> 2;
+  if (first == 0u) return false;
+  return first == side + 1u || (second == side + 1u && first != side + 1u);
+}
+// Whether code c opens child `side2` of its own child `side`, which only the
+// first opened child's children can be: its left one took its slot, its
+// right one slot 2.
+__device__ __forceinline__ bool opens_grandchild(uint32_t c, uint32_t side, uint32_t side2) {
+  const uint32_t first = c & 3u, second = c >> 2;
+  return first == side + 1u && second == (side2 ? 3u : first);
+}
+
+// The traversal tree without an order between levels. Which nodes a node
+// would open if it had a traversal node of its own depends on the boxes
+// below it alone, so every interior node computes its code at once
+// (k_wide_open). A node then is the root of a traversal node (state R),
+// opened by its parent (O1) or opened by its grandparent (O2), and its state
+// follows from its parent's: R -> opens_child(parent) ? O1 : R,
+// O1 -> opens_grandchild(grandparent) ? O2 : R, O2 -> R (a traversal node
+// reaches three levels down at most). k_place composes these steps up to the
+// first node whose step is the same from every state -- two or three levels
+// on average -- and numbers the roots; k_wide_emit writes their nodes.
+// What bounds it is the node reads, L2 for the most part; the level-by-level
+// frontier it replaces spent a grid barrier per level: 200k sphere triangles
+// 195 us, now k_wide_open 10, its part of k_place, k_wide_emit 15 us; 4M
+// clustered 414 + 84 (compact nodes), now 93 and 167 us.
+__global__ void __launch_bounds__(kBlock) k_wide_open(WideParams p) {
+  const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
+  if (c >= p.node_count) return;
+  const bool below_root = counted(__ldg(p.cnt + c));
+  if (!below_root && !p.check_nested) return;
+  const DAabb cur = load_aabb(p.nodes + c);
+  if (!interior(cur)) return;
+  const uint32_t lf = (uint32_t)cur.left_first;
+  if (lf + 1u >= p.node_count) {
+    if (p.check_nested) atomicOr(p.check, 1u);
+    return;
+  }
+  DAabb box[4];
+  box[0] = load_aabb(p.nodes + lf);
+  box[1] = load_aabb(p.nodes + lf + 1u);
+  // Nesting check: every interior node's box contains both children's boxes.
+  // The traversal tree finds the nearest hit only if the boxes it reads
+  // contain their triangles, which holds for nested trees (leaf boxes are
+  // always built from their primitives). A binned-SAH tree can violate it:
+  // the reference sizes a left child's box from the bins before
+  // best_splits[axis].count, a primitive count, instead of the split bin
+  // (src/builders/binned_sah.rs), so the reference's own traversal can miss
+  // hits there, and only its exact node order reproduces them.
+  if (p.check_nested && !(box_contains(cur, box[0]) && box_contains(cur, box[1]))) atomicOr(p.check, 1u);
+  if (!below_root) return;
+  const int first = largest_interior(box, 2);
+  int second = -1;
+  if (first >= 0) {
+    const uint32_t l2 = (uint32_t)box[first].left_first;
+    if (l2 + 1u < p.node_count) {
+      box[first] = load_aabb(p.nodes + l2);
+      box[2] = load_aabb(p.nodes + l2 + 1u);
+      second = largest_interior(box, 3);
+    }
+  }
+  p.opened[c] = (uint8_t)((first + 1) | ((second + 1) << 2));
+}
+
+__device__ bool wide_checks_failed(const WideParams& p) {
+  if (!p.check) return false;
+  return __ldg(p.check) != 0u || (p.expect_seen != kNone && __ldg(p.check + 1) != p.expect_seen);
+}
+
+// Whether node x (below a root) is the root of a traversal node.
+__device__ bool wide_root(const WideParams& p, uint32_t x) {
+  // f: state of the current node -> x is in state R, one bit per state R, O1, O2
+  uint32_t f = 1u;
+  uint32_t cur = x;
+  for (uint32_t k = 0; k < p.node_count; ++k) {
+    const uint32_t w = __ldg(p.parent + cur);
+    if (w == kNone) break;  // a tree's root: state R
+    const uint32_t par = parent_of(w), side = w & 1u;
+    const uint32_t gw = __ldg(p.parent + par);
+    const bool a = opens_child(p.opened[par], side);
+    const bool b = gw != kNone && opens_grandchild(p.opened[parent_of(gw)], gw & 1u, side);
+    const uint32_t r = f & 1u, o1 = (f >> 1) & 1u, o2 = (f >> 2) & 1u;
+    // state of the parent R, O1, O2 -> state of cur
+    f = (a ? o1 : r) | ((b ? o2 : r) << 1) | (r << 2);
+    if (f == 0u || f == 7u) break;
+    cur = par;
+  }
+  return (f & 1u) != 0u;
+}
+
+// One thread per BVH2 node: places the interior ones (and the roots), lists
+// the quad nodes among them by index and, with WIDE, numbers and lists the
+// roots of traversal nodes.
+template <bool TRIS, bool WIDE>
+__global__ void __launch_bounds__(kBlock) k_place(CollapseParams p, WideParams q) {
+  __shared__ uint32_t s_warp[kBlock / 32];
+  __shared__ uint32_t s_base;
+  const uint32_t x = blockIdx.x * kBlock + threadIdx.x;
+  bool placed = x < p.node_count && counted(__ldg(p.cnt + x));
+  if (placed) {
+    const bool leaf = __ldg(&p.nodes[x].count) >= 0;
+    placed = !leaf || (__ldg(p.parent + x) == kNone && ld_place(p.known + x).x != kNone);
+  }
+  if (placed) {
+    const Place pl = find_place<TRIS>(p, x);
+    placed = pl.ok;  // else not below a root
+    if (placed) {
+      st_place(p.known + x, make_uint2(pl.pos << 1 | pl.parity, pl.bad));
+      if (pl.parity == 0u) {
+        if (pl.pos < p.m_total) p.quads[pl.pos] = x;
+        else atomicOr(p.status, kStatusBadIndex);
+      }
+    }
+  }
+  if (!WIDE) return;
+  if (wide_checks_failed(q)) return;  // the same words for every block
+  const bool root = placed && wide_root(q, x);
+  // node 0 has traversal node 0 (the counter starts at 1)
+  const uint32_t mine = root && x != 0u ? 1u : 0u;
+  uint32_t total;
+  const uint32_t incl = block_inclusive_scan<kBlock>(mine, s_warp, &total);
+  if (threadIdx.x == 0) s_base = total ? atomicAdd(q.walloc, total) : 0u;
+  __syncthreads();
+  if (x >= p.node_count) return;
+  const uint32_t wi = !root ? kNone : (mine ? s_base + incl - 1u : 0u);
+  q.index[x] = wi;
+  if (!root) return;
+  if (wi < q.capacity) q.roots[wi] = x;
+  else atomicOr(p.status, kStatusBadIndex);
+}
+
+__global__ void __launch_bounds__(kBlock) k_wide_emit(WideParams p) {
+  if (wide_checks_failed(p)) return;
+  const uint32_t wi = blockIdx.x * kBlock + threadIdx.x;
+  for (uint32_t m = wi; m < p.mesh_count; m += gridDim.x * kBlock)
+    p.qroot[m] = __ldg(p.index + 2u * __ldg(p.prim_off + m) - m);
+  if (wi >= min(__ldg(p.walloc), p.capacity)) return;
+  const uint32_t c = __ldg(p.roots + wi);
+  if (c >= p.node_count) {  // not listed: only after another error
+    atomicOr(p.status, kStatusBadIndex);
+    return;
+  }
   uint32_t slot[4];
   DAabb box[4];
   int ns = 0;
-  bool ok = valid;
   const DAabb cur = load_aabb(p.nodes + c);
-  if (!ok) {
-  } else if (cur.count >= 0 || cur.left_first < 0) {
+  if (!interior(cur)) {  // a root leaf
     slot[0] = c;
     box[0] = cur;
     ns = 1;
-  } else if ((uint32_t)cur.left_first + 1u < p.node_count) {
+  } else {
     slot[0] = (uint32_t)cur.left_first;
     slot[1] = slot[0] + 1u;
     box[0] = load_aabb(p.nodes + slot[0]);
     box[1] = load_aabb(p.nodes + slot[1]);
     ns = 2;
-    while (ns < 4) {
-      int best = -1;
-      float best_area = -1.0f;
-      for (int i = 0; i < ns; ++i) {
-        if (box[i].count >= 0 || box[i].left_first < 0) continue;
-        const float a = half_area(box[i].min[0], box[i].min[1], box[i].min[2], box[i].max[0], box[i].max[1],
-                                  box[i].max[2]);
-        if (a > best_area) {
-          best_area = a;
-          best = i;
+    const uint32_t code = p.opened[c];
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+      const int at = (int)((code >> (2 * o)) & 3u) - 1;
+      if (at < 0) break;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        if (i != at) continue;
+        const uint32_t lf = (uint32_t)box[i].left_first;
+        if (lf + 1u >= p.node_count) {
+          atomicOr(p.status, kStatusBadIndex);
+          return;
         }
+        slot[i] = lf;
+        box[i] = load_aabb(p.nodes + lf);
+        slot[2 + o] = lf + 1u;
+        box[2 + o] = load_aabb(p.nodes + lf + 1u);
       }
-      if (best < 0) break;
-      const uint32_t lf = (uint32_t)box[best].left_first;
-      if (lf + 1u >= p.node_count) {
-        atomicOr(p.status, kStatusBadIndex);
-        break;
-      }
-      slot[best] = lf;
-      box[best] = load_aabb(p.nodes + lf);
-      slot[ns] = lf + 1u;
-      box[ns] = load_aabb(p.nodes + lf + 1u);
       ++ns;
     }
-  } else {
-    atomicOr(p.status, kStatusBadIndex);
-    ok = false;
-  }
-  uint32_t n_int = 0;
-  if (ok)
-    for (int i = 0; i < ns; ++i) n_int += (box[i].count < 0 && box[i].left_first >= 0) ? 1u : 0u;
-  uint32_t base = 0, qbase = 0;
-  if (AGG) {
-    base = warp_reserve(p.alloc, n_int);
-    qbase = warp_reserve(next_count, n_int);
-  } else if (n_int) {
-    base = atomicAdd(p.alloc, n_int);
-    qbase = atomicAdd(next_count, n_int);
-  }
-  if (!ok) return;
-  if (n_int && base + n_int > p.alloc_end) {
-    atomicOr(p.status, kStatusBadIndex);
-    return;
   }
   DMNode m;
-  uint32_t k = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const DAabb& b = box[i < ns ? i : 0];
+    const DAabb& b = i < ns ? box[i] : box[0];
     m.min_x[i] = b.min[0]; m.min_y[i] = b.min[1]; m.min_z[i] = b.min[2];
     m.max_x[i] = b.max[0]; m.max_y[i] = b.max[1]; m.max_z[i] = b.max[2];
-    if (i >= ns) {
-      m.children[i] = -1;
-      m.counts[i] = -1;
-    } else if (b.count >= 0 || b.left_first < 0) {
+    m.children[i] = -1;
+    m.counts[i] = -1;
+    if (i < ns && !interior(b)) {
       m.children[i] = b.left_first;
       m.counts[i] = b.count;
-    } else {
-      const uint32_t q = qbase + k;
-      const uint32_t child = base + k++;
-      m.children[i] = (int32_t)child;
-      m.counts[i] = -1;
-      if (q < p.next_cap) next[q] = make_uint2(slot[i], child);
+    } else if (i < ns) {
+      const uint32_t child = __ldg(p.index + slot[i]);
+      if (child < p.capacity) m.children[i] = (int32_t)child;
       else atomicOr(p.status, kStatusBadIndex);
     }
   }
-  float4* dst = reinterpret_cast<float4*>(p.wnodes + wi);
-  const float4* src = reinterpret_cast<const float4*>(&m);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) dst[j] = src[j];
-}
-
-__global__ void __launch_bounds__(kBlock) k_wide_collapse(WideParams p) {
-  if (p.check) {  // the same words for every block: all return or none
-    const uint32_t bad = __ldcg(p.check), seen = __ldcg(p.check + 1);
-    if (bad || (p.expect_seen != kNone && seen != p.expect_seen)) return;
-  }
-  const uint32_t G = gridDim.x;
-  const uint32_t tid = blockIdx.x * kBlock + threadIdx.x, nthreads = G * kBlock;
-  WideCtx ctx;
-  ctx.nodes = p.nodes;
-  ctx.node_count = p.node_count;
-  ctx.wnodes = p.wnodes;
-  ctx.alloc = p.walloc;
-  ctx.alloc_end = p.capacity;
-  ctx.next_cap = p.capacity;
-  ctx.status = p.status;
-  for (uint32_t level = 0; level < p.capacity + 1; ++level) {
-    uint32_t size = __ldcg(p.qcount + (level % 3));
-    if (size == 0) break;
-    if (size > p.capacity) size = p.capacity;  // only after a kStatusBadIndex
-    const uint2* q = p.queue[level & 1];
-    uint2* next = p.queue[(level + 1) & 1];
-    uint32_t* next_count = p.qcount + ((level + 1) % 3);
-    // warp-uniform loop: every lane takes part in the reservations
-    for (uint32_t k0 = tid - (threadIdx.x & 31u); k0 < size; k0 += nthreads) {
-      const uint32_t k = k0 + (threadIdx.x & 31u);
-      const bool valid = k < size;
-      const uint2 item = valid ? __ldcg(q + k) : make_uint2(0u, 0u);
-      emit_wide<true>(ctx, item.x, item.y, next, next_count, valid);
-    }
-    if (tid == 0) p.qcount[(level + 2) % 3] = 0;
-    if (!grid_sync(p.bar, G, p.status)) return;
-  }
-}
-
-// Nesting check: every interior node's box contains both children's boxes.
-// The traversal tree finds the nearest hit only if the boxes it reads
-// contain their triangles, which holds for nested trees (leaf boxes are
-// always built from their primitives). A binned-SAH tree can violate it:
-// the reference sizes a left child's box from the bins before
-// best_splits[axis].count, a primitive count, instead of the split bin
-// (src/builders/binned_sah.rs), so the reference's own traversal can miss
-// hits there, and only its exact node order reproduces them.
-__global__ void __launch_bounds__(kBlock) k_check_nested(const DAabb* __restrict__ nodes, uint32_t node_count,
-                                                          uint32_t* __restrict__ not_nested) {
-  const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
-  if (c >= node_count) return;
-  const DAabb n = load_aabb(nodes + c);
-  if (n.count >= 0 || n.left_first < 0) return;
-  const uint32_t lf = (uint32_t)n.left_first;
-  if (lf + 1u >= node_count) {
-    atomicOr(not_nested, 1u);
-    return;
-  }
-  bool ok = true;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const DAabb ch = load_aabb(nodes + lf + k);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) ok = ok && ch.min[a] >= n.min[a] && ch.max[a] <= n.max[a];
-  }
-  if (!ok) atomicOr(not_nested, 1u);
+  store_node(p.wnodes + wi, m);
+  quantize_node(m, p.wq + wi);
 }
 
 // The leaves of the object-split builders hold every index slot once and
@@ -1150,156 +1013,201 @@ __global__ void __launch_bounds__(kBlock) k_check_leaves(const DAabb* __restrict
   }
 }
 
-__global__ void k_wide_init(uint2* queue0, uint32_t* qcount, uint32_t* walloc) {
-  if (threadIdx.x == 0) {
-    queue0[0] = make_uint2(0u, 0u);
-    qcount[0] = 1;
-    qcount[1] = 0;
-    qcount[2] = 0;
-    *walloc = 1;
+}  // namespace
+
+// Scratch words per node of the collapse passes: parent, arrive, cnt (2),
+// known (2), traversal index, the two lists of quad and traversal nodes (a
+// forest of single leaves has as many as nodes), opened codes (a byte,
+// rounded up).
+size_t collapse_scratch_words(size_t node_count) { return 9 * node_count + (node_count + 3) / 4 + 8; }
+
+namespace {
+
+__global__ void k_set_word(uint32_t* p, uint32_t v) { *p = v; }
+
+struct CollapseScratch {
+  uint32_t *parent, *arrive, *index, *quads, *roots;
+  uint2 *cnt, *known;
+  uint8_t* opened;
+  // words holds collapse_scratch_words(node_count) words, 8-byte aligned
+  CollapseScratch(uint32_t* words, size_t n) {
+    cnt = reinterpret_cast<uint2*>(words);
+    known = cnt + n;
+    parent = reinterpret_cast<uint32_t*>(known + n);
+    arrive = parent + n;
+    index = arrive + n;
+    quads = index + n;
+    roots = quads + n;
+    opened = reinterpret_cast<uint8_t*>(roots + n);
   }
+};
+
+// Parents and counts (with `tri` also the boxes from the triangles).
+cudaError_t launch_counts(const DAabb* nodes, uint32_t node_count, const CollapseScratch& w, const MbvhTriangles* tri,
+                          uint32_t* status, cudaStream_t s) {
+  cudaError_t e;
+  if ((e = cudaMemsetAsync(w.parent, 0xff, (size_t)node_count * 4, s))) return e;
+  const unsigned blocks = (node_count + kBlock - 1) / kBlock;
+  k_parents<<<blocks, kBlock, 0, s>>>(nodes, node_count, w.parent, w.arrive, w.cnt, w.known, status);
+  if (tri)
+    k_counts_bottom_up<true><<<blocks, kBlock, 0, s>>>(nodes, node_count, w.parent, w.arrive, w.cnt, *tri, status);
+  else
+    k_counts_bottom_up<false><<<blocks, kBlock, 0, s>>>(nodes, node_count, w.parent, w.arrive, w.cnt,
+                                                        MbvhTriangles(), status);
+  return cudaGetLastError();
 }
 
-// Many meshes: one block per mesh builds the mesh's traversal tree in the
-// node range [off_m, off_m + n_m) (a mesh of n primitives has at most n - 1
-// interior BVH2 nodes), root at off_m, with the frontier in the same range
-// of the two queues.
-__global__ void __launch_bounds__(kBlock)
-    k_wide_segments(const DAabb* __restrict__ nodes, uint32_t node_count, const uint32_t* __restrict__ prim_off,
-                    const uint32_t* __restrict__ order, uint32_t mesh_count, DMNode* wnodes, uint2* q0, uint2* q1,
-                    uint32_t* status) {
-  __shared__ uint32_t s_count[2];
-  __shared__ uint32_t s_alloc;
-  for (uint32_t q = blockIdx.x; q < mesh_count; q += gridDim.x) {
-    const uint32_t m = order[q];
-    const uint32_t off = prim_off[m], n = prim_off[m + 1] - off;
-    if (n == 0) continue;
-    WideCtx ctx;
-    ctx.nodes = nodes;
-    ctx.node_count = node_count;
-    ctx.wnodes = wnodes;
-    ctx.alloc = &s_alloc;
-    ctx.alloc_end = off + n;
-    ctx.next_cap = n;
-    ctx.status = status;
-    if (threadIdx.x == 0) {
-      q0[off] = make_uint2(2u * off - m, off);
-      s_count[0] = 1;
-      s_count[1] = 0;
-      s_alloc = off + 1u;
-    }
-    __syncthreads();
-    int cur = 0;
-    for (uint32_t level = 0; level <= n; ++level) {
-      uint32_t size = s_count[cur];
-      if (size == 0) break;
-      if (size > n) size = n;
-      const uint2* qin = (cur ? q1 : q0) + off;
-      uint2* qout = (cur ? q0 : q1) + off;
-      for (uint32_t k = threadIdx.x; k < size; k += kBlock) {
-        const uint2 item = qin[k];
-        emit_wide<false>(ctx, item.x, item.y, qout, &s_count[cur ^ 1]);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) s_count[cur] = 0;
-      __syncthreads();
-      cur ^= 1;
-    }
-    __syncthreads();
-  }
+// The quad nodes and, with q, the traversal nodes.
+cudaError_t launch_nodes(const CollapseParams& p, bool tris, const WideParams* q, cudaStream_t s) {
+  const unsigned blocks = (p.node_count + kBlock - 1) / kBlock, quad_blocks = (p.m_total + kBlock - 1) / kBlock;
+  if (q) k_wide_open<<<blocks, kBlock, 0, s>>>(*q);
+  auto place = tris ? (q ? k_place<true, true> : k_place<true, false>)
+                    : (q ? k_place<false, true> : k_place<false, false>);
+  place<<<blocks, kBlock, 0, s>>>(p, q ? *q : WideParams());
+  auto quads = tris ? k_quads<true> : k_quads<false>;
+  quads<<<quad_blocks, kBlock, 0, s>>>(p);
+  if (q) k_wide_emit<<<(q->capacity + kBlock - 1) / kBlock, kBlock, 0, s>>>(*q);
+  return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_wide_segments(const DAabb* nodes, uint32_t node_count, const uint32_t* prim_off,
-                                 const uint32_t* order, uint32_t mesh_count, uint32_t total_prims, DMNode* wnodes,
-                                 DQNode* wq, uint2* q0, uint2* q1, uint32_t* status, unsigned blocks, cudaStream_t s) {
-  if (mesh_count == 0 || total_prims == 0) return cudaSuccess;
-  k_wide_segments<<<blocks, kBlock, 0, s>>>(nodes, node_count, prim_off, order, mesh_count, wnodes, q0, q1, status);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  // slots of a mesh's range past its own tree are converted too and never read
-  return launch_quantize_mbvh(wnodes, total_prims, wq, s);
-}
-
-ResultCode build_wide(const DAabb* nodes, uint32_t node_count, const uint32_t* indices, uint32_t index_count,
-                      cudaStream_t s, DMNode** wnodes_out, DQNode** wq_out, uint32_t* wcount, bool nested) {
-  *wnodes_out = nullptr;
-  *wq_out = nullptr;
-  *wcount = 0;
-  if (node_count == 0) return Ok;
-  // one traversal node per BVH2 interior node at most, or the root leaf
-  const uint32_t capacity = node_count < 3u ? 1u : (node_count + 1u) / 2u;
+cudaError_t launch_collapse_forest(const DAabb* nodes, uint32_t node_count, const uint32_t* prim_off,
+                                   uint32_t mesh_count, uint32_t total_prims, uint32_t* scratch, uint32_t* mbase,
+                                   DMNode* mnodes, DMNode* wnodes, DQNode* wq, uint32_t* qroot, uint32_t* walloc,
+                                   uint32_t* status, cudaStream_t s) {
+  if (node_count == 0 || mesh_count == 0) return cudaSuccess;
   cudaError_t e;
-  Scratch<uint32_t> status, qcount, walloc;
-  Scratch<uint2> q0, q1;
-  Scratch<GridBarrier> bar;
-  if ((e = status.alloc(4, s)) || (e = qcount.alloc(4, s)) || (e = walloc.alloc(1, s)) || (e = q0.alloc(capacity, s)) ||
-      (e = q1.alloc(capacity, s)) || (e = bar.alloc(1, s)))
-    return cuda_rc(e);
-  DMNode* wn = nullptr;
-  DQNode* wq = nullptr;
-  auto fail = [&](ResultCode rc) {
-    pool_free(wn, s);
-    pool_free(wq, s);
-    return rc;
-  };
-  if ((e = device_alloc(&wn, capacity, s))) return fail(cuda_rc(e));
-  if ((e = cudaMemsetAsync(status.ptr, 0, 16, s)) || (e = cudaMemsetAsync(bar.ptr, 0, sizeof(GridBarrier), s)))
-    return fail(cuda_rc(e));
-  const unsigned node_blocks = (node_count + kBlock - 1) / kBlock;
-  // status[1]: not nested, or leaves that are not whole primitives once
-  // each -> no traversal tree (closest hit uses the exact nodes); the
-  // collapse reads the result on the device and does nothing then
-  const bool checked = !nested || indices;
-  Scratch<uint32_t> seen;
-  if (checked) {
-    if (!nested) k_check_nested<<<node_blocks, kBlock, 0, s>>>(nodes, node_count, status.ptr + 1);
-    if (indices) {
-      if ((e = seen.alloc(index_count, s)) || (e = cudaMemsetAsync(seen.ptr, 0, (size_t)index_count * 4, s)))
-        return fail(cuda_rc(e));
-      k_check_leaves<<<node_blocks, kBlock, 0, s>>>(nodes, node_count, indices, index_count, seen.ptr, status.ptr + 2,
-                                                    status.ptr + 1);
-    }
-  }
-  k_wide_init<<<1, 32, 0, s>>>(q0.ptr, qcount.ptr, walloc.ptr);
-  int per_sm = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_wide_collapse, kBlock, 0);
-  if (per_sm < 1) per_sm = 1;
-  unsigned grid = (unsigned)(sm_count() * per_sm);
-  const unsigned useful = (capacity + kBlock - 1) / kBlock;
-  if (grid > useful) grid = useful;
-  if (grid < 1) grid = 1;
-  WideParams p;
+  const CollapseScratch w(scratch, node_count);
+  if ((e = launch_counts(nodes, node_count, w, nullptr, status, s))) return e;
+  k_seg_mbase<<<1, 1024, 0, s>>>(nodes, w.cnt, prim_off, mesh_count, w.known, mbase);
+  CollapseParams p = {};
   p.nodes = nodes;
   p.node_count = node_count;
-  p.wnodes = wn;
-  p.capacity = capacity;
-  p.walloc = walloc.ptr;
-  p.queue[0] = q0.ptr;
-  p.queue[1] = q1.ptr;
-  p.qcount = qcount.ptr;
-  p.bar = bar.ptr;
-  p.status = status.ptr;
-  p.check = checked ? status.ptr + 1 : nullptr;
-  p.expect_seen = indices ? index_count : kNone;
-  void* args[] = {&p};
-  if ((e = cudaLaunchCooperativeKernel((void*)k_wide_collapse, dim3(grid), dim3(kBlock), args, 0, s)))
-    return fail(cuda_rc(e));
-  // compact nodes for the live part of the tree (the node count is read on
-  // the device), then one readback for everything
-  if ((e = device_alloc(&wq, capacity, s))) return fail(cuda_rc(e));
-  if ((e = launch_quantize_mbvh(wn, capacity, wq, s, walloc.ptr))) return fail(cuda_rc(e));
-  uint32_t h[4] = {0, 0, 0, 0};
-  if ((e = cudaMemcpyAsync(h, walloc.ptr, 4, cudaMemcpyDeviceToHost, s)) ||
-      (e = cudaMemcpyAsync(h + 1, status.ptr, 12, cudaMemcpyDeviceToHost, s)) || (e = cudaStreamSynchronize(s)))
-    return fail(cuda_rc(e));
-  if (checked && (h[2] || (indices && h[3] != index_count))) return fail(Ok);
-  if (h[1] != 0) return fail((h[1] & kStatusTimeout) ? Timeout : Error);
-  if (h[0] == 0 || h[0] > capacity) return fail(Error);
-  *wnodes_out = wn;
-  *wq_out = wq;
-  *wcount = h[0];
+  p.parent = w.parent;
+  p.cnt = w.cnt;
+  p.known = w.known;
+  p.quads = w.quads;
+  p.mnodes = mnodes;
+  p.m_total = total_prims;  // a mesh of n > 1 primitives has at most n - 1 interior nodes
+  p.m_count = mbase + mesh_count;
+  p.forest = true;
+  p.status = status;
+  if (!wnodes) return launch_nodes(p, false, nullptr, s);
+  WideParams q = {};
+  q.nodes = nodes;
+  q.node_count = node_count;
+  q.parent = w.parent;
+  q.cnt = w.cnt;
+  q.opened = w.opened;
+  q.index = w.index;
+  q.roots = w.roots;
+  q.wnodes = wnodes;
+  q.wq = wq;
+  q.capacity = total_prims;
+  q.walloc = walloc;
+  q.status = status;
+  q.expect_seen = kNone;
+  q.prim_off = prim_off;
+  q.mesh_count = mesh_count;
+  q.qroot = qroot;
+  k_set_word<<<1, 1, 0, s>>>(walloc, 1u);
+  return launch_nodes(p, false, &q, s);
+}
+
+ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, const MbvhRequest& req, MbvhOutput* out) {
+  *out = MbvhOutput();
+  if (node_count == 0) return Ok;  // Mbvh::default()
+  const MbvhTriangles* tri = req.tri;
+  if (tri && (!tri->indices || !tri->vertices || !tri->tris || !tri->tb)) return Error;
+  // The node counts stay on the device until the end; arrays are sized by
+  // their bounds: quad nodes are interior BVH2 nodes, at most
+  // (node_count - 1) / 2 of a binary tree, or the root leaf; the same holds
+  // for traversal nodes.
+  const uint32_t m_cap = (node_count + 1u) / 2u;
+  const bool check_nested = req.wide && !tri;
+  const uint32_t* check_indices = req.wide ? req.check_indices : nullptr;
+  cudaError_t e;
+  Scratch<uint32_t> words, seen;
+  // result words: 0 status, 1 check (not nested, duplicate leaf slots), 2
+  // primitives in leaves, 3 escaped triangles, 4 quad nodes, 5 traversal nodes
+  Scratch<uint32_t> res;
+  if ((e = words.alloc(collapse_scratch_words(node_count), s)) || (e = res.alloc(8, s))) return cuda_rc(e);
+  auto drop = [&](ResultCode rc) {
+    pool_free(out->mnodes, s);
+    pool_free(out->tboxes, s);
+    pool_free(out->wnodes, s);
+    pool_free(out->wq, s);
+    *out = MbvhOutput();
+    return rc;
+  };
+  if ((e = device_alloc(&out->mnodes, m_cap, s))) return drop(cuda_rc(e));
+  if (tri && (e = device_alloc(&out->tboxes, m_cap, s))) return drop(cuda_rc(e));
+  if (req.wide && ((e = device_alloc(&out->wnodes, m_cap, s)) || (e = device_alloc(&out->wq, m_cap, s))))
+    return drop(cuda_rc(e));
+  if ((e = cudaMemsetAsync(res.ptr, 0, 32, s))) return drop(cuda_rc(e));
+  const CollapseScratch w(words.ptr, node_count);
+  if ((e = launch_counts(nodes, node_count, w, tri, res.ptr, s))) return drop(cuda_rc(e));
+  const unsigned blocks = (node_count + kBlock - 1) / kBlock;
+  k_root_place<<<1, 32, 0, s>>>(w.cnt, nodes, w.known, m_cap, res.ptr + 4, res.ptr + 5, res.ptr);
+  CollapseParams p = {};
+  p.nodes = nodes;
+  p.node_count = node_count;
+  p.parent = w.parent;
+  p.cnt = w.cnt;
+  p.known = w.known;
+  p.quads = w.quads;
+  p.mnodes = out->mnodes;
+  p.m_total = m_cap;
+  p.m_count = res.ptr + 4;
+  p.status = res.ptr;
+  if (tri) p.tri = *tri;
+  p.escaped = res.ptr + 3;
+  p.tboxes = out->tboxes;
+  if (!req.wide) {
+    if ((e = launch_nodes(p, tri != nullptr, nullptr, s))) return drop(cuda_rc(e));
+  } else {
+    if (check_indices) {
+      if ((e = seen.alloc(req.index_count, s)) || (e = cudaMemsetAsync(seen.ptr, 0, (size_t)req.index_count * 4, s)))
+        return drop(cuda_rc(e));
+      k_check_leaves<<<blocks, kBlock, 0, s>>>(nodes, node_count, check_indices, req.index_count, seen.ptr,
+                                               res.ptr + 2, res.ptr + 1);
+    }
+    WideParams q = {};
+    q.nodes = tri ? tri->tb : nodes;
+    q.node_count = node_count;
+    q.parent = w.parent;
+    q.cnt = w.cnt;
+    q.opened = w.opened;
+    q.index = w.index;
+    q.roots = w.roots;
+    q.wnodes = out->wnodes;
+    q.wq = out->wq;
+    q.capacity = m_cap;
+    q.walloc = res.ptr + 5;
+    q.status = res.ptr;
+    q.check = res.ptr + 1;
+    q.check_nested = check_nested;
+    q.expect_seen = check_indices ? req.index_count : kNone;
+    if ((e = launch_nodes(p, tri != nullptr, &q, s))) return drop(cuda_rc(e));
+  }
+  uint32_t h[6];
+  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(h, res.ptr, 24, cudaMemcpyDeviceToHost, s)) ||
+      (e = cudaStreamSynchronize(s)))
+    return drop(cuda_rc(e));
+  if (h[0] != 0) return drop((h[0] & kStatusTimeout) ? Timeout : Error);
+  out->mcount = h[4];
+  out->escaped = h[3];
+  if (req.wide && (h[1] || (check_indices && h[2] != req.index_count))) {
+    // no traversal tree: closest hit reads the exact nodes
+    pool_free(out->wnodes, s);
+    pool_free(out->wq, s);
+    out->wnodes = nullptr;
+    out->wq = nullptr;
+  } else if (req.wide) {
+    out->wcount = h[5];
+    if (out->wcount == 0 || out->wcount > m_cap) return drop(Error);
+  }
   return Ok;
 }
 
