@@ -350,7 +350,7 @@ ResultCode rtbvh_gpu_batch_create(const float* vertices, const uint32_t* prim_of
   for (uint32_t q = 0; q < mesh_count; ++q) p->sizes_in_order[q] = prim_offsets[order[q] + 1] - prim_offsets[order[q]];
   set_cluster_min(*p, kSegClusterMinPrims);
   cudaError_t e;
-  if ((e = p->cluster_sums.alloc((size_t)kSegCluster * std::min<uint32_t>(mesh_count, kMaxClusters))) ||
+  if ((e = p->cluster_sums.alloc((size_t)kSegCluster * std::min<uint32_t>(mesh_count, kMaxClusters) + mesh_count)) ||
       (e = cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking)) ||
       (e = cudaEventCreateWithFlags(&p->fork, cudaEventDisableTiming)) ||
       (e = cudaEventCreateWithFlags(&p->join, cudaEventDisableTiming)))

@@ -264,9 +264,12 @@ cudaError_t launch_trace_packets(const PacketArgs& a, bool mbvh, cudaStream_t s)
 // Per-mesh clustering of a concatenated forest (see locb.cu).
 // Meshes order[0, big_count) (the largest, more than kSegClusterMinPrims
 // primitives) are clustered by `clusters` thread-block clusters of
-// kSegCluster blocks (cluster_sums: kSegCluster words per cluster); the rest
-// by up to `blocks` single blocks, on `side` (between the events fork and
-// join) when it is given.
+// kSegCluster blocks; the rest by up to `blocks` single blocks, on `side`
+// (between the events fork and join) when it is given. cluster_sums:
+// kSegCluster words per cluster and a word per mesh. Eight blocks per
+// cluster: 16 are faster for a few large meshes (8 of up to 200k primitives
+// 1.73 against 2.07 ms, build and trace) and slower for many (512 of them 62.8
+// against 60.2 ms), 4 are slower for 64 (9.7 against 8.5 ms).
 constexpr uint32_t kSegCluster = 8;
 constexpr uint32_t kSegClusterMinPrims = 4096;  // default threshold (RTBatchTuning::cluster_min_prims)
 cudaError_t launch_locb_segments(const DAabb* aabbs, const uint32_t* sorted, uint32_t* indices,
