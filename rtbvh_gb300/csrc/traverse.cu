@@ -492,6 +492,15 @@ __device__ __forceinline__ void slot_key(float tn, float tx, float t, int32_t ch
 }
 
 
+// q0 * a + b and q1 * a + b in one instruction (two fmas, rounded as fmaf).
+__device__ __forceinline__ void fma2(float q0, float q1, float a, float b, float& r0, float& r1) {
+  asm("{\n\t.reg .b64 q, f, c, r;\n\t"
+      "mov.b64 q, {%2, %3};\n\tmov.b64 f, {%4, %4};\n\tmov.b64 c, {%5, %5};\n\t"
+      "fma.rn.f32x2 r, q, f, c;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r0), "=f"(r1)
+      : "f"(q0), "f"(q1), "f"(a), "f"(b));
+}
+
 // The slab test of quad_intersect<true> on a compact node: the plane of step
 // q is at lo + q * step, so its ray parameter is q * (step * inv) +
 // (lo - o) * inv (one fma). With a negative inverse direction the upper
@@ -522,11 +531,22 @@ __device__ __forceinline__ void slot_keys_q(const float (&h0)[8], const float (&
   ch[1] = __float_as_int(h1[3]);
   ch[2] = __float_as_int(h1[4]);
   ch[3] = __float_as_int(h1[5]);
+  // two slots per instruction: 12 issue slots fewer per node, 2 % on every
+  // kind of rays
+  float nx[4], ny[4], nz[4], fx[4], fy[4], fz[4];
+#pragma unroll
+  for (int i = 0; i < 4; i += 2) {
+    fma2(qbyte(xn, i), qbyte(xn, i + 1), ax, bx, nx[i], nx[i + 1]);
+    fma2(qbyte(yn, i), qbyte(yn, i + 1), ay, by, ny[i], ny[i + 1]);
+    fma2(qbyte(zn, i), qbyte(zn, i + 1), az, bz, nz[i], nz[i + 1]);
+    fma2(qbyte(xf, i), qbyte(xf, i + 1), ax, bx, fx[i], fx[i + 1]);
+    fma2(qbyte(yf, i), qbyte(yf, i + 1), ay, by, fy[i], fy[i + 1]);
+    fma2(qbyte(zf, i), qbyte(zf, i + 1), az, bz, fz[i], fz[i + 1]);
+  }
   leaves = 0;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float tn = fmaxf(fmaf(qbyte(xn, i), ax, bx), fmaxf(fmaf(qbyte(yn, i), ay, by), fmaf(qbyte(zn, i), az, bz)));
-    const float tx = fminf(fmaf(qbyte(xf, i), ax, bx), fminf(fmaf(qbyte(yf, i), ay, by), fmaf(qbyte(zf, i), az, bz)));
+    const float tn = fmaxf(nx[i], fmaxf(ny[i], nz[i])), tx = fminf(fx[i], fminf(fy[i], fz[i]));
     const bool inner = (ct[i >> 1] & (0x8000u << (16 * (i & 1)))) != 0u;
     slot_key(tn, tx, t, ch[i], inner, i, key[i], leaves);
     ich[i] = ch[i];
