@@ -682,8 +682,15 @@ __global__ void __launch_bounds__(kBlock, 9) k_trace_compact(TraceArgs a, unsign
     active = true;
   };
   for (;;) {
-    if (!pool.exhausted) pool.refill(active, batch, ray_count, work, start_ray);
-    const uint32_t amask = __ballot_sync(0xffffffffu, active);
+    // refill once four lanes are idle: the ray set-up runs for the refilled
+    // lanes only (and finds each ray's mesh in a forest). Two idle lanes: 64
+    // meshes 7.67 instead of 7.33 ms, camera rays over 200k triangles +2 %,
+    // incoherent rays +1 %; eight: incoherent +3 %.
+    uint32_t amask = __ballot_sync(0xffffffffu, active);
+    if (!pool.exhausted && __popc(amask) <= 28) {
+      pool.refill(active, batch, ray_count, work, start_ray);
+      amask = __ballot_sync(0xffffffffu, active);
+    }
     if (!amask) {
       if (pool.exhausted) break;
       continue;
