@@ -219,6 +219,7 @@ struct TraceArgs {
   uint32_t* walk_stats = nullptr;
   // Internal: the ray count is read from this device word (at most ray_count).
   const unsigned int* ray_count_dev = nullptr;
+  uint32_t sms = 0;  // with ray_count_dev: SMs of the device
 };
 cudaError_t launch_trace_mbvh(const TraceArgs& a, cudaStream_t s);
 cudaError_t launch_trace_bvh(const TraceArgs& a, cudaStream_t s);

@@ -282,6 +282,284 @@ __device__ __forceinline__ uint32_t subtree_mask(const DTBox* box, const RayStat
   return m;
 }
 
+// ------------------------------------------------------------------ four lanes per ray
+// Few rays leave most of the GPU idle and the launch as long as its longest
+// walk: then four neighbouring lanes take a ray together, one slot of a node
+// each, which shortens a node visit to the test of one slot and a few
+// shuffles. The visits, their order and the result are those of the walks
+// with a lane per ray: the slots go through the same sorting network, lane by
+// lane, and where the leaves of one node are tested side by side, a hit counts
+// if no leaf before it in the walk's order has a nearer one.
+// The stack is the four lanes' in shared memory.
+struct FourLanes {
+  uint32_t first;  // lane 0 of the four
+  uint32_t l;      // this lane of the four
+  __device__ __forceinline__ FourLanes() : first(threadIdx.x & 28u), l(threadIdx.x & 3u) {}
+  template <class T>
+  __device__ __forceinline__ T from(T v, uint32_t k) const {
+    return __shfl_sync(0xffffffffu, v, (int)(first + k));
+  }
+  __device__ __forceinline__ uint32_t ballot(bool b) const {
+    return (__ballot_sync(0xffffffffu, b) >> first) & 15u;
+  }
+};
+
+// Warps that `rays` rays are spread over, at most eight to a warp: about
+// kFewWarpsPerScheduler for each of an SM's four schedulers as long as there
+// are rays for that many. Ray i goes to warp i % warps.
+constexpr uint32_t kFewWarpsPerScheduler = 3;
+// Launches of at most so many rays take four lanes per ray. Closest hit, one
+// lane against four, in us: 4,096 rays 102 / 76 (6,400-triangle sphere, SAH),
+// 246 / 226 (200k soup, LOCB), 301 / 224 (300k clustered, SAH); 16,384: 111 /
+// 98, 264 / 255, 315 / 245; 32,768: 102 / 78, 273 / 298, 317 / 261. Any hit
+// (300k clustered): 4,096 rays 194 / 132, 65,536: 281 / 235, 131,072: 301 /
+// 319. Rays handed on by the compact walk come from binned-SAH trees.
+constexpr uint32_t kFewClosest = 20480, kFewAny = 65536, kFewDeferred = 32768;
+__device__ __host__ __forceinline__ uint32_t few_warps(uint32_t rays, uint32_t sms) {
+  const uint32_t spread = sms * 4u * kFewWarpsPerScheduler;
+  const uint32_t least = (rays + 7u) / 8u;
+  return least > spread ? least : (rays < spread ? rays : spread);
+}
+
+// Best of the four lanes' hits of one node: t is every lane's nearest t (the
+// entry t where it has none). HIGH_FIRST: the walk tests the leaves of higher
+// lanes first, else those of lower lanes. Returns the lane of the first
+// nearest hit, -1 for none below `entry`, and the nearest t of the lanes
+// before this one.
+template <bool HIGH_FIRST>
+__device__ __forceinline__ int first_nearest(const FourLanes& q, float t, float entry, float& best, float& before) {
+  const float t0 = q.from(t, 0), t1 = q.from(t, 1), t2 = q.from(t, 2), t3 = q.from(t, 3);
+  best = fminf(fminf(t0, t1), fminf(t2, t3));
+  before = entry;
+  if (HIGH_FIRST) {
+    if (q.l < 3u) before = fminf(before, t3);
+    if (q.l < 2u) before = fminf(before, t2);
+    if (q.l < 1u) before = fminf(before, t1);
+  } else {
+    if (q.l > 0u) before = fminf(before, t0);
+    if (q.l > 1u) before = fminf(before, t1);
+    if (q.l > 2u) before = fminf(before, t2);
+  }
+  if (!(best < entry)) return -1;
+  if (HIGH_FIRST) return t3 == best ? 3 : (t2 == best ? 2 : (t1 == best ? 1 : 0));
+  return t0 == best ? 0 : (t1 == best ? 1 : (t2 == best ? 2 : 3));
+}
+
+constexpr int kCullNone = 0, kCullSubtree = 1, kCullBehind = 2;  // see k_trace_mbvh
+
+// Whether slots may be skipped for this ray.
+template <int CULL>
+__device__ __forceinline__ bool cull_ray(const TraceArgs& a, const RayState& ray) {
+  const DAabb root = load_aabb(a.nodes);
+  // |x| <= bound is false for NaN and infinities
+  bool cull = fabsf(ray.ox) <= kCompactRange && fabsf(ray.oy) <= kCompactRange && fabsf(ray.oz) <= kCompactRange &&
+              fabsf(ray.dx) <= 3.0e38f && fabsf(ray.dy) <= 3.0e38f && fabsf(ray.dz) <= 3.0e38f &&
+              fabsf(ray.ix) <= kQuantRange && fabsf(ray.iy) <= kQuantRange && fabsf(ray.iz) <= kQuantRange;
+  if (CULL == kCullSubtree) {
+    // Only rays that start inside the scene's root box: boxes behind
+    // them are most of what the cull saves; for rays from outside the
+    // extra box loads cost more than they save
+    cull = cull && ray.ox >= root.min[0] && ray.oy >= root.min[1] && ray.oz >= root.min[2] &&
+           ray.ox <= root.max[0] && ray.oy <= root.max[1] && ray.oz <= root.max[2];
+  } else {
+    // the margin argument needs the boxes within the range too
+    for (int k = 0; k < 3; ++k) cull = cull && root.min[k] >= -kCompactRange && root.max[k] <= kCompactRange;
+  }
+  return cull;
+}
+
+// Start of ray r's walk over the quad nodes: the root (of its mesh); false:
+// no nodes, a miss.
+__device__ __forceinline__ bool mbvh_root(const TraceArgs& a, uint32_t r, int32_t& root) {
+  root = 0;
+  if (a.node_count == 0) return false;
+  if (a.seg_count) {
+    const uint32_t m = ray_mesh(a, r);
+    root = (int32_t)__ldg(a.seg_root + m);
+    if ((uint32_t)root == __ldg(a.seg_root + m + 1)) return false;
+  }
+  return true;
+}
+
+// One lane's slot of a quad node.
+struct LaneQuad {
+  float x0, x1, y0, y1, z0, z1;
+  int32_t child, count;
+  __device__ __forceinline__ void load(const DMNode* node, uint32_t l) {
+    const float* n = reinterpret_cast<const float*>(node) + l;
+    x0 = __ldg(n);
+    x1 = __ldg(n + 4);
+    y0 = __ldg(n + 8);
+    y1 = __ldg(n + 12);
+    z0 = __ldg(n + 16);
+    z1 = __ldg(n + 20);
+    child = __float_as_int(__ldg(n + 24));
+    count = __float_as_int(__ldg(n + 28));
+  }
+};
+
+// k_trace_mbvh's walk, four lanes per ray, for ray_count rays; s_stack: the
+// block's stacks. The next node is popped and asked for before the leaves are
+// tested.
+template <bool ANY_HIT, int CULL>
+__device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warps, int32_t (*s_stack)[kStack]) {
+  const FourLanes q;
+  int32_t* stack = s_stack[threadIdx.x >> 2];
+  const uint32_t warp = blockIdx.x * (kBlock / 32u) + (threadIdx.x >> 5);
+  RayState ray;
+  float hu = 0.0f, hv = 0.0f;
+  int32_t prim = -1, current = -1;  // the node whose slots are in `slot`
+  int sp = -1;
+  bool active = false, fast = true, cull = false;
+  uint32_t r = 0;
+  LaneQuad slot;
+  auto fetch = [&]() {
+    if ((uint32_t)current >= a.node_count) {
+      if (q.l == 0u) atomicOr(a.status, kStatusBadIndex);
+      active = false;
+    } else {
+      slot.load(a.mnodes + current, q.l);
+    }
+  };
+  for (size_t i = warp < warps ? warp + (size_t)warps * (q.first >> 2) : ray_count;;) {
+    if (!active && i < ray_count) {
+      r = a.order ? __ldg(a.order + i) : (uint32_t)i;
+      i += 8u * (size_t)warps;
+      ray = load_ray(a.rays, r, a.t_max);
+      fast = finite_ray(ray);
+      if (CULL != kCullNone && a.node_count > 0) cull = cull_ray<CULL>(a, ray);
+      hu = hv = 0.0f;
+      prim = -1;
+      sp = -1;
+      active = mbvh_root(a, r, current);
+      if (active) fetch();
+      else if (q.l == 0u) a.hits[r] = make_float4(ray.t, 0.0f, 0.0f, __int_as_float(-1));
+    }
+    if (!__any_sync(0xffffffffu, active)) {
+      if (!__any_sync(0xffffffffu, i < ray_count)) break;
+      continue;
+    }
+    // own slot, then the network of quad_intersect over the four lanes
+    float t = __int_as_float(0x7f800000);
+    int32_t child = -1, count = -1;
+    bool hit = false;
+    if (active) {
+      const float tx0 = (slot.x0 - ray.ox) * ray.ix, tx1 = (slot.x1 - ray.ox) * ray.ix;
+      const float ty0 = (slot.y0 - ray.oy) * ray.iy, ty1 = (slot.y1 - ray.oy) * ray.iy;
+      const float tz0 = (slot.z0 - ray.oz) * ray.iz, tz1 = (slot.z1 - ray.oz) * ray.iz;
+      child = slot.child;
+      count = slot.count;
+      float tx;
+      if (fast) {
+        t = fmaxf(fminf(tx0, tx1), fmaxf(fminf(ty0, ty1), fminf(tz0, tz1)));
+        tx = fminf(fmaxf(tx0, tx1), fminf(fmaxf(ty0, ty1), fmaxf(tz0, tz1)));
+      } else {
+        t = sse_max(sse_min(tx0, tx1), sse_max(sse_min(ty0, ty1), sse_min(tz0, tz1)));
+        tx = sse_min(sse_max(tx0, tx1), sse_min(sse_max(ty0, ty1), sse_max(tz0, tz1)));
+      }
+      hit = (tx >= t) && (t < ray.t);
+      if (CULL == kCullBehind && cull) hit = hit && tx >= 0.0f;
+      if (CULL == kCullSubtree && cull && hit) {
+        const float* b = reinterpret_cast<const float*>(a.tboxes + current) + q.l;
+        const float bx0 = (__ldg(b) - ray.ox) * ray.ix, bx1 = (__ldg(b + 4) - ray.ox) * ray.ix;
+        const float by0 = (__ldg(b + 8) - ray.oy) * ray.iy, by1 = (__ldg(b + 12) - ray.oy) * ray.iy;
+        const float bz0 = (__ldg(b + 16) - ray.oz) * ray.iz, bz1 = (__ldg(b + 20) - ray.oz) * ray.iz;
+        const float bn = fmaxf(fminf(bx0, bx1), fmaxf(fminf(by0, by1), fminf(bz0, bz1)));
+        const float bf = fminf(fmaxf(bx0, bx1), fminf(fmaxf(by0, by1), fmaxf(bz0, bz1)));
+        hit = bf >= bn && bf >= 0.0f && bn < ray.t;
+      }
+    }
+    const uint32_t hits = q.ballot(hit);
+    uint32_t id = q.l;
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) {
+      const float ot = __shfl_xor_sync(0xffffffffu, t, o);
+      const uint32_t oid = __shfl_xor_sync(0xffffffffu, id, o);
+      const bool low = (q.l & (uint32_t)o) == 0u;
+      if (low ? t > ot : ot > t) {
+        t = ot;
+        id = oid;
+      }
+    }
+    {
+      const float ot = __shfl_xor_sync(0xffffffffu, t, 1);
+      const uint32_t oid = __shfl_xor_sync(0xffffffffu, id, 1);
+      if (q.l >= 2u && (q.l == 2u ? t > ot : ot > t)) id = oid;
+    }
+    // the slot at this lane's place; places are visited from 3 down to 0
+    child = q.from(child, id);
+    count = q.from(count, id);
+    hit = (hits >> id) & 1u;
+    const bool inner = hit && count <= -1 && child > -1, leaf = hit && count > -1;
+    const uint32_t inners = q.ballot(inner);
+    const int n = __popc(inners);
+    const int32_t nearest = q.from(child, inners ? (uint32_t)__ffs(inners) - 1u : 0u);
+    bool done = false;
+    int32_t next = -1;
+    if (n > 0) {
+      next = nearest;
+      if (sp + n - 1 >= kStack) {
+        if (q.l == 0u) atomicOr(a.status, kStatusStackOverflow);
+        prim = -2;
+        done = true;
+      } else {
+        // farther slots below nearer ones
+        if (inner && (inners & ((1u << q.l) - 1u))) stack[sp + 1 + __popc(inners >> (q.l + 1u))] = child;
+        sp += n - 1;
+      }
+    }
+    __syncwarp();
+    if (active && !done) {
+      current = next;
+      if (next < 0 && sp >= 0) current = stack[sp--];
+      if (current >= 0) fetch();
+    }
+    if (__any_sync(0xffffffffu, leaf)) {
+      const float entry = ray.t;
+      float u = hu, v = hv;
+      int32_t p = prim;
+      bool bad = false, found = false;
+      if (leaf) {
+        bad = child < 0 || (uint32_t)child + (uint32_t)count > a.prim_count;
+        if (bad) atomicOr(a.status, kStatusBadIndex);
+        for (int32_t j = 0; !bad && j < count; ++j) {
+          if (mt_test(a.tris + kTriFloat4 * (size_t)(child + j), ray, u, v, p)) {
+            found = true;
+            if (ANY_HIT) break;
+          }
+        }
+      }
+      const uint32_t founds = q.ballot(found);
+      if (q.ballot(bad)) done = true;
+      float best, before;
+      int w = first_nearest<true>(q, ray.t, entry, best, before);
+      if (ANY_HIT) w = founds ? 31 - __clz(founds) : -1;  // the first leaf in the walk's order
+      const uint32_t src = w < 0 ? q.l : (uint32_t)w;
+      const float wt = q.from(ray.t, src), wu = q.from(u, src), wv = q.from(v, src);
+      const int32_t wp = q.from(p, src);
+      ray.t = entry;
+      if (w >= 0 && prim != -2) {
+        ray.t = wt;
+        hu = wu;
+        hv = wv;
+        prim = wp;
+        if (ANY_HIT) done = true;
+      }
+    }
+    if (active && (done || current < 0)) {
+      if (q.l == 0u) a.hits[r] = make_float4(ray.t, hu, hv, __int_as_float(prim));
+      active = false;
+    }
+  }
+}
+
+// Few rays over the exact quad nodes.
+template <bool ANY_HIT, int CULL>
+__global__ void __launch_bounds__(kBlock) k_trace_mbvh4(TraceArgs a, uint32_t warps) {
+  __shared__ int32_t s_stack[kBlock / 4][kStack];
+  walk_mbvh4<ANY_HIT, CULL>(a, (uint32_t)a.ray_count, warps, s_stack);
+}
+
 // Persistent MBVH traversal over the exact quad nodes with per-lane ray
 // refill. Each loop iteration visits one quad node per lane; a ray's
 // node/triangle order is the reference's. With ray_count_dev the number of
@@ -300,8 +578,9 @@ __device__ __forceinline__ uint32_t subtree_mask(const DTBox* box, const RayStat
 //   shadow ray that leaves a surface walks the whole scene behind it too.
 //   4.2M shadow rays over 1M clustered triangles: 10.74 ms without the skip,
 //   3.80 ms with it.
-constexpr int kCullNone = 0, kCullSubtree = 1, kCullBehind = 2;
-template <bool ANY_HIT, bool STATS, int CULL = kCullNone>
+// FEW: a launch whose ray count is read from the device walks with four lanes
+// per ray when that is at most kFewDeferred.
+template <bool ANY_HIT, bool STATS, int CULL = kCullNone, bool FEW = false>
 __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int* work) {
   RayState ray;
   float hu = 0.0f, hv = 0.0f;
@@ -319,6 +598,14 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int
   WarpPool pool;
   uint32_t batch = a.ray_batch ? a.ray_batch : kPoolBatch;
   const uint32_t ray_count = a.ray_count_dev ? *a.ray_count_dev : (uint32_t)a.ray_count;
+  if (FEW) {
+    __shared__ int32_t s_stack[kBlock / 4][kStack];
+    if (ray_count <= kFewDeferred) {
+      const uint32_t launched = gridDim.x * (kBlock / 32u), wanted = few_warps(ray_count, a.sms);
+      walk_mbvh4<ANY_HIT, CULL>(a, ray_count, wanted < launched ? wanted : launched, s_stack);
+      return;
+    }
+  }
   if (a.ray_count_dev) {
     // few rays (deferred by the compact walk): spread them over all warps,
     // down to one ray per refill, so that their walks run side by side
@@ -329,24 +616,7 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int
     r = a.order ? __ldg(a.order + rr) : rr;
     ray = load_ray(a.rays, r, a.t_max);
     fast = finite_ray(ray);
-    if (CULL != kCullNone && a.node_count > 0) {
-      const DAabb root = load_aabb(a.nodes);
-      // |x| <= bound is false for NaN and infinities
-      cull = fabsf(ray.ox) <= kCompactRange && fabsf(ray.oy) <= kCompactRange && fabsf(ray.oz) <= kCompactRange &&
-             fabsf(ray.dx) <= 3.0e38f && fabsf(ray.dy) <= 3.0e38f && fabsf(ray.dz) <= 3.0e38f &&
-             fabsf(ray.ix) <= kQuantRange && fabsf(ray.iy) <= kQuantRange && fabsf(ray.iz) <= kQuantRange;
-      if (CULL == kCullSubtree) {
-        // Only rays that start inside the scene's root box: boxes behind
-        // them are most of what the cull saves; for rays from outside the
-        // extra box loads cost more than they save
-        cull = cull && ray.ox >= root.min[0] && ray.oy >= root.min[1] && ray.oz >= root.min[2] &&
-               ray.ox <= root.max[0] && ray.oy <= root.max[1] && ray.oz <= root.max[2];
-      } else {
-        // the margin argument needs the boxes within the range too
-        for (int k = 0; k < 3; ++k)
-          cull = cull && root.min[k] >= -kCompactRange && root.max[k] <= kCompactRange;
-      }
-    }
+    if (CULL != kCullNone && a.node_count > 0) cull = cull_ray<CULL>(a, ray);
     hu = hv = 0.0f;
     prim = -1;
     visits = tests = max_depth = 0;
@@ -588,6 +858,26 @@ __device__ __forceinline__ void slot_keys_exact(const DMNode* node, const RaySta
   sort_slots(key, ich);
 }
 
+// Whether the compact walk takes this ray (|x| <= bound is false for NaN and
+// infinities).
+__device__ __forceinline__ bool compact_ray(const RayState& ray) {
+  return fabsf(ray.ox) <= kCompactRange && fabsf(ray.oy) <= kCompactRange && fabsf(ray.oz) <= kCompactRange &&
+         fabsf(ray.dx) <= 3.0e38f && fabsf(ray.dy) <= 3.0e38f && fabsf(ray.dz) <= 3.0e38f &&
+         fabsf(ray.ix) <= kQuantRange && fabsf(ray.iy) <= kQuantRange && fabsf(ray.iz) <= kQuantRange;
+}
+// Start of ray r's walk over the traversal tree (of its mesh); false: no
+// nodes, a miss.
+__device__ __forceinline__ bool compact_root(const TraceArgs& a, uint32_t r, int32_t& root) {
+  root = 0;
+  if (a.node_count == 0) return false;
+  if (a.seg_count) {
+    const uint32_t m = ray_mesh(a, r);
+    if (__ldg(a.seg_root + m) == __ldg(a.seg_root + m + 1)) return false;
+    root = (int32_t)__ldg(a.seg_qroot + m);
+  }
+  return true;
+}
+
 // Closest hit over the compact (64-byte) nodes of the traversal tree, with
 // the leaf tests taken out of the slot loop. A loop iteration has a node
 // phase -- each lane with no untested leaf visits its next node, pushes the
@@ -656,26 +946,12 @@ __global__ void __launch_bounds__(kBlock, 9) k_trace_compact(TraceArgs a, unsign
     prim = -1;
     sp = -1;
     pend = 0;
-    next = 0;
     w_visits = w_tests = 0;
-    if (a.node_count == 0) {
+    if (!compact_root(a, r, next)) {
       finish();
       return;
     }
-    if (a.seg_count) {
-      const uint32_t m = ray_mesh(a, r);
-      if (__ldg(a.seg_root + m) == __ldg(a.seg_root + m + 1)) {
-        finish();  // a mesh without nodes: a miss
-        return;
-      }
-      next = (int32_t)__ldg(a.seg_qroot + m);
-    }
-    // |x| <= bound is false for NaN and infinities
-    const bool ok = fabsf(ray.ox) <= kCompactRange && fabsf(ray.oy) <= kCompactRange &&
-                    fabsf(ray.oz) <= kCompactRange && fabsf(ray.dx) <= 3.0e38f && fabsf(ray.dy) <= 3.0e38f &&
-                    fabsf(ray.dz) <= 3.0e38f && fabsf(ray.ix) <= kQuantRange && fabsf(ray.iy) <= kQuantRange &&
-                    fabsf(ray.iz) <= kQuantRange;
-    if (!ok) {
+    if (!compact_ray(ray)) {
       defer();
       return;
     }
@@ -762,6 +1038,194 @@ __global__ void __launch_bounds__(kBlock, 9) k_trace_compact(TraceArgs a, unsign
       }
     }
     if (active && pend == 0 && next < 0 && sp < 0) finish();
+  }
+}
+
+// One lane's slot of a compact node: the node's grid and the slot's near and
+// far bounds as floats q * 2^-133 (see qbyte), picked by address.
+struct LaneSlot {
+  float4 head;
+  uint32_t nx, fx, ny, fy, nz, fz;
+  int32_t child, count;
+  __device__ __forceinline__ void load(const DQNode* n, const RayState& ray, uint32_t l) {
+    const uint8_t* node = reinterpret_cast<const uint8_t*>(n);
+    const uint8_t* b = node + 16 + l;
+    head = __ldg(reinterpret_cast<const float4*>(node));
+    nx = __ldg(b + (ray.ix < 0.0f ? 4 : 0));
+    fx = __ldg(b + (ray.ix < 0.0f ? 0 : 4));
+    ny = __ldg(b + (ray.iy < 0.0f ? 12 : 8));
+    fy = __ldg(b + (ray.iy < 0.0f ? 8 : 12));
+    nz = __ldg(b + (ray.iz < 0.0f ? 20 : 16));
+    fz = __ldg(b + (ray.iz < 0.0f ? 16 : 20));
+    child = __ldg(reinterpret_cast<const int32_t*>(node + 40) + l);
+    count = __ldg(reinterpret_cast<const int16_t*>(node + 56) + l);
+  }
+};
+
+// k_trace_compact's walk, four lanes per ray, for few rays: every lane reads
+// its own slot of a node and, where it is a leaf, tests it. The next node is
+// popped and its slots are asked for before the leaves are tested.
+template <bool GATES>
+__global__ void __launch_bounds__(kBlock) k_trace_compact4(TraceArgs a, uint32_t warps, uint32_t* deferred,
+                                                          unsigned int* deferred_count) {
+  __shared__ int32_t s_stack[kBlock / 4][kStack];
+  const FourLanes q;
+  int32_t* stack = s_stack[threadIdx.x >> 2];
+  const uint32_t warp = blockIdx.x * (kBlock / 32u) + (threadIdx.x >> 5);
+  const float inf = __int_as_float(0x7f800000);
+  RayState ray;
+  float hu = 0.0f, hv = 0.0f;
+  int32_t prim = -1, current = -1;  // the node whose slots are in `slot`
+  int sp = -1;
+  bool active = false;
+  LaneSlot slot;
+  // asks for the slots of `current`; false (the ray ends) when it is no node
+  auto fetch = [&]() {
+    if ((uint32_t)current >= a.q_count) {
+      if (q.l == 0u) atomicOr(a.status, kStatusBadIndex);
+      active = false;
+    } else {
+      slot.load(a.qnodes + current, ray, q.l);
+    }
+  };
+  uint32_t r = 0;
+  auto defer = [&]() {
+    if (q.l == 0u) deferred[atomicAdd(deferred_count, 1u)] = r;
+    active = false;
+  };
+  for (size_t i = warp < warps ? warp + (size_t)warps * (q.first >> 2) : a.ray_count;;) {
+    if (!active && i < a.ray_count) {
+      r = a.order ? __ldg(a.order + i) : (uint32_t)i;
+      i += 8u * (size_t)warps;
+      ray = load_ray(a.rays, r, a.t_max);
+      hu = hv = 0.0f;
+      prim = -1;
+      sp = -1;
+      active = compact_root(a, r, current);
+      if (!active) {
+        if (q.l == 0u) a.hits[r] = make_float4(ray.t, 0.0f, 0.0f, __int_as_float(-1));
+      } else if (!compact_ray(ray)) {
+        defer();
+      } else {
+        fetch();
+      }
+    }
+    if (!__any_sync(0xffffffffu, active)) {
+      if (!__any_sync(0xffffffffu, i < a.ray_count)) break;
+      continue;
+    }
+    bool hit = false, inner = false, large = false;
+    float key = inf;
+    int32_t child = -1, count = -1;
+    if (active) {
+      const float4 head = slot.head;
+      child = slot.child;
+      count = slot.count;
+      const uint32_t exps = __float_as_uint(head.w), flags = exps >> 24;
+      float tn, tx, t;
+      if (flags == 0u) {  // slot_keys_q
+        const float sx = __uint_as_float(((exps & 0xffu) << 23) + kStepBias);
+        const float sy = __uint_as_float(((exps >> 8 & 0xffu) << 23) + kStepBias);
+        const float sz = __uint_as_float(((exps >> 16 & 0xffu) << 23) + kStepBias);
+        const float ax = sx * ray.ix, bx = (head.x - ray.ox) * ray.ix * kKeyScale;
+        const float ay = sy * ray.iy, by = (head.y - ray.oy) * ray.iy * kKeyScale;
+        const float az = sz * ray.iz, bz = (head.z - ray.oz) * ray.iz * kKeyScale;
+        tn = fmaxf(fmaf(__uint_as_float(slot.nx << 16), ax, bx),
+                   fmaxf(fmaf(__uint_as_float(slot.ny << 16), ay, by), fmaf(__uint_as_float(slot.nz << 16), az, bz)));
+        tx = fminf(fmaf(__uint_as_float(slot.fx << 16), ax, bx),
+                   fminf(fmaf(__uint_as_float(slot.fy << 16), ay, by), fmaf(__uint_as_float(slot.fz << 16), az, bz)));
+        t = ray.t * kKeyScale;
+      } else {  // slot_keys_exact
+        const float* n = reinterpret_cast<const float*>(a.qexact + current) + q.l;
+        const float tx0 = (__ldg(n) - ray.ox) * ray.ix, tx1 = (__ldg(n + 4) - ray.ox) * ray.ix;
+        const float ty0 = (__ldg(n + 8) - ray.oy) * ray.iy, ty1 = (__ldg(n + 12) - ray.oy) * ray.iy;
+        const float tz0 = (__ldg(n + 16) - ray.oz) * ray.iz, tz1 = (__ldg(n + 20) - ray.oz) * ray.iz;
+        child = __float_as_int(__ldg(n + 24));
+        count = __float_as_int(__ldg(n + 28));
+        large = count > 32767;
+        tn = fmaxf(fminf(tx0, tx1), fmaxf(fminf(ty0, ty1), fminf(tz0, tz1)));
+        tx = fminf(fmaxf(tx0, tx1), fminf(fmaxf(ty0, ty1), fmaxf(tz0, tz1)));
+        t = ray.t;
+      }
+      hit = tx >= tn && tx >= 0.0f && tn < t && child >= 0;
+      inner = hit && count < 0;
+      if (inner) key = tn;
+      large = large || (flags & kQFlagOutOfRange);
+    }
+    if (q.ballot(large)) {  // the exact walk's
+      if (active) defer();
+      hit = inner = false;
+      key = inf;
+    }
+    // sort_slots over the four lanes
+    int32_t near_child = child;
+    auto exchange = [&](uint32_t with) {
+      const float ok = q.from(key, with);
+      const int32_t oc = q.from(near_child, with);
+      if (q.l < with ? ok < key : (q.l > with && key < ok)) {
+        key = ok;
+        near_child = oc;
+      }
+    };
+    exchange(q.l ^ 1u);
+    exchange(q.l ^ 2u);
+    exchange(q.l == 1u ? 2u : (q.l == 2u ? 1u : q.l));
+    const int n = __popc(q.ballot(key < inf));
+    const int32_t nearest = q.from(near_child, 0);
+    bool done = false;
+    int32_t next = -1;
+    if (n > 0) {
+      next = nearest;
+      if (sp + n - 1 >= kStack) {
+        if (q.l == 0u) atomicOr(a.status, kStatusStackOverflow);
+        prim = -2;
+        done = true;
+      } else {
+        if (q.l >= 1u && (int)q.l < n) stack[sp + n - (int)q.l] = near_child;
+        sp += n - 1;
+      }
+    }
+    __syncwarp();
+    const bool leaf = hit && !inner && !done;
+    if (active && !done) {
+      current = next;
+      if (next < 0 && sp >= 0) current = stack[sp--];
+      if (current >= 0) fetch();
+    }
+    if (__any_sync(0xffffffffu, leaf)) {
+      const float entry = ray.t;
+      float u = hu, v = hv, escaped = inf;
+      int32_t p = prim;
+      bool bad = false;
+      if (leaf) {
+        bad = (uint32_t)child + (uint32_t)count > a.prim_count;
+        if (bad) atomicOr(a.status, kStatusBadIndex);
+        for (int32_t j = 0; !bad && j < count; ++j) {
+          const float4* tri = a.tris + kTriFloat4 * (size_t)(child + j);
+          if (mt_test(tri, ray, u, v, p) && GATES && (__float_as_uint(__ldg(&tri[1].w)) & kTriEscape)) escaped = ray.t;
+        }
+      }
+      float best, before;
+      const int w = first_nearest<false>(q, ray.t, entry, best, before);
+      const uint32_t src = w < 0 ? q.l : (uint32_t)w;
+      const float wt = q.from(ray.t, src), wu = q.from(u, src), wv = q.from(v, src);
+      const int32_t wp = q.from(p, src);
+      ray.t = entry;
+      if (w >= 0) {
+        ray.t = wt;
+        hu = wu;
+        hv = wv;
+        prim = wp;
+      }
+      const uint32_t bads = q.ballot(bad);
+      const uint32_t escapes = q.ballot(GATES && escaped < before);
+      if (active && bads) active = false;
+      else if (active && escapes) defer();  // an escaped triangle is hit: its hits are the exact walk's
+    }
+    if (active && (done || current < 0)) {
+      if (q.l == 0u) a.hits[r] = make_float4(ray.t, hu, hv, __int_as_float(prim));
+      active = false;
+    }
   }
 }
 
@@ -1090,13 +1554,13 @@ __global__ void __launch_bounds__(256) k_ray_keys(const float* __restrict__ rays
 // Persistent grid: resident blocks per SM (occupancy, capped by
 // blocks_per_sm) on every SM, no more blocks than the rays need.
 template <class K>
-unsigned persistent_grid(K kern, const TraceArgs& a) {
+unsigned persistent_grid(K kern, const TraceArgs& a, size_t rays_per_block = kBlock) {
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kBlock, 0);
   if (per_sm < 1) per_sm = 1;
   if (a.blocks_per_sm > 0 && (int)a.blocks_per_sm < per_sm) per_sm = (int)a.blocks_per_sm;
   size_t grid = (size_t)sm_count() * per_sm;
-  const size_t need = (a.ray_count + kBlock - 1) / kBlock;
+  const size_t need = (a.ray_count + rays_per_block - 1) / rays_per_block;
   if (grid > need) grid = need;
   return (unsigned)grid;
 }
@@ -1121,9 +1585,28 @@ auto compact_kernel(const TraceArgs& a) {
                                             : k_trace_compact<64, false, WSTATS>);
 }
 
+// Launches of few rays with no launch shape asked for: four lanes per ray.
+bool few_rays(const TraceArgs& a) {
+  return a.ray_count <= (a.any_hit ? kFewAny : kFewClosest) && a.ray_batch == 0 && a.blocks_per_sm == 0 &&
+         (a.stack_limit == 0 || a.stack_limit == (uint32_t)kStack);
+}
+
+template <bool ANY_HIT, int CULL>
+cudaError_t launch_few(const TraceArgs& a, cudaStream_t s) {
+  const uint32_t warps = few_warps((uint32_t)a.ray_count, (uint32_t)sm_count());
+  k_trace_mbvh4<ANY_HIT, CULL><<<(warps + 3u) / 4u, kBlock, 0, s>>>(a, warps);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_compact(const TraceArgs& a, cudaStream_t s, unsigned int* counters, uint32_t* deferred) {
-  auto kern = a.walk_stats ? compact_kernel<true>(a) : compact_kernel<false>(a);
-  kern<<<persistent_grid(kern, a), kBlock, 0, s>>>(a, counters, deferred, counters + 1);
+  if (few_rays(a) && !a.walk_stats) {
+    const uint32_t warps = few_warps((uint32_t)a.ray_count, (uint32_t)sm_count());
+    auto kern = a.q_gates ? k_trace_compact4<true> : k_trace_compact4<false>;
+    kern<<<(warps + 3u) / 4u, kBlock, 0, s>>>(a, warps, deferred, counters + 1);
+  } else {
+    auto kern = a.walk_stats ? compact_kernel<true>(a) : compact_kernel<false>(a);
+    kern<<<persistent_grid(kern, a), kBlock, 0, s>>>(a, counters, deferred, counters + 1);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   TraceArgs b = a;
@@ -1132,12 +1615,10 @@ cudaError_t launch_compact(const TraceArgs& a, cudaStream_t s, unsigned int* cou
   // at most 32 rays per refill (the kernel takes fewer when few rays were
   // deferred)
   b.ray_batch = 32;
-  if (b.tboxes) {
-    auto cull_kern = k_trace_mbvh<false, false, kCullSubtree>;
-    cull_kern<<<persistent_grid(cull_kern, b), kBlock, 0, s>>>(b, counters + 2);
-    return cudaGetLastError();
-  }
-  return launch3<true, false, false>(b, s, counters + 2);
+  b.sms = (uint32_t)sm_count();
+  auto rest = b.tboxes ? k_trace_mbvh<false, false, kCullSubtree, true> : k_trace_mbvh<false, false, kCullNone, true>;
+  rest<<<persistent_grid(rest, b, kBlock / 4), kBlock, 0, s>>>(b, counters + 2);
+  return cudaGetLastError();
 }
 
 template <bool MBVH>
@@ -1151,8 +1632,14 @@ cudaError_t launch_any(const TraceArgs& a0, cudaStream_t s) {
   TraceArgs a = a0;
   // any hit: most walks end after a few nodes, so refills are frequent and
   // larger pools cost fewer counter atomics (128: 34.0 against 28.7 Grays/s
-  // with 32 on the 1M incoherent scene's occlusion rays)
-  if (a.any_hit && a.ray_batch == 0) a.ray_batch = 128u;
+  // with 32 on the 1M incoherent scene's occlusion rays), but not so large
+  // that a launch has fewer pools than warps (131,072 shadow rays over 300k
+  // clustered triangles: 301 us with pools of 32, 500 with 128)
+  const bool few = few_rays(a);
+  if (a.any_hit && a.ray_batch == 0) {
+    const size_t even = a.ray_count / ((size_t)sm_count() * 32u);  // rays per resident warp
+    a.ray_batch = even < 32u ? 32u : (even < 128u ? (uint32_t)even : 128u);
+  }
   Scratch<unsigned int> work;
   Scratch<uint32_t> keys, order, acc, deferred;
   Scratch<char> sort_temp;
@@ -1173,16 +1660,23 @@ cudaError_t launch_any(const TraceArgs& a0, cudaStream_t s) {
     a.order = order.ptr;
   }
   const bool st = a.stats != nullptr;
-  if (a.any_hit && MBVH && !st && (a.quads_cover || a.tboxes)) {
-    auto kern = a.quads_cover ? k_trace_mbvh<true, false, kCullBehind> : k_trace_mbvh<true, false, kCullSubtree>;
-    kern<<<persistent_grid(kern, a), kBlock, 0, s>>>(a, work.ptr);
-    e = cudaGetLastError();
+  if (a.any_hit && MBVH && !st) {
+    if (few) {
+      e = a.quads_cover ? launch_few<true, kCullBehind>(a, s)
+                        : (a.tboxes ? launch_few<true, kCullSubtree>(a, s) : launch_few<true, kCullNone>(a, s));
+    } else {
+      auto kern = a.quads_cover ? k_trace_mbvh<true, false, kCullBehind>
+                                : (a.tboxes ? k_trace_mbvh<true, false, kCullSubtree> : k_trace_mbvh<true, false>);
+      kern<<<persistent_grid(kern, a), kBlock, 0, s>>>(a, work.ptr);
+      e = cudaGetLastError();
+    }
   } else if (a.any_hit) e = st ? launch3<MBVH, true, true>(a, s, work.ptr) : launch3<MBVH, true, false>(a, s, work.ptr);
   else if (st) e = launch3<MBVH, false, true>(a, s, work.ptr);
   else if (MBVH && a.qnodes && a.q_count > 0) {
     if ((e = deferred.alloc(a.ray_count, s))) return e;
     e = launch_compact(a, s, work.ptr, deferred.ptr);
-  } else e = launch3<MBVH, false, false>(a, s, work.ptr);
+  } else if (MBVH && few) e = launch_few<false, kCullNone>(a, s);
+  else e = launch3<MBVH, false, false>(a, s, work.ptr);
   return e;
 }
 
