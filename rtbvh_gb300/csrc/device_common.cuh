@@ -107,11 +107,11 @@ __device__ __forceinline__ float sse_max(float a, float b) { return a > b ? a : 
 // Order-preserving map of floats to uint32 (-0 sorts below +0) for atomic
 // min/max reductions.
 __device__ __forceinline__ uint32_t float_to_ordered(float f) {
-  uint32_t b = __float_as_uint(f);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  const uint32_t b = __float_as_uint(f);
+  return b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
 }
 __device__ __forceinline__ float ordered_to_float(uint32_t k) {
-  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+  return __uint_as_float(k ^ ((uint32_t)((int32_t)~k >> 31) | 0x80000000u));
 }
 
 // Aabb::half_area (src/aabb.rs:342-346), no FMA.

@@ -15,16 +15,17 @@
 //     deterministic) and builds the next level's task list. Children of at
 //     most sub_max primitives are not split level by level: they go to a
 //     subtree list. sub_max = n / 2048 clamped to [32, kWarpMax], so a small
-//     build keeps enough subtrees to fill the GPU.
+//     build keeps enough subtrees to fill the GPU. (It also decides the node
+//     numbering: breadth first above it.)
 //
 // After the last level, k_sub_build builds every listed subtree depth first,
 // one warp per subtree (bins in shared memory, the warp-parallel decision,
-// ballot partition; tasks of at most kThreadMax primitives are finished by
-// single lanes, exact sweep over the non-empty bins), with no grid-wide
-// phases. The node pair of a split at primitive position m goes to scratch
-// slots 2(m-1), 2(m-1)+1 -- split positions are distinct across the whole
-// tree -- and a scan over the positions places the pairs after the
-// breadth-first part in position order, so the numbering stays
+// ballot partition); what is left, subtrees of at most kSmall primitives, is
+// built by k_sub_small, one lane per primitive and several subtrees per warp.
+// Neither has grid-wide phases. The node pair of a split at primitive position
+// m goes to scratch slots 2(m-1), 2(m-1)+1 -- split positions are distinct
+// across the whole tree -- and a scan over the positions places the pairs after
+// the breadth-first part in position order, so the numbering stays
 // deterministic and gap-free.
 //
 // The split arithmetic is the reference's: node box + 1e-4; 16 bins per axis
@@ -78,8 +79,8 @@ struct Counters {
   uint32_t ticket;      // chunk ticket of the partition kernel
   uint32_t sub_head;    // next subtree a warp of k_sub_build takes
   uint32_t sub_splits;  // splits inside the subtrees (the scan's total)
-  uint32_t tiny;        // subtrees of at most kThreadMax primitives listed by k_sub_build
-  uint32_t tiny_head;   // next one a thread of k_sub_tiny takes
+  uint32_t tiny;        // entries of the small-subtree list
+  uint32_t tiny_head;   // next ones a warp of k_sub_small takes
 };
 
 struct BinMap {
@@ -356,7 +357,8 @@ struct SahParams {
   uint32_t sub_max;     // largest task built as a subtree (<= kWarpMax)
   Task* large[2];       // task lists of even / odd levels
   Task* subs;           // subtree tasks (at most sub_max primitives), all levels
-  void* tiny;           // SubTask list: subtrees of at most kThreadMax primitives
+  void* tiny;           // SubTask list: subtrees of at most kSmall primitives (empty entries have end 0)
+  uint32_t small_cap;   // its capacity
   Decision* dec;        // large tasks of the level
   float* tbox;          // 6 floats per large task (box with first offset)
   uint32_t* bins;       // kTaskBinWords per large task
@@ -697,172 +699,16 @@ __device__ void large_copyback_chunk(const SahParams& p, const Level& lv, uint32
 }
 
 // ------------------------------------------------------------------ small tasks
-// A task of at most kThreadMax primitives is decided by one thread. Its
-// bins hold at most kThreadMax primitives, and find_split's cost at bin i
-// depends only on which primitives lie left and right of i: it is NaN while
-// a side is empty and constant between two non-empty bins. So the first
-// minimum over i is found by visiting the non-empty bins in ascending order
-// and evaluating the cost at each (the same float expression over the same
-// unions, hence the same bits). Larger small tasks take a warp each.
-constexpr uint32_t kThreadMax = 8;
+// Subtrees of at most kSmall primitives are listed and built by k_sub_small.
+// 4M clustered triangles, build with both trees: 8 primitives 9.44 ms, 12
+// 9.20, 16 9.20, 24 9.58, 32 9.86.
+constexpr uint32_t kSmall = 16;
+static_assert(kSmall <= 32, "a lane per primitive");
 
-// Union, from Aabb::empty(), of the primitives in `sel` (keys, decoded).
-__device__ __forceinline__ void union_sel(const uint32_t (&kb)[kThreadMax][6], uint32_t ws, uint32_t sel, float mn[3],
-                                          float mx[3]) {
-  uint32_t umn[3], umx[3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    umn[k] = float_to_ordered(1e34f);
-    umx[k] = float_to_ordered(-1e34f);
-  }
-#pragma unroll
-  for (uint32_t j = 0; j < kThreadMax; ++j) {
-    if (j < ws && ((sel >> j) & 1u)) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        umn[k] = min(umn[k], kb[j][k]);
-        umx[k] = max(umx[k], kb[j][3 + k]);
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    mn[k] = ordered_to_float(umn[k]);
-    mx[k] = ordered_to_float(umx[k]);
-  }
-}
-
-__device__ __forceinline__ uint32_t bin_at(uint32_t packed, uint32_t j) { return (packed >> (4 * j)) & 15u; }
-
-// Mask of the primitives whose bin is below `bound`.
-__device__ __forceinline__ uint32_t below(uint32_t packed, uint32_t ws, uint32_t bound) {
-  uint32_t m = 0;
-#pragma unroll
-  for (uint32_t j = 0; j < kThreadMax; ++j)
-    if (j < ws && bin_at(packed, j) < bound) m |= 1u << j;
-  return m;
-}
-
-// Smallest bin above `after` (16: none) -- ascending visit of non-empty bins.
-__device__ __forceinline__ uint32_t next_bin(uint32_t packed, uint32_t ws, int after) {
-  uint32_t nb = (uint32_t)kBins;
-#pragma unroll
-  for (uint32_t j = 0; j < kThreadMax; ++j) {
-    const uint32_t b = bin_at(packed, j);
-    if (j < ws && (int)b > after && b < nb) nb = b;
-  }
-  return nb;
-}
-
-// BinnedSahBuildTask::run (binned_sah.rs:132-282) after the node box is
-// known, for a task of at most kThreadMax primitives by one thread: `mn` /
-// `mx` is the node box with its first offset. On a split the task's indices
-// are left stably partitioned (left primitives first, in order).
-__device__ void decide_thread(const SahParams& p, uint32_t begin, uint32_t ws, uint32_t depth, const float mn[3],
-                              const float mx[3], Decision& d) {
-  d.split = 0;
-  if (ws > 1 && depth < kMaxDepth) {
-    uint32_t prim[kThreadMax];
-    uint32_t kb[kThreadMax][6];
-    uint32_t packed[3] = {0u, 0u, 0u};
-    const BinMap bm = make_binmap(mn, mx);
-#pragma unroll
-    for (uint32_t j = 0; j < kThreadMax; ++j) {
-      if (j < ws) {
-        prim[j] = p.idx_a[begin + j];
-        const float4 c = __ldg(p.centers + prim[j]);
-        const DAabb box = load_aabb(p.aabbs + prim[j]);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          kb[j][k] = float_to_ordered(box.min[k]);
-          kb[j][3 + k] = float_to_ordered(box.max[k]);
-        }
-        packed[0] |= bin_of(c.x, bm.c2b[0], bm.off[0]) << (4 * j);
-        packed[1] |= bin_of(c.y, bm.c2b[1], bm.off[1]) << (4 * j);
-        packed[2] |= bin_of(c.z, bm.c2b[2], bm.off[2]) << (4 * j);
-      }
-    }
-    const uint32_t all = (1u << ws) - 1u;
-    float best_cost[3];
-    uint32_t best_count[3];
-#pragma unroll 1
-    for (int a = 0; a < 3; ++a) {
-      float bc = kF32Max;
-      uint32_t bn = (uint32_t)kBins;
-      for (int b = -1;;) {
-        b = (int)next_bin(packed[a], ws, b);
-        if (b >= kBins) break;
-        const uint32_t left = below(packed[a], ws, (uint32_t)b + 1u);
-        if (left == all) break;  // right side empty from here on
-        float lmn[3], lmx[3], rmn[3], rmx[3];
-        union_sel(kb, ws, left, lmn, lmx);
-        union_sel(kb, ws, all & ~left, rmn, rmx);
-        const uint32_t nl = (uint32_t)__popc(left);
-        const float cost = ha6(lmn, lmx) * (float)nl + ha6(rmn, rmx) * (float)(ws - nl);
-        if (cost < bc) {
-          bc = cost;
-          bn = (uint32_t)b + 1u;
-        }
-      }
-      best_cost[a] = bc;
-      best_count[a] = bn;
-    }
-    int axis = 0;
-    if (best_cost[0] > best_cost[1]) axis = 1;
-    if (best_cost[axis] > best_cost[2]) axis = 2;
-    uint32_t split_index = best_count[axis];
-    const float max_split_cost = ha6(mn, mx) * ((float)ws - kTraversalCost);
-    bool leaf = false;
-    if (best_count[axis] == (uint32_t)kBins || best_cost[axis] >= max_split_cost) {
-      if (ws <= p.max_leaf) {
-        leaf = true;
-      } else {
-        int la = 0;
-        if ((mx[1] - mn[1]) > (mx[0] - mn[0])) la = 1;
-        if ((mx[2] - mn[2]) > (mx[la] - mn[la])) la = 2;
-        axis = la;
-        const uint32_t target = ws * 2 / 5 + 1;
-        for (int b = -1;;) {
-          b = (int)next_bin(packed[la], ws, b);
-          if (b >= kBins - 1) break;  // the reference's loop stops before bin 15
-          if ((uint32_t)__popc(below(packed[la], ws, (uint32_t)b + 1u)) >= target) {
-            split_index = (uint32_t)b + 1u;
-            break;
-          }
-        }
-      }
-    }
-    if (!leaf) {
-      const uint32_t left = below(packed[axis], ws, split_index);
-      const uint32_t n_left = (uint32_t)__popc(left);
-      if (n_left > 0 && n_left < ws) {
-        d.split = 1;
-        d.axis = (uint32_t)axis;
-        d.split_index = split_index;
-        d.n_left = n_left;
-        float lmn[3], lmx[3], rmn[3], rmx[3];
-        union_sel(kb, ws, below(packed[axis], ws, best_count[axis]), lmn, lmx);
-        union_sel(kb, ws, all & ~left, rmn, rmx);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          d.lbox[k] = lmn[k];
-          d.lbox[3 + k] = lmx[k];
-          d.rbox[k] = rmn[k];
-          d.rbox[3 + k] = rmx[k];
-        }
-        uint32_t tpos = begin, fpos = begin + n_left;
-#pragma unroll
-        for (uint32_t j = 0; j < kThreadMax; ++j) {
-          if (j < ws) p.idx_a[((left >> j) & 1u) ? tpos++ : fpos++] = prim[j];
-        }
-      }
-    }
-  }
-}
-
-// The same for a task of more than kThreadMax primitives by one warp: bins
-// in shared memory (wb), indices staged in sidx, the warp-parallel decision,
-// a ballot-based stable partition. The decision is left in `d` (shared
+// BinnedSahBuildTask::run (binned_sah.rs:132-282) after the node box is known,
+// for a task of more than kSmall primitives by one warp: bins in shared memory
+// (wb), indices staged in sidx, the warp-parallel decision, a ballot-based
+// stable partition. The decision is left in `d` (shared
 // memory, written by lane 0) for every lane.
 __device__ void decide_warp(const SahParams& p, uint32_t begin, uint32_t ws, uint32_t depth, const float mn[3],
                             const float mx[3], uint32_t* wb, uint32_t* sidx, Decision& d) {
@@ -996,44 +842,34 @@ __device__ __forceinline__ void first_offset(const SubTask& tk, float mn[3], flo
   }
 }
 
-// A subtree whose root holds at most kThreadMax primitives, by one lane,
-// depth first (at most kThreadMax - 1 splits, so the stack stays below
-// kThreadMax + 1 entries).
-__device__ void sub_tiny(const SahParams& p, const SubTask& t0) {
-  SubTask st[kThreadMax + 1];
-  int sp = 0;
-  st[0] = t0;
-  while (sp >= 0) {
-    const SubTask tk = st[sp--];
-    float mn[3], mx[3];
-    first_offset(tk, mn, mx);
-    Decision d;
-    decide_thread(p, tk.begin, tk.end - tk.begin, tk.depth, mn, mx, d);
-    SubTask l, r;
-    if (sub_write(p, tk, mn, mx, d, l, r)) {
-      if (sp + 2 >= (int)kThreadMax + 1) {
-        atomicOr(&p.cnt->status, kStatusBadIndex);
-        return;
-      }
-      st[++sp] = r;
-      st[++sp] = l;
+// Entries of the small-subtree list that a warp reserves at a time: one atomic
+// per so many subtrees; what is left over when the warp ends is marked empty.
+constexpr uint32_t kListChunk = 32;
+struct SmallList {
+  uint32_t next = 0, end = 0;
+  // by one lane of the warp
+  __device__ __forceinline__ void add(const SahParams& p, const SubTask& t) {
+    if (next == end) {
+      next = atomicAdd(&p.cnt->tiny, kListChunk);
+      end = next + kListChunk;
+    }
+    if (next < p.small_cap) reinterpret_cast<SubTask*>(p.tiny)[next] = t;
+    else atomicOr(&p.cnt->status, kStatusBadIndex);
+    ++next;
+  }
+  __device__ __forceinline__ void finish(const SahParams& p) {
+    for (; next < end && next < p.small_cap; ++next) {
+      SubTask t = {};
+      reinterpret_cast<SubTask*>(p.tiny)[next] = t;
     }
   }
-}
+};
 
-// Appends a subtree of at most kThreadMax primitives to the list that
-// k_sub_tiny finishes, one thread per subtree.
-__device__ __forceinline__ void sub_list_tiny(const SahParams& p, const SubTask& t) {
-  const uint32_t k = atomicAdd(&p.cnt->tiny, 1u);
-  if (k < p.n) reinterpret_cast<SubTask*>(p.tiny)[k] = t;
-  else atomicOr(&p.cnt->status, kStatusBadIndex);
-}
-
-// One subtree by one warp, depth first: tasks of more than kThreadMax
-// primitives by the whole warp; smaller ones are listed for k_sub_tiny.
-// Every write goes to a place fixed by the task's primitive range, so the
-// order in which tasks run does not matter.
-__device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& sh) {
+// One subtree by one warp, depth first: tasks of more than kSmall primitives
+// by the whole warp; smaller ones are listed for k_sub_small. Every write goes
+// to a place fixed by the task's primitive range, so the order in which tasks
+// run does not matter.
+__device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& sh, SmallList& list) {
   const int lane = threadIdx.x & 31;
   int sp = -1;  // warp-uniform
   const uint32_t rws = root.end - root.begin;
@@ -1049,10 +885,10 @@ __device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& s
       t.box[k] = rb.min[k];
       t.box[3 + k] = rb.max[k];
     }
-    if (rws <= kThreadMax) sub_list_tiny(p, t);
+    if (rws <= kSmall) list.add(p, t);
     else sh.stack[0] = t;
   }
-  if (rws > kThreadMax) sp = 0;
+  if (rws > kSmall) sp = 0;
   __syncwarp();
   while (sp >= 0) {
     const SubTask tk = sh.stack[sp--];
@@ -1070,14 +906,14 @@ __device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& s
         return;
       }
       // right child first onto the stack: the left one is taken next
-      if (nr <= kThreadMax) {
-        if (lane == 0) sub_list_tiny(p, r);
+      if (nr <= kSmall) {
+        if (lane == 0) list.add(p, r);
       } else {
         if (lane == 0) sh.stack[sp + 1] = r;
         ++sp;
       }
-      if (nl <= kThreadMax) {
-        if (lane == 0) sub_list_tiny(p, l);
+      if (nl <= kSmall) {
+        if (lane == 0) list.add(p, l);
       } else {
         if (lane == 0) sh.stack[sp + 1] = l;
         ++sp;
@@ -1085,6 +921,229 @@ __device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& s
     }
     __syncwarp();
   }
+}
+
+// ------------------------------------------------------------------ subtrees of at most kSmall primitives
+// Shared memory of one warp of k_sub_small: the primitives in lane order, their
+// boxes ({min, bins}, {max, primitive}; w as integers) and centres.
+struct SmallShared {
+  float4 lo[32], hi[32];
+  float4 centre[32];
+  uint8_t entry[32];  // list entry that starts at a lane
+};
+
+// (cost key, bin) pairs: the smaller first.
+__device__ __forceinline__ bool pair_less(uint32_t a, uint32_t ab, uint32_t b, uint32_t bb) {
+  return a < b || (a == b && ab < bb);
+}
+
+// Several subtrees at once, one primitive per lane: a task is a run of lanes
+// [s, e), its children are the runs its stable partition leaves, so all tasks
+// of a level are decided side by side (BinnedSahBuildTask::run,
+// binned_sah.rs:132-282). There are no bins: find_split's cost at bin i
+// depends only on which primitives lie left and right of i -- it is NaN while
+// a side is empty and constant between two non-empty bins -- so every lane
+// evaluates the cost at its own primitive's bin of each axis, over the boxes of
+// its run (the same unions, hence the same bits), and the first minimum is the
+// smallest (cost, bin) pair of the run. What bounds it is instruction issue
+// (60 % of the slots), about 50 per member of the longest run and 500 per
+// level. Before, subtrees of at most 8 primitives took a thread each, which
+// left 114 us of latency at 6,400 triangles (34 now).
+__device__ void small_subtrees(const SahParams& p, SmallShared& sh, bool valid, SubTask tk, uint32_t first_lane) {
+  const uint32_t lane = threadIdx.x & 31u;
+  constexpr uint32_t all = 0xffffffffu;
+  uint32_t s = first_lane, e = first_lane + (tk.end - tk.begin);
+  const uint32_t pos = tk.begin + (lane - first_lane);  // the lane's index slot
+  if (valid) {
+    const uint32_t prim = p.idx_a[pos];
+    const DAabb b = load_aabb(p.aabbs + prim);
+    sh.centre[lane] = __ldg(p.centers + prim);
+    sh.lo[lane] = make_float4(b.min[0], b.min[1], b.min[2], 0.0f);
+    sh.hi[lane] = make_float4(b.max[0], b.max[1], b.max[2], __uint_as_float(prim));
+  }
+  bool open = valid;  // the lane's task is not finished
+  while (__any_sync(all, open)) {
+    const uint32_t ws = open ? e - s : 0u;
+    float mn[3], mx[3];
+    first_offset(tk, mn, mx);
+    const bool decide = open && ws > 1u && tk.depth < kMaxDepth;
+    uint32_t packed = 0;
+    __syncwarp();
+    if (decide) {
+      const BinMap bm = make_binmap(mn, mx);
+      const float4 c = sh.centre[lane];
+      packed = bin_of(c.x, bm.c2b[0], bm.off[0]) | bin_of(c.y, bm.c2b[1], bm.off[1]) << 4 |
+               bin_of(c.z, bm.c2b[2], bm.off[2]) << 8;
+      sh.lo[lane].w = __uint_as_float(packed);
+    }
+    __syncwarp();
+    // costs at the own primitive's bins (areas: the sign of a zero does not
+    // matter, native min/max will do)
+    float lmn[3][3], lmx[3][3], rmn[3][3], rmx[3][3];
+    uint32_t nl[3] = {0u, 0u, 0u};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        lmn[a][k] = rmn[a][k] = 1e34f;
+        lmx[a][k] = rmx[a][k] = -1e34f;
+      }
+    const uint32_t members = decide ? ws : 0u;
+    const uint32_t longest = __reduce_max_sync(all, members);
+    for (uint32_t k = 0; k < members; ++k) {
+      const float4 lo = sh.lo[s + k], hi = sh.hi[s + k];
+      const uint32_t bins = __float_as_uint(lo.w);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const bool left = (bins >> (4 * a) & 15u) <= (packed >> (4 * a) & 15u);
+        if (left) {
+          ++nl[a];
+          lmn[a][0] = fminf(lmn[a][0], lo.x); lmn[a][1] = fminf(lmn[a][1], lo.y); lmn[a][2] = fminf(lmn[a][2], lo.z);
+          lmx[a][0] = fmaxf(lmx[a][0], hi.x); lmx[a][1] = fmaxf(lmx[a][1], hi.y); lmx[a][2] = fmaxf(lmx[a][2], hi.z);
+        } else {
+          rmn[a][0] = fminf(rmn[a][0], lo.x); rmn[a][1] = fminf(rmn[a][1], lo.y); rmn[a][2] = fminf(rmn[a][2], lo.z);
+          rmx[a][0] = fmaxf(rmx[a][0], hi.x); rmx[a][1] = fmaxf(rmx[a][1], hi.y); rmx[a][2] = fmaxf(rmx[a][2], hi.z);
+        }
+      }
+    }
+    __syncwarp();
+    float best_cost[3];
+    uint32_t best_count[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      uint32_t key = all, bin = (uint32_t)kBins;  // none: above every cost below f32::MAX
+      if (decide && nl[a] < ws) {
+        const float cost = ha6(lmn[a], lmx[a]) * (float)nl[a] + ha6(rmn[a], rmx[a]) * (float)(ws - nl[a]);
+        if (cost < kF32Max) {
+          key = float_to_ordered(cost + 0.0f);  // -0 and +0 compare equal
+          bin = packed >> (4 * a) & 15u;
+        }
+      }
+      // smallest pair of the run: inclusive over [s, lane], then the last lane's
+#pragma unroll 1
+      for (uint32_t o = 1; o < longest; o <<= 1) {
+        const uint32_t ok = __shfl_up_sync(all, key, o), ob = __shfl_up_sync(all, bin, o);
+        if (lane >= s + o && pair_less(ok, ob, key, bin)) {
+          key = ok;
+          bin = ob;
+        }
+      }
+      const uint32_t last = (e - 1u) & 31u;
+      key = __shfl_sync(all, key, last);
+      bin = __shfl_sync(all, bin, last);
+      best_cost[a] = bin < (uint32_t)kBins ? ordered_to_float(key) : kF32Max;
+      best_count[a] = bin < (uint32_t)kBins ? bin + 1u : (uint32_t)kBins;
+    }
+    int axis = 0;
+    if (best_cost[0] > best_cost[1]) axis = 1;
+    if ((axis ? best_cost[1] : best_cost[0]) > best_cost[2]) axis = 2;
+    uint32_t split_index = axis == 0 ? best_count[0] : (axis == 1 ? best_count[1] : best_count[2]);
+    const float cost = axis == 0 ? best_cost[0] : (axis == 1 ? best_cost[1] : best_cost[2]);
+    const float max_split_cost = ha6(mn, mx) * ((float)ws - kTraversalCost);
+    const bool fallback = decide && (split_index == (uint32_t)kBins || cost >= max_split_cost);
+    bool leaf = !decide;
+    if (__any_sync(all, fallback)) {
+      int la = 0;
+      if ((mx[1] - mn[1]) > (mx[0] - mn[0])) la = 1;
+      if ((mx[2] - mn[2]) > (la ? mx[1] - mn[1] : mx[0] - mn[0])) la = 2;
+      // the first bin below 15 whose cumulative count reaches ws * 2 / 5 + 1
+      const uint32_t bin = packed >> (4 * la) & 15u, upto = la == 0 ? nl[0] : (la == 1 ? nl[1] : nl[2]);
+      uint32_t b = fallback && bin < (uint32_t)kBins - 1u && upto >= ws * 2u / 5u + 1u ? bin : (uint32_t)kBins;
+#pragma unroll 1
+      for (uint32_t o = 1; o < longest; o <<= 1) {
+        const uint32_t ob = __shfl_up_sync(all, b, o);
+        if (lane >= s + o) b = min(b, ob);
+      }
+      b = __shfl_sync(all, b, (e - 1u) & 31u);
+      if (fallback) {
+        if (ws <= p.max_leaf) {
+          leaf = true;
+        } else {
+          axis = la;
+          if (b < (uint32_t)kBins) split_index = b + 1u;
+        }
+      }
+    }
+    const uint32_t mine = packed >> (4 * axis) & 15u;
+    const bool goes_left = decide && !leaf && mine < split_index;
+    const uint32_t run = open ? (all >> (32u - ws)) << s : 0u;
+    const uint32_t lefts = __ballot_sync(all, goes_left) & run;
+    const uint32_t n_left = __popc(lefts);
+    const bool split = open && !leaf && n_left > 0u && n_left < ws;
+    // the children's boxes: left over the bins below best_count of the axis (a
+    // quirk of the reference), right over the bins from split_index
+    const uint32_t lcount = axis == 0 ? best_count[0] : (axis == 1 ? best_count[1] : best_count[2]);
+    uint32_t cmn[3], cmx[3];  // ordered keys: the boxes' bits count here
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      cmn[k] = float_to_ordered(1e34f);
+      cmx[k] = float_to_ordered(-1e34f);
+    }
+    const uint32_t more = split ? ws : 0u;
+    for (uint32_t k = 0; k < more; ++k) {
+      const float4 lo = sh.lo[s + k], hi = sh.hi[s + k];
+      const uint32_t b = __float_as_uint(lo.w) >> (4 * axis) & 15u;
+      if (goes_left ? b < lcount : b >= split_index) {
+        cmn[0] = min(cmn[0], float_to_ordered(lo.x));
+        cmn[1] = min(cmn[1], float_to_ordered(lo.y));
+        cmn[2] = min(cmn[2], float_to_ordered(lo.z));
+        cmx[0] = max(cmx[0], float_to_ordered(hi.x));
+        cmx[1] = max(cmx[1], float_to_ordered(hi.y));
+        cmx[2] = max(cmx[2], float_to_ordered(hi.z));
+      }
+    }
+    __syncwarp();
+    if (open && lane == s) {
+      Decision d;
+      d.split = split ? 1u : 0u;
+      d.n_left = n_left;
+      SubTask l, r;
+      sub_write(p, tk, mn, mx, d, l, r);
+    }
+    uint32_t to = lane;
+    if (split) {
+      const uint32_t before = (1u << lane) - 1u;
+      to = goes_left ? s + __popc(lefts & before) : s + n_left + __popc(run & ~lefts & before);
+    }
+    // the lane's new primitive and task (its own where nothing moved)
+    const float4 lo = sh.lo[lane], hi = sh.hi[lane], c = sh.centre[lane];
+    // both children's boxes, from a lane of either side
+    const uint32_t lsrc = split ? (uint32_t)__ffs(lefts) - 1u : lane;
+    const uint32_t rsrc = split ? (uint32_t)__ffs(run & ~lefts) - 1u : lane;
+    __syncwarp();
+    if (split) {
+      sh.lo[to] = lo;
+      sh.hi[to] = hi;
+      sh.centre[to] = c;
+    }
+    const uint32_t m = tk.begin + n_left;
+    const bool now_left = lane < s + n_left;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const uint32_t bl = __shfl_sync(all, cmn[k], lsrc), br = __shfl_sync(all, cmn[k], rsrc);
+      const uint32_t tl = __shfl_sync(all, cmx[k], lsrc), tr = __shfl_sync(all, cmx[k], rsrc);
+      if (split) {
+        tk.box[k] = ordered_to_float(now_left ? bl : br);
+        tk.box[3 + k] = ordered_to_float(now_left ? tl : tr);
+      }
+    }
+    if (split) {
+      tk.loc = kTemp | (2u * (m - 1u) + (now_left ? 0u : 1u));
+      tk.depth += 1u;
+      if (now_left) {
+        tk.end = m;
+        e = s + n_left;
+      } else {
+        tk.begin = m;
+        s += n_left;
+      }
+    } else {
+      open = false;
+    }
+  }
+  __syncwarp();
+  if (valid) p.idx_a[pos] = __float_as_uint(sh.hi[lane].w);
+  __syncwarp();
 }
 
 // ------------------------------------------------------------------ level scan + emit
@@ -1338,23 +1397,65 @@ __global__ void __launch_bounds__(kSubBlock) k_sub_build(SahParams p) {
   SubShared& sh = reinterpret_cast<SubShared*>(sub_dyn)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t S = __ldcg(&p.cnt->sub);
+  SmallList list;  // lane 0's
   for (;;) {
     uint32_t t = 0;
     if (lane == 0) t = atomicAdd(&p.cnt->sub_head, 1u);
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t >= S) break;
-    sub_warp_tree(p, ld_task(p.subs + t), sh);
+    sub_warp_tree(p, ld_task(p.subs + t), sh, list);
   }
+  if (lane == 0) list.finish(p);
 }
 
-// The listed subtrees of at most kThreadMax primitives, one thread each
-// (two blocks per SM: 128 registers, 16 bytes of spills, twice the warps of
-// the unbounded 143-register form).
-__global__ void __launch_bounds__(kLargeBlock, 2) k_sub_tiny(SahParams p) {
-  const uint32_t T = __ldcg(&p.cnt->tiny);
+// The listed subtrees of at most kSmall primitives: a warp takes 32 entries at a
+// time and builds as many of them side by side as fit its lanes.
+__global__ void __launch_bounds__(kSubBlock) k_sub_small(SahParams p) {
+  __shared__ SmallShared sh[kSubBlock / 32];
+  const uint32_t lane = threadIdx.x & 31u;
+  constexpr uint32_t all = 0xffffffffu;
+  const uint32_t T = min(__ldcg(&p.cnt->tiny), p.small_cap);
   const SubTask* list = reinterpret_cast<const SubTask*>(p.tiny);
-  for (uint32_t t = blockIdx.x * kLargeBlock + threadIdx.x; t < T && t < p.n; t += gridDim.x * kLargeBlock)
-    sub_tiny(p, list[t]);
+  for (;;) {
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&p.cnt->tiny_head, 32u);
+    base = __shfl_sync(all, base, 0);
+    if (base >= T) break;
+    SubTask mine = {};
+    if (base + lane < T) mine = list[base + lane];
+    uint32_t size = mine.end - mine.begin;
+    if (size > kSmall) {
+      atomicOr(&p.cnt->status, kStatusBadIndex);
+      size = 0;
+    }
+    uint32_t incl = size;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(all, incl, o);
+      if (lane >= (uint32_t)o) incl += v;
+    }
+    const uint32_t total = __shfl_sync(all, incl, 31);
+    for (uint32_t done = 0; done < total;) {
+      // the entries after the first `done` primitives that fit 32 lanes
+      const bool in = size > 0u && incl > done && incl <= done + 32u;
+      SmallShared& own = sh[threadIdx.x >> 5];
+      if (in) own.entry[incl - size - done] = (uint8_t)lane;
+      __syncwarp();
+      const uint32_t starts = __reduce_or_sync(all, in ? 1u << (incl - size - done) : 0u);
+      const uint32_t used = __reduce_max_sync(all, in ? incl : done) - done;
+      const uint32_t first = 31u - __clz(starts & (all >> (31u - lane)));  // start of the lane's entry
+      const uint32_t src = own.entry[first];
+      SubTask tk;
+      tk.loc = __shfl_sync(all, mine.loc, src);
+      tk.begin = __shfl_sync(all, mine.begin, src);
+      tk.end = __shfl_sync(all, mine.end, src);
+      tk.depth = __shfl_sync(all, mine.depth, src);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) tk.box[k] = __shfl_sync(all, mine.box[k], src);
+      small_subtrees(p, own, lane < used, tk, first);
+      done += used;
+    }
+  }
 }
 
 constexpr uint32_t kScanTile = 4096;  // split positions per tile: 1024 threads x 4
@@ -1522,6 +1623,16 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   const uint32_t sub_cap = n + 1;
   const uint32_t chunk_cap = n / kChunk + large_cap + 2;
   const uint32_t tiles = (n + kScanTile - 1) / kScanTile;
+  int sub_per_sm = 0;
+  const size_t sub_smem = (kSubBlock / 32) * sizeof(SubShared);
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sub_per_sm, k_sub_build, kSubBlock, sub_smem)))
+    return fail(cuda_rc(e));
+  if (sub_per_sm < 1) return fail(DeviceError);
+  uint32_t sub_grid = (uint32_t)sm_count() * (uint32_t)sub_per_sm;
+  const uint32_t want = (n / (sub_max > 8u ? 8u : sub_max) + kSubBlock / 32) / (kSubBlock / 32) + 1u;
+  if (want < sub_grid) sub_grid = want;
+  // listed subtrees hold a primitive or more; every warp may leave a chunk
+  const uint32_t small_cap = n + sub_grid * (kSubBlock / 32) * kListChunk;
   Scratch<DAabb> world, tnodes;
   Scratch<uint32_t> acc, idx_b, bins, chunk_base, chunk_status, sflag, srank, tile_off;
   Scratch<Task> large0, large1, subs;
@@ -1537,7 +1648,7 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
       (e = subs.alloc(sub_cap, s)) || (e = dec.alloc(large_cap, s)) || (e = tbox.alloc((size_t)large_cap * 6, s)) ||
       (e = scan_vals.alloc(large_cap, s)) || (e = scan_sums.alloc(grid, s)) || (e = cnt.alloc(1, s)) ||
       (e = bar.alloc(1, s)) || (e = tnodes.alloc(2 * (size_t)n, s)) || (e = sflag.alloc(n, s)) ||
-      (e = srank.alloc(n, s)) || (e = tile_off.alloc(tiles + 1, s)) || (e = tiny.alloc(n, s)))
+      (e = srank.alloc(n, s)) || (e = tile_off.alloc(tiles + 1, s)) || (e = tiny.alloc(small_cap, s)))
     return fail(cuda_rc(e));
   if ((e = cudaMemsetAsync(chunk_status.ptr, 0, (size_t)chunk_cap * 4, s)) ||
       (e = cudaMemsetAsync(bar.ptr, 0, sizeof(GridBarrier), s)) ||
@@ -1558,6 +1669,7 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   p.large[1] = large1.ptr;
   p.subs = subs.ptr;
   p.tiny = tiny.ptr;
+  p.small_cap = small_cap;
   p.dec = dec.ptr;
   p.tbox = tbox.ptr;
   p.bins = bins.ptr;
@@ -1607,22 +1719,13 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   // kernels read the subtree count and the breadth-first node count on the
   // device)
   {
-    int sub_per_sm = 0;
-    const size_t sub_smem = (kSubBlock / 32) * sizeof(SubShared);
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sub_per_sm, k_sub_build, kSubBlock, sub_smem)))
-      return fail(cuda_rc(e));
-    if (sub_per_sm < 1) return fail(DeviceError);
-    uint32_t sub_grid = (uint32_t)sm_count() * (uint32_t)sub_per_sm;
-    const uint32_t want = (n / (sub_max > 8u ? 8u : sub_max) + kSubBlock / 32) / (kSubBlock / 32) + 1u;
-    if (want < sub_grid) sub_grid = want;
     k_sub_build<<<sub_grid, kSubBlock, sub_smem, s>>>(p);
-    {
-      int tiny_per_sm = 0;
-      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tiny_per_sm, k_sub_tiny, kLargeBlock, 0)))
-        return fail(cuda_rc(e));
-      const uint32_t tiny_grid = (uint32_t)sm_count() * (uint32_t)(tiny_per_sm < 1 ? 1 : tiny_per_sm);
-      k_sub_tiny<<<tiny_grid, kLargeBlock, 0, s>>>(p);
-    }
+    int small_per_sm = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&small_per_sm, k_sub_small, kSubBlock, 0)))
+      return fail(cuda_rc(e));
+    const uint32_t small_grid = (uint32_t)sm_count() * (uint32_t)(small_per_sm < 1 ? 1 : small_per_sm);
+    const uint32_t small_want = (small_cap / 32u + kSubBlock / 32) / (kSubBlock / 32);
+    k_sub_small<<<small_want < small_grid ? small_want : small_grid, kSubBlock, 0, s>>>(p);
     k_tile_sums<<<tiles, 1024, 0, s>>>(sflag.ptr, n, tile_off.ptr);
     k_tile_scan<<<1, 1024, 0, s>>>(tile_off.ptr, tiles, cnt.ptr);
     k_rank<<<tiles, 1024, 0, s>>>(sflag.ptr, n, tile_off.ptr, srank.ptr);
