@@ -49,7 +49,8 @@ constexpr uint32_t kMaxDepth = 64;
 constexpr float kTraversalCost = 1.0f;
 constexpr int kChunk = 2048;
 constexpr int kLargeBlock = 256;
-constexpr uint32_t kWarpMax = 1024;
+constexpr uint32_t kWarpMax = 1024;  // largest subtree
+constexpr uint32_t kTaskWarp = 64;  // largest task of k_sah_build's lists that one warp does
 constexpr uint32_t kCoopMaxPrims = 1u << 20;      // larger builds launch the phases separately
 constexpr int kBinWords = 8;  // ordered min xyz, ordered max xyz, count, pad
 constexpr int kTaskBinWords = 3 * kBins * kBinWords;
@@ -72,6 +73,7 @@ static_assert(sizeof(Decision) == 80, "Decision layout");
 
 struct Counters {
   uint32_t large;       // tasks in the current large list
+  uint32_t big[2];      // k_sah_build: whether the list of an even / odd level has tasks above kChunk
   uint32_t sub;         // subtree tasks listed so far (all levels)
   uint32_t node_count;  // nodes of the breadth-first part so far
   uint32_t chunks;      // chunks of the current large list
@@ -380,6 +382,7 @@ struct Level {
   const Task* large;
   Task* large_next;
   uint32_t L, node_base, sub_base;
+  uint32_t next_parity;  // of the next level
 };
 
 // Reads of data written earlier in the same launch (by any block) go to L2:
@@ -421,25 +424,37 @@ struct alignas(16) SahShared {
   uint64_t scan[kLargeBlock / 32];
   uint32_t warp[32];
   uint32_t chunk, fail, prefix, pad;
+  uint32_t chunk_idx[kChunk];                      // the indices of a chunk
   uint32_t bins[kLargeBlock / 32][kTaskBinWords];  // per-warp bins
   Decision dec[kLargeBlock / 32];
-  uint32_t idx[kLargeBlock / 32][kWarpMax];        // per-warp partition buffer
+  uint32_t idx[kLargeBlock / 32][kTaskWarp];       // per-warp partition buffer
 };
-constexpr size_t kShSmall = offsetof(SahShared, bins);  // scans, partition scalars
-constexpr size_t kShBins = offsetof(SahShared, dec);    // + per-warp bins
+constexpr size_t kShSmall = offsetof(SahShared, chunk_idx);  // scans, partition scalars
+constexpr size_t kShBins = offsetof(SahShared, dec);         // + a chunk's indices, per-warp bins
 
-// Bins primitives sidx-ordered positions [i0, i1) into `wb` (one warp's or
-// block's shared bins). Neighbours in the index array are usually neighbours
-// in space and share bins, so a run of primitives in one bin is merged in
-// registers and written with atomics only when an axis changes bin.
+// Bins the primitives at positions [i0, i1) of every lane of a warp into `wb`
+// (the warp's own shared bins; all 32 lanes call it). Neighbours in the index
+// array are usually neighbours in space and share bins, so a lane merges a run
+// of primitives in one bin in registers. At the end the lanes' last runs,
+// which usually share a few bins, are merged over the warp bin by bin and
+// written by one atomic per word; atomics of all lanes on one bin would take
+// their turns. The next primitive is loaded before the current one is binned.
+// What bounds it is the latency of these loads. One lane at a time and atomics
+// of every lane took 58 us for an 800-primitive task of one warp.
 template <class IdxFn>
 __device__ __forceinline__ void bin_run(const SahParams& p, const BinMap& bm, uint32_t i0, uint32_t i1, IdxFn idx,
                                         uint32_t* wb) {
+  constexpr uint32_t all = 0xffffffffu;
   uint32_t rbin[3], rmn[3][3], rmx[3][3], rcnt[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    rbin[a] = 0xffffffffu;
+    rbin[a] = all;
     rcnt[a] = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      rmn[a][q] = all;
+      rmx[a][q] = 0u;
+    }
   }
   auto flush = [&](int a) {
     if (rcnt[a] == 0) return;
@@ -451,11 +466,16 @@ __device__ __forceinline__ void bin_run(const SahParams& p, const BinMap& bm, ui
     }
     atomicAdd(b + 6, rcnt[a]);
   };
+  float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  DAabb box = {};
+  auto load = [&](uint32_t i) {
+    const uint32_t prim = idx(i);
+    c = __ldg(p.centers + prim);
+    box = load_aabb(p.aabbs + prim);
+  };
+  if (i0 < i1) load(i0);
 #pragma unroll 1
   for (uint32_t i = i0; i < i1; ++i) {
-    const uint32_t prim = idx(i);
-    const float4 c = __ldg(p.centers + prim);
-    const DAabb box = load_aabb(p.aabbs + prim);
     const float cc[3] = {c.x, c.y, c.z};
     uint32_t kmn[3], kmx[3];
 #pragma unroll
@@ -463,6 +483,7 @@ __device__ __forceinline__ void bin_run(const SahParams& p, const BinMap& bm, ui
       kmn[q] = float_to_ordered(box.min[q]);
       kmx[q] = float_to_ordered(box.max[q]);
     }
+    if (i + 1u < i1) load(i + 1u);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const uint32_t bin = bin_of(cc[a], bm.c2b[a], bm.off[a]);
@@ -484,14 +505,43 @@ __device__ __forceinline__ void bin_run(const SahParams& p, const BinMap& bm, ui
       ++rcnt[a];
     }
   }
+  __syncwarp();
+  const uint32_t lane = threadIdx.x & 31u;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) flush(a);
+  for (int a = 0; a < 3; ++a) {
+    uint32_t pending = __ballot_sync(all, rcnt[a] != 0u);
+    // bins that four lanes or more hold, as long as many lanes are left
+#pragma unroll 1
+    for (int round = 0; round < 4 && __popc(pending) >= 8; ++round) {
+      const uint32_t b = __shfl_sync(all, rbin[a], __ffs(pending) - 1);
+      const bool in = rcnt[a] != 0u && rbin[a] == b;
+      const uint32_t group = __ballot_sync(all, in);
+      if (__popc(group) < 4) break;
+      uint32_t v = 0;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const uint32_t mn = __reduce_min_sync(all, in ? rmn[a][q] : all);
+        const uint32_t mx = __reduce_max_sync(all, in ? rmx[a][q] : 0u);
+        if (lane == (uint32_t)q) v = mn;
+        if (lane == 3u + (uint32_t)q) v = mx;
+      }
+      const uint32_t n = __reduce_add_sync(all, in ? rcnt[a] : 0u);
+      uint32_t* w = wb + (a * kBins + b) * kBinWords + lane;
+      if (lane < 3u) atomicMin(w, v);
+      else if (lane < 6u) atomicMax(w, v);
+      else if (lane == 6u) atomicAdd(w, n);
+      if (in) rcnt[a] = 0u;
+      pending &= ~group;
+    }
+    flush(a);
+  }
 }
 
 // ------------------------------------------------------------------ large tasks
 // Block 0: task boxes (with the first 1e-4 offset) and chunk offsets of the
 // level's large tasks.
-__device__ void large_prep(const SahParams& p, const Level& lv, SahShared& sh) {
+// `above`: tasks of at most so many primitives get no chunks (a warp does them).
+__device__ void large_prep(const SahParams& p, const Level& lv, SahShared& sh, uint32_t above) {
   uint32_t carry = 0;
   for (uint32_t base = 0; base < lv.L; base += kLargeBlock) {
     const uint32_t t = base + threadIdx.x;
@@ -507,7 +557,7 @@ __device__ void large_prep(const SahParams& p, const Level& lv, SahShared& sh) {
         tb[3 + k] = mx[k];
       }
       const uint32_t ws = tk.end - tk.begin;
-      if (ws > 1 && tk.depth < kMaxDepth) chunks = (ws + kChunk - 1) / kChunk;
+      if (ws > above && tk.depth < kMaxDepth) chunks = (ws + kChunk - 1) / kChunk;
     }
     uint32_t total;
     const uint32_t incl = block_inclusive_scan<kLargeBlock>(chunks, sh.warp, &total);
@@ -541,6 +591,7 @@ __device__ void large_bin_chunk(const SahParams& p, const Level& lv, uint32_t ch
   const uint32_t c0 = tk.begin + k * kChunk;
   const uint32_t c1 = min(c0 + kChunk, tk.end);
   init_bins(&sh.bins[warp][0], threadIdx.x & 31, 32);
+  for (uint32_t i = c0 + threadIdx.x; i < c1; i += kLargeBlock) sh.chunk_idx[i - c0] = __ldcg(p.idx_a + i);
   __syncthreads();
   float mn[3], mx[3];
   ld_tbox(p.tbox + 6 * (size_t)t, mn, mx);
@@ -549,7 +600,7 @@ __device__ void large_bin_chunk(const SahParams& p, const Level& lv, uint32_t ch
   // each thread bins kChunk / kLargeBlock consecutive primitives
   constexpr uint32_t PER = kChunk / kLargeBlock;
   const uint32_t s0 = c0 + threadIdx.x * PER;
-  bin_run(p, bm, min(s0, c1), min(s0 + PER, c1), [&](uint32_t i) { return __ldcg(p.idx_a + i); }, wb);
+  bin_run(p, bm, min(s0, c1), min(s0 + PER, c1), [&](uint32_t i) { return sh.chunk_idx[i - c0]; }, wb);
   __syncthreads();
   uint32_t* gb = p.bins + (size_t)t * kTaskBinWords;
   for (int i = threadIdx.x; i < 3 * kBins; i += kLargeBlock) {
@@ -601,6 +652,11 @@ __device__ void large_decide(const SahParams& p, const Level& lv, uint32_t t, Sa
     p.dec[t] = d;
   }
 }
+
+// Task t whole -- bins, decision and partition -- by one warp (at most kTaskWarp
+// primitives) or by the block (at most a chunk).
+__device__ void large_task_warp(const SahParams& p, const Level& lv, uint32_t t, SahShared& sh);
+__device__ void large_task_block(const SahParams& p, const Level& lv, uint32_t t, SahShared& sh);
 
 // Stable partition of a large task's chunk into idx_b; the number of left
 // primitives in the task's earlier chunks comes from a decoupled look-back
@@ -718,7 +774,7 @@ __device__ void decide_warp(const SahParams& p, uint32_t begin, uint32_t ws, uin
   if (ws > 1 && depth < kMaxDepth && ws <= kWarpMax) {
     init_bins(wb, lane, 32);
     // stage the task's indices (independent loads, all in flight at once)
-    for (uint32_t i = lane; i < ws; i += 32) sidx[i] = p.idx_a[begin + i];
+    for (uint32_t i = lane; i < ws; i += 32) sidx[i] = __ldcg(p.idx_a + begin + i);
     __syncwarp();
     const BinMap bm = make_binmap(mn, mx);
     {
@@ -766,6 +822,86 @@ __device__ void decide_warp(const SahParams& p, uint32_t begin, uint32_t ws, uin
     }
   }
   __syncwarp();
+}
+
+__device__ void large_task_warp(const SahParams& p, const Level& lv, uint32_t t, SahShared& sh) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Task tk = ld_task(lv.large + t);
+  float mn[3], mx[3];
+  task_box(p.nodes, tk.node, mn, mx);
+  decide_warp(p, tk.begin, tk.end - tk.begin, tk.depth, mn, mx, sh.bins[warp], sh.idx[warp], sh.dec[warp]);
+  if (lane == 0) {
+    if (sh.dec[warp].split) write_interior_box(p.nodes, tk.node, mn, mx);
+    else write_leaf(p.nodes, tk, mn, mx);
+    p.dec[t] = sh.dec[warp];
+  }
+  __syncwarp();
+}
+
+__device__ void large_task_block(const SahParams& p, const Level& lv, uint32_t t, SahShared& sh) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Task tk = ld_task(lv.large + t);
+  const uint32_t ws = tk.end - tk.begin;
+  float mn[3], mx[3];
+  task_box(p.nodes, tk.node, mn, mx);
+  if (threadIdx.x == 0) sh.dec[0].split = 0;
+  if (ws > 1 && tk.depth < kMaxDepth) {
+    init_bins(&sh.bins[warp][0], lane, 32);
+    for (uint32_t i = threadIdx.x; i < ws; i += kLargeBlock) sh.chunk_idx[i] = __ldcg(p.idx_a + tk.begin + i);
+    __syncthreads();
+    const BinMap bm = make_binmap(mn, mx);
+    const uint32_t per = (ws + kLargeBlock - 1) / kLargeBlock;
+    const uint32_t i0 = min(threadIdx.x * per, ws), i1 = min(i0 + per, ws);
+    bin_run(p, bm, i0, i1, [&](uint32_t i) { return sh.chunk_idx[i]; }, &sh.bins[warp][0]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 3 * kBins; i += kLargeBlock) {
+      uint32_t* b0 = &sh.bins[0][i * kBinWords];
+      for (int w = 1; w < kLargeBlock / 32; ++w) {
+        const uint32_t* b = &sh.bins[w][i * kBinWords];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          b0[q] = min(b0[q], b[q]);
+          b0[3 + q] = max(b0[3 + q], b[3 + q]);
+        }
+        b0[6] += b[6];
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      Decision d;
+      sah_decide_warp(BinsView{&sh.bins[0][0]}, mn, mx, ws, p.max_leaf, d);
+      if (lane == 0) sh.dec[0] = d;
+    }
+    __syncthreads();
+    if (sh.dec[0].split) {
+      const int ax = (int)sh.dec[0].axis;
+      const uint32_t split_index = sh.dec[0].split_index;
+      uint32_t flags = 0, mine = 0;  // per <= 8
+      for (uint32_t i = i0; i < i1; ++i) {
+        const float4 c = __ldg(p.centers + sh.chunk_idx[i]);
+        const float cc = ax == 0 ? c.x : (ax == 1 ? c.y : c.z);
+        if (bin_of(cc, bm.c2b[ax], bm.off[ax]) < split_index) {
+          flags |= 1u << (i - i0);
+          ++mine;
+        }
+      }
+      uint32_t total;
+      const uint32_t before = block_inclusive_scan<kLargeBlock>(mine, sh.warp, &total) - mine;
+      uint32_t tpos = tk.begin + before, fpos = tk.begin + sh.dec[0].n_left + (i0 - before);
+      for (uint32_t i = i0; i < i1; ++i) {
+        const uint32_t dst = ((flags >> (i - i0)) & 1u) ? tpos++ : fpos++;
+        if (dst < tk.end) p.idx_a[dst] = sh.chunk_idx[i];
+        else atomicOr(&p.cnt->status, kStatusBadIndex);
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (sh.dec[0].split) write_interior_box(p.nodes, tk.node, mn, mx);
+    else write_leaf(p.nodes, tk, mn, mx);
+    p.dec[t] = sh.dec[0];
+  }
+  __syncthreads();
 }
 
 // ------------------------------------------------------------------ subtrees
@@ -1212,6 +1348,34 @@ __device__ void scan_segment(const SahParams& p, const Level& lv, SahShared& sh)
 
 // Node numbering (breadth first), the next level's task list and the
 // subtree list.
+__device__ void emit_children(const SahParams& p, const Level& lv, const Decision& d, const Task& tk, uint64_t ex) {
+  uint32_t li = (uint32_t)(ex >> 32), si = (uint32_t)(ex & 0xffffffffu);
+  const uint32_t child = lv.node_base + li + si;
+  DAabb nd = load_aabb_cg(p.nodes + tk.node);
+  nd.left_first = (int32_t)child;
+  nd.count = -1;
+  store_aabb(p.nodes + tk.node, nd);
+  DAabb lb, rb;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    lb.min[k] = d.lbox[k];
+    lb.max[k] = d.lbox[3 + k];
+    rb.min[k] = d.rbox[k];
+    rb.max[k] = d.rbox[3 + k];
+  }
+  lb.count = rb.count = 0;
+  lb.left_first = rb.left_first = 0;
+  store_aabb(p.nodes + child, lb);
+  store_aabb(p.nodes + child + 1, rb);
+  const Task lt{child, tk.begin, tk.begin + d.n_left, tk.depth + 1};
+  const Task rt{child + 1, tk.begin + d.n_left, tk.end, tk.depth + 1};
+  if (lt.end - lt.begin > p.sub_max) lv.large_next[li++] = lt;
+  else p.subs[lv.sub_base + si++] = lt;
+  if (rt.end - rt.begin > p.sub_max) lv.large_next[li++] = rt;
+  else p.subs[lv.sub_base + si++] = rt;
+  if (max(d.n_left, tk.end - tk.begin - d.n_left) > (uint32_t)kChunk) p.cnt->big[lv.next_parity] = 1u;
+}
+
 __device__ void emit_segment(const SahParams& p, const Level& lv, SahShared& sh, bool advance) {
   // prefix of the block totals before this block, and the level total
   uint64_t before = 0, all = 0;
@@ -1229,36 +1393,37 @@ __device__ void emit_segment(const SahParams& p, const Level& lv, SahShared& sh,
   segment(lv.L, lo, hi);
   for (uint32_t t = lo + threadIdx.x; t < hi; t += kLargeBlock) {
     const Decision d = ld_dec(p.dec + t);
-    if (!d.split) continue;
-    const Task tk = level_task(lv, t);
-    const uint64_t ex = __ldcg(p.scan_vals + t) + before;
-    uint32_t li = (uint32_t)(ex >> 32), si = (uint32_t)(ex & 0xffffffffu);
-    const uint32_t child = lv.node_base + li + si;
-    DAabb nd = load_aabb_cg(p.nodes + tk.node);
-    nd.left_first = (int32_t)child;
-    nd.count = -1;
-    store_aabb(p.nodes + tk.node, nd);
-    DAabb lb, rb;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      lb.min[k] = d.lbox[k];
-      lb.max[k] = d.lbox[3 + k];
-      rb.min[k] = d.rbox[k];
-      rb.max[k] = d.rbox[3 + k];
-    }
-    lb.count = rb.count = 0;
-    lb.left_first = rb.left_first = 0;
-    store_aabb(p.nodes + child, lb);
-    store_aabb(p.nodes + child + 1, rb);
-    const Task lt{child, tk.begin, tk.begin + d.n_left, tk.depth + 1};
-    const Task rt{child + 1, tk.begin + d.n_left, tk.end, tk.depth + 1};
-    if (lt.end - lt.begin > p.sub_max) lv.large_next[li++] = lt;
-    else p.subs[lv.sub_base + si++] = lt;
-    if (rt.end - rt.begin > p.sub_max) lv.large_next[li++] = rt;
-    else p.subs[lv.sub_base + si++] = rt;
+    if (d.split) emit_children(p, lv, d, level_task(lv, t), __ldcg(p.scan_vals + t) + before);
   }
   if (advance && blockIdx.x == 0 && threadIdx.x == 0) {
     const uint32_t nl = (uint32_t)(all >> 32), ns = (uint32_t)(all & 0xffffffffu);
+    p.cnt->node_count = lv.node_base + nl + ns;
+    p.cnt->large = nl;
+    p.cnt->sub = lv.sub_base + ns;
+  }
+}
+
+// Scan and emission of a level of few tasks by one block.
+constexpr uint32_t kFewTasks = 4u * kLargeBlock;
+__device__ void scan_emit_block(const SahParams& p, const Level& lv, SahShared& sh) {
+  uint64_t carry = 0;
+  for (uint32_t base = 0; base < lv.L; base += kLargeBlock) {
+    const uint32_t t = base + threadIdx.x;
+    Decision d;
+    d.split = 0;
+    Task tk{0u, 0u, 0u, 0u};
+    if (t < lv.L) {
+      d = ld_dec(p.dec + t);
+      tk = level_task(lv, t);
+    }
+    const uint64_t v = t < lv.L ? children_value(d, tk, p.sub_max) : 0ull;
+    uint64_t total;
+    const uint64_t incl = block_scan_incl<uint64_t>(v, sh.scan, &total);
+    if (d.split) emit_children(p, lv, d, tk, carry + incl - v);
+    carry += total;
+  }
+  if (threadIdx.x == 0) {
+    const uint32_t nl = (uint32_t)(carry >> 32), ns = (uint32_t)(carry & 0xffffffffu);
     p.cnt->node_count = lv.node_base + nl + ns;
     p.cnt->large = nl;
     p.cnt->sub = lv.sub_base + ns;
@@ -1284,46 +1449,71 @@ __device__ __forceinline__ Level read_level(const SahParams& p, uint32_t level) 
   lv.sub_base = __ldcg(&p.cnt->sub);
   lv.large = p.large[level & 1];
   lv.large_next = p.large[(level + 1) & 1];
+  lv.next_parity = (level + 1) & 1;
   return lv;
 }
 
 // The breadth-first part of the build: one cooperative launch, the levels of
 // the tree one after another, phases separated by grid barriers. Level l
-// reads task list large[l & 1] and writes the other one.
+// reads task list large[l & 1] and writes the other one. What bounds it is the
+// number of barriers (about 5 us each with the dependent reads around them):
+// tasks of at most a chunk are done whole by a block or, up to kTaskWarp
+// primitives, a warp, so a level of such tasks needs no binning and partition
+// phases, and a level of few tasks is numbered by block 0 alone -- two
+// barriers instead of six. 6,400 triangles 397 -> 220 us (12 levels); a warp for
+// tasks of up to 256 instead of 64 costs 10 us there.
 __global__ void __launch_bounds__(kLargeBlock, 2) k_sah_build(SahParams p) {
   __shared__ SahShared sh;
   const uint32_t G = gridDim.x;
   const uint32_t gwarp = (blockIdx.x * kLargeBlock + threadIdx.x) >> 5, nwarps = G * (kLargeBlock / 32);
+  // a level's few tasks go to different blocks first
+  const uint32_t spread = (threadIdx.x >> 5) * G + blockIdx.x;
   uint32_t* status = &p.cnt->status;
   for (uint32_t level = 0;; ++level) {
     const Level lv = read_level(p, level);
+    const bool big = __ldcg(&p.cnt->big[level & 1]) != 0u;
     if (lv.L == 0) break;
     if (level > kMaxDepth + 1) {
       if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(status, kStatusBadIndex);
       break;
     }
     uint32_t chunks = 0;
-    if (lv.L > 0) {
-      if (blockIdx.x == 0) large_prep(p, lv, sh);
+    if (big) {
+      if (blockIdx.x == 0) large_prep(p, lv, sh, kChunk);
       large_bins_init(p, lv);
       if (!grid_sync(p.bar, G, status)) return;
       chunks = __ldcg(&p.cnt->chunks);
       for (uint32_t c = blockIdx.x; c < chunks; c += G) large_bin_chunk(p, lv, c, sh);
       if (!grid_sync(p.bar, G, status)) return;
-      for (uint32_t t = gwarp; t < lv.L; t += nwarps) large_decide(p, lv, t, sh);
+    }
+    for (uint32_t t = blockIdx.x; t < lv.L; t += G) {  // the same tasks for every thread of the block
+      const Task tk = ld_task(lv.large + t);
+      const uint32_t ws = tk.end - tk.begin;
+      if (ws > kTaskWarp && ws <= (uint32_t)kChunk) large_task_block(p, lv, t, sh);
+    }
+    for (uint32_t t = nwarps > lv.L ? spread : gwarp; t < lv.L; t += nwarps) {
+      const Task tk = ld_task(lv.large + t);
+      const uint32_t ws = tk.end - tk.begin;
+      if (ws > (uint32_t)kChunk) large_decide(p, lv, t, sh);
+      else if (ws <= kTaskWarp) large_task_warp(p, lv, t, sh);
     }
     if (!grid_sync(p.bar, G, status)) return;
-    // large partitions (chunks in ticket order)
-    if (lv.L > 0) large_partition_phase(p, lv, chunks, sh);
-    if (!grid_sync(p.bar, G, status)) return;
-    if (lv.L > 0) {
+    if (big) {
+      // large partitions (chunks in ticket order)
+      large_partition_phase(p, lv, chunks, sh);
+      if (!grid_sync(p.bar, G, status)) return;
       for (uint32_t c = blockIdx.x; c < chunks; c += G) large_copyback_chunk(p, lv, c);
       for (uint32_t c = blockIdx.x * kLargeBlock + threadIdx.x; c < chunks; c += G * kLargeBlock)
         p.chunk_status[c] = 0;
     }
-    scan_segment(p, lv, sh);
-    if (!grid_sync(p.bar, G, status)) return;
-    emit_segment(p, lv, sh, true);
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.cnt->big[level & 1] = 0u;  // the level after the next sets it again
+    if (lv.L <= kFewTasks) {
+      if (blockIdx.x == 0) scan_emit_block(p, lv, sh);
+    } else {
+      scan_segment(p, lv, sh);
+      if (!grid_sync(p.bar, G, status)) return;
+      emit_segment(p, lv, sh, true);
+    }
     if (!grid_sync(p.bar, G, status)) return;
   }
 }
@@ -1340,7 +1530,7 @@ __device__ __forceinline__ SahShared& dyn_shared() {
 __global__ void __launch_bounds__(kLargeBlock) k_ph_prep(SahParams p, uint32_t level) {
   SahShared& sh = dyn_shared();
   const Level lv = read_level(p, level);
-  if (blockIdx.x == 0) large_prep(p, lv, sh);
+  if (blockIdx.x == 0) large_prep(p, lv, sh, 1u);
   large_bins_init(p, lv);
 }
 __global__ void __launch_bounds__(kLargeBlock) k_ph_bin(SahParams p, uint32_t level) {
@@ -1569,6 +1759,8 @@ __global__ void k_sah_init(SahParams p, const DAabb* world) {
       p.cnt->sub = 1;
     }
     p.cnt->node_count = 1;
+    p.cnt->big[0] = p.n > (uint32_t)kChunk ? 1u : 0u;
+    p.cnt->big[1] = 0u;
     p.cnt->status = 0;
     p.cnt->chunks = 0;
     p.cnt->ticket = 0;
@@ -1601,12 +1793,11 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
     return rc;
   };
   // The breadth-first part of builds up to kCoopMaxPrims runs as one
-  // cooperative launch on the full resident grid: the middle levels hold
-  // many small tasks, each binned and partitioned as its own chunk, and a
-  // grid sized to the primitive count (one block per 512) left each block
-  // a long serial loop of them (6,400 triangles: 0.96 -> 0.73 ms with the
-  // full grid; the cheaper barriers of the small grid did not make up for
-  // it). Large builds launch the phases separately, which lets each phase
+  // cooperative launch: the middle levels hold many small tasks, so the grid
+  // covers every SM, with one block each for small builds, whose time is the
+  // barriers', and the full resident grid above (builds with both trees, one
+  // block against two: 20k triangles 723 / 780 us, 100k 1,217 / 1,176, 400k
+  // 2,047 / 1,887). Large builds launch the phases separately, which lets each phase
   // run at its own occupancy, and read the level's counts back between
   // levels.
   const bool coop = n <= kCoopMaxPrims;
@@ -1616,7 +1807,7 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
                                                          kLargeBlock, coop ? 0 : kShSmall)))
     return fail(cuda_rc(e));
   if (per_sm < 1) return fail(DeviceError);
-  const uint32_t grid = (uint32_t)sm_count() * (uint32_t)per_sm;
+  const uint32_t grid = (uint32_t)sm_count() * (coop && n <= 65536u ? 1u : (uint32_t)per_sm);
   uint32_t sub_max = n / 2048u;
   sub_max = sub_max < 32u ? 32u : (sub_max > kWarpMax ? kWarpMax : sub_max);
   const uint32_t large_cap = n / (sub_max + 1) + 2;
