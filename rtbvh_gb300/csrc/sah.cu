@@ -73,6 +73,7 @@ static_assert(sizeof(Decision) == 80, "Decision layout");
 
 struct Counters {
   uint32_t large;       // tasks in the current large list
+  uint32_t next_large, next_sub;  // large tasks and subtrees of the level numbered by one block
   uint32_t big[2];      // k_sah_build: whether the list of an even / odd level has tasks above kChunk
   uint32_t sub;         // subtree tasks listed so far (all levels)
   uint32_t node_count;  // nodes of the breadth-first part so far
@@ -353,7 +354,7 @@ struct SahParams {
   const float4* centers;
   DAabb* nodes;
   uint32_t* idx_a;  // primitive indices (final output)
-  uint32_t* idx_b;  // partition scratch
+  uint32_t* idx_b;  // the other index array of the levels (see Level)
   uint32_t n;
   uint32_t max_leaf;
   uint32_t sub_max;     // largest task built as a subtree (<= kWarpMax)
@@ -382,7 +383,12 @@ struct Level {
   const Task* large;
   Task* large_next;
   uint32_t L, node_base, sub_base;
-  uint32_t next_parity;  // of the next level
+  uint32_t parity, next_parity;  // of this level and the next
+  // Indices: a level reads its tasks' ranges from one array and leaves the
+  // partitioned ranges in the other (idx_a at even levels, as the final
+  // output is: a task that ends at an odd level is copied there).
+  const uint32_t* src;
+  uint32_t* dst;
 };
 
 // Reads of data written earlier in the same launch (by any block) go to L2:
@@ -407,12 +413,17 @@ __device__ __forceinline__ void ld_tbox(const float* tb, float mn[3], float mx[3
   }
 }
 
+// Last t with chunk_base[t] <= chunk, 32 ways per read; all lanes of a warp
+// call it.
 __device__ __forceinline__ uint32_t find_task(const uint32_t* chunk_base, uint32_t L, uint32_t chunk) {
-  uint32_t lo = 0, hi = L;  // last t with chunk_base[t] <= chunk
-  while (hi - lo > 1) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (__ldcg(chunk_base + mid) <= chunk) lo = mid;
-    else hi = mid;
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t lo = 0, n = L;  // the answer lies in [lo, lo + n)
+  while (n > 1u) {
+    const uint32_t step = (n + 31u) / 32u, at = lane * step;
+    const uint32_t in = __ballot_sync(0xffffffffu, at < n && __ldcg(chunk_base + lo + at) <= chunk);
+    const uint32_t k = (31u - __clz(in)) * step;  // lane 0 is always in
+    lo += k;
+    n = min(step, n - k);
   }
   return lo;
 }
@@ -430,6 +441,7 @@ struct alignas(16) SahShared {
   uint32_t idx[kLargeBlock / 32][kTaskWarp];       // per-warp partition buffer
 };
 constexpr size_t kShSmall = offsetof(SahShared, chunk_idx);  // scans, partition scalars
+constexpr size_t kShChunk = offsetof(SahShared, bins);       // + a chunk's indices
 constexpr size_t kShBins = offsetof(SahShared, dec);         // + a chunk's indices, per-warp bins
 
 // Bins the primitives at positions [i0, i1) of every lane of a warp into `wb`
@@ -591,7 +603,7 @@ __device__ void large_bin_chunk(const SahParams& p, const Level& lv, uint32_t ch
   const uint32_t c0 = tk.begin + k * kChunk;
   const uint32_t c1 = min(c0 + kChunk, tk.end);
   init_bins(&sh.bins[warp][0], threadIdx.x & 31, 32);
-  for (uint32_t i = c0 + threadIdx.x; i < c1; i += kLargeBlock) sh.chunk_idx[i - c0] = __ldcg(p.idx_a + i);
+  for (uint32_t i = c0 + threadIdx.x; i < c1; i += kLargeBlock) sh.chunk_idx[i - c0] = __ldcg(lv.src + i);
   __syncthreads();
   float mn[3], mx[3];
   ld_tbox(p.tbox + 6 * (size_t)t, mn, mx);
@@ -658,19 +670,25 @@ __device__ void large_decide(const SahParams& p, const Level& lv, uint32_t t, Sa
 __device__ void large_task_warp(const SahParams& p, const Level& lv, uint32_t t, SahShared& sh);
 __device__ void large_task_block(const SahParams& p, const Level& lv, uint32_t t, SahShared& sh);
 
-// Stable partition of a large task's chunk into idx_b; the number of left
-// primitives in the task's earlier chunks comes from a decoupled look-back
+// Stable partition of a large task's chunk from lv.src to lv.dst; the number of
+// left primitives in the task's earlier chunks comes from a decoupled look-back,
+// 32 chunks at a time
 // (chunks are taken in ticket order, so every chunk waited on is held by a
 // running block).
 __device__ void large_partition_chunk(const SahParams& p, const Level& lv, uint32_t chunk, SahShared& sh) {
   const uint32_t t = find_task(p.chunk_base, lv.L, chunk);
   const Decision d = ld_dec(p.dec + t);
-  if (!d.split) return;  // no chunk of this task waits on another
   const Task tk = ld_task(lv.large + t);
   const uint32_t first_chunk = __ldcg(p.chunk_base + t);
   const uint32_t k = chunk - first_chunk;
   const uint32_t c0 = tk.begin + k * kChunk;
   const uint32_t c1 = min(c0 + kChunk, tk.end);
+  if (!d.split) {  // no chunk of this task waits on another
+    if (lv.parity)
+      for (uint32_t i = c0 + threadIdx.x; i < c1; i += kLargeBlock) p.idx_a[i] = __ldcg(lv.src + i);
+    return;
+  }
+  for (uint32_t i = c0 + threadIdx.x; i < c1; i += kLargeBlock) sh.chunk_idx[i - c0] = __ldcg(lv.src + i);
   float mn[3], mx[3];
   ld_tbox(p.tbox + 6 * (size_t)t, mn, mx);
   const BinMap bm = make_binmap(mn, mx);
@@ -679,79 +697,75 @@ __device__ void large_partition_chunk(const SahParams& p, const Level& lv, uint3
   uint32_t prim[PER];
   uint32_t flags = 0, mine = 0;
   const uint32_t s = c0 + threadIdx.x * PER;
+  __syncthreads();
+  float cc[PER];
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
     const uint32_t i = s + j;
     prim[j] = 0;
+    cc[j] = 0.0f;
     if (i < c1) {
-      prim[j] = __ldcg(p.idx_a + i);
-      const float4 c = __ldg(p.centers + prim[j]);
-      const float cc = ax == 0 ? c.x : (ax == 1 ? c.y : c.z);
-      if (bin_of(cc, bm.c2b[ax], bm.off[ax]) < d.split_index) {
-        flags |= 1u << j;
-        ++mine;
-      }
+      prim[j] = sh.chunk_idx[i - c0];
+      cc[j] = __ldg(reinterpret_cast<const float*>(p.centers + prim[j]) + ax);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    if (s + j < c1 && bin_of(cc[j], bm.c2b[ax], bm.off[ax]) < d.split_index) {
+      flags |= 1u << j;
+      ++mine;
     }
   }
   uint32_t chunk_true;
   const uint32_t incl = block_inclusive_scan<kLargeBlock>(mine, sh.warp, &chunk_true);
   const uint32_t before_me = incl - mine;
   volatile uint32_t* st = p.chunk_status;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {  // 32 earlier chunks per look
+    const uint32_t lane = threadIdx.x;
     uint32_t excl = 0;
-    sh.fail = 0;
-    if (k == 0) {
-      st[chunk] = kFlagInc | chunk_true;
-    } else {
-      st[chunk] = kFlagAgg | chunk_true;
-      uint32_t j = chunk - 1;
-      uint32_t spins = 0;
-      for (;;) {
-        const uint32_t v = st[j];
-        const uint32_t f = v & ~kCountMask;
-        if (f == 0u) {
-          if (++spins > kSpinLimit) {
-            atomicOr(&p.cnt->status, kStatusTimeout);
-            sh.fail = 1;
-            break;
-          }
-          __nanosleep(64);
-          continue;
+    bool ok = true;
+    if (lane == 0) st[chunk] = (k == 0 ? kFlagInc : kFlagAgg) | chunk_true;
+    for (uint32_t end = chunk; end > first_chunk && ok;) {  // chunks [first_chunk, end) are to be added
+      const bool there = end - first_chunk > lane;
+      uint32_t v = 0, spins = 0;
+      if (there) {
+        while (((v = st[end - 1u - lane]) & ~kCountMask) == 0u) {
+          if (++spins > kSpinLimit) break;
+          __nanosleep(32);
         }
-        excl += v & kCountMask;
-        if (f == kFlagInc || j == first_chunk) break;
-        --j;
       }
-      st[chunk] = kFlagInc | (excl + chunk_true);
+      ok = __all_sync(0xffffffffu, !there || (v & ~kCountMask) != 0u);
+      const uint32_t incs = __ballot_sync(0xffffffffu, there && (v & ~kCountMask) == kFlagInc);
+      const uint32_t last = incs ? (uint32_t)__ffs(incs) - 1u : 31u;  // the nearest inclusive count
+      excl += __reduce_add_sync(0xffffffffu, there && lane <= last ? v & kCountMask : 0u);
+      if (incs) break;
+      end -= min(32u, end - first_chunk);
     }
-    sh.prefix = excl;
+    if (lane == 0) {
+      if (!ok) atomicOr(&p.cnt->status, kStatusTimeout);
+      else if (k > 0) st[chunk] = kFlagInc | (excl + chunk_true);
+      sh.fail = ok ? 0u : 1u;
+      sh.prefix = excl;
+    }
   }
   __syncthreads();
   const bool fail = sh.fail != 0;
-  const uint32_t true_before = sh.prefix + before_me;
-  __syncthreads();  // sh.prefix / sh.fail are rewritten by the block's next chunk
-  if (fail) return;
-  uint32_t tpos = tk.begin + true_before;
-  uint32_t fpos = tk.begin + d.n_left + ((s - tk.begin) - true_before);
+  const uint32_t true_before = sh.prefix;
+  // the chunk's left ones to the front of the staged indices, in order
+  uint32_t tl = before_me, fl = chunk_true + (threadIdx.x * PER - before_me);
 #pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const uint32_t i = s + j;
-    if (i < c1) {
-      uint32_t dst = ((flags >> j) & 1u) ? tpos++ : fpos++;
-      if (dst < tk.end) p.idx_b[dst] = prim[j];
-      else atomicOr(&p.cnt->status, kStatusBadIndex);
-    }
+  for (int j = 0; j < PER; ++j)
+    if (s + j < c1) sh.chunk_idx[((flags >> j) & 1u) ? tl++ : fl++] = prim[j];
+  __syncthreads();
+  if (fail) return;
+  const uint32_t left_at = tk.begin + true_before;
+  const uint32_t right_at = tk.begin + d.n_left + ((c0 - tk.begin) - true_before);
+  for (uint32_t i = threadIdx.x; i < c1 - c0; i += kLargeBlock) {
+    const uint32_t dst = i < chunk_true ? left_at + i : right_at + (i - chunk_true);
+    if (dst < tk.end) lv.dst[dst] = sh.chunk_idx[i];
+    else atomicOr(&p.cnt->status, kStatusBadIndex);
   }
-}
-
-__device__ void large_copyback_chunk(const SahParams& p, const Level& lv, uint32_t chunk) {
-  const uint32_t t = find_task(p.chunk_base, lv.L, chunk);
-  if (!__ldcg(&p.dec[t].split)) return;
-  const Task tk = ld_task(lv.large + t);
-  const uint32_t k = chunk - __ldcg(p.chunk_base + t);
-  const uint32_t c0 = tk.begin + k * kChunk;
-  const uint32_t c1 = min(c0 + kChunk, tk.end);
-  for (uint32_t i = c0 + threadIdx.x; i < c1; i += kLargeBlock) p.idx_a[i] = __ldcg(p.idx_b + i);
+  __syncthreads();  // the staged indices are rewritten by the block's next chunk
 }
 
 // ------------------------------------------------------------------ small tasks
@@ -766,15 +780,18 @@ static_assert(kSmall <= 32, "a lane per primitive");
 // (wb), indices staged in sidx, the warp-parallel decision, a ballot-based
 // stable partition. The decision is left in `d` (shared
 // memory, written by lane 0) for every lane.
-__device__ void decide_warp(const SahParams& p, uint32_t begin, uint32_t ws, uint32_t depth, const float mn[3],
-                            const float mx[3], uint32_t* wb, uint32_t* sidx, Decision& d) {
+// The indices are read from src and written, partitioned, to dst (which may be
+// the same).
+__device__ void decide_warp(const SahParams& p, const uint32_t* src, uint32_t* dst_idx, uint32_t begin, uint32_t ws,
+                            uint32_t depth, const float mn[3], const float mx[3], uint32_t* wb, uint32_t* sidx,
+                            Decision& d) {
   const int lane = threadIdx.x & 31;
   if (lane == 0) d.split = 0;
   __syncwarp();
   if (ws > 1 && depth < kMaxDepth && ws <= kWarpMax) {
     init_bins(wb, lane, 32);
     // stage the task's indices (independent loads, all in flight at once)
-    for (uint32_t i = lane; i < ws; i += 32) sidx[i] = __ldcg(p.idx_a + begin + i);
+    for (uint32_t i = lane; i < ws; i += 32) sidx[i] = __ldcg(src + begin + i);
     __syncwarp();
     const BinMap bm = make_binmap(mn, mx);
     {
@@ -811,10 +828,10 @@ __device__ void decide_warp(const SahParams& p, uint32_t begin, uint32_t ws, uin
         const uint32_t V = __ballot_sync(0xffffffffu, valid);
         const uint32_t F = V & ~T;
         // written straight to the task's range: the staged copy is the source
-        if (pred) p.idx_a[begin + tb + __popc(T & lt)] = prim;
+        if (pred) dst_idx[begin + tb + __popc(T & lt)] = prim;
         else if (valid) {
           const uint32_t dst = n_left + fb + __popc(F & lt);
-          if (dst < ws) p.idx_a[begin + dst] = prim;
+          if (dst < ws) dst_idx[begin + dst] = prim;
         }
         tb += __popc(T);
         fb += __popc(F);
@@ -829,7 +846,10 @@ __device__ void large_task_warp(const SahParams& p, const Level& lv, uint32_t t,
   const Task tk = ld_task(lv.large + t);
   float mn[3], mx[3];
   task_box(p.nodes, tk.node, mn, mx);
-  decide_warp(p, tk.begin, tk.end - tk.begin, tk.depth, mn, mx, sh.bins[warp], sh.idx[warp], sh.dec[warp]);
+  decide_warp(p, lv.src, lv.dst, tk.begin, tk.end - tk.begin, tk.depth, mn, mx, sh.bins[warp], sh.idx[warp],
+              sh.dec[warp]);
+  if (lv.parity && !sh.dec[warp].split)  // (a task at the depth limit ends at an even level)
+    for (uint32_t i = tk.begin + lane; i < tk.end; i += 32) p.idx_a[i] = __ldcg(lv.src + i);
   if (lane == 0) {
     if (sh.dec[warp].split) write_interior_box(p.nodes, tk.node, mn, mx);
     else write_leaf(p.nodes, tk, mn, mx);
@@ -847,7 +867,7 @@ __device__ void large_task_block(const SahParams& p, const Level& lv, uint32_t t
   if (threadIdx.x == 0) sh.dec[0].split = 0;
   if (ws > 1 && tk.depth < kMaxDepth) {
     init_bins(&sh.bins[warp][0], lane, 32);
-    for (uint32_t i = threadIdx.x; i < ws; i += kLargeBlock) sh.chunk_idx[i] = __ldcg(p.idx_a + tk.begin + i);
+    for (uint32_t i = threadIdx.x; i < ws; i += kLargeBlock) sh.chunk_idx[i] = __ldcg(lv.src + tk.begin + i);
     __syncthreads();
     const BinMap bm = make_binmap(mn, mx);
     const uint32_t per = (ws + kLargeBlock - 1) / kLargeBlock;
@@ -890,9 +910,11 @@ __device__ void large_task_block(const SahParams& p, const Level& lv, uint32_t t
       uint32_t tpos = tk.begin + before, fpos = tk.begin + sh.dec[0].n_left + (i0 - before);
       for (uint32_t i = i0; i < i1; ++i) {
         const uint32_t dst = ((flags >> (i - i0)) & 1u) ? tpos++ : fpos++;
-        if (dst < tk.end) p.idx_a[dst] = sh.chunk_idx[i];
+        if (dst < tk.end) lv.dst[dst] = sh.chunk_idx[i];
         else atomicOr(&p.cnt->status, kStatusBadIndex);
       }
+    } else if (lv.parity) {
+      for (uint32_t i = threadIdx.x; i < ws; i += kLargeBlock) p.idx_a[tk.begin + i] = sh.chunk_idx[i];
     }
   }
   __syncthreads();
@@ -1009,6 +1031,10 @@ __device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& s
   const int lane = threadIdx.x & 31;
   int sp = -1;  // warp-uniform
   const uint32_t rws = root.end - root.begin;
+  // a subtree that hangs below an even level has its indices in idx_b
+  if (root.depth & 1u)
+    for (uint32_t i = root.begin + lane; i < root.end; i += 32) p.idx_a[i] = __ldcg(p.idx_b + i);
+  __syncwarp();
   if (lane == 0) {
     const DAabb rb = load_aabb_cg(p.nodes + root.node);
     SubTask t;
@@ -1030,7 +1056,7 @@ __device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& s
     const SubTask tk = sh.stack[sp--];
     float mn[3], mx[3];
     first_offset(tk, mn, mx);
-    decide_warp(p, tk.begin, tk.end - tk.begin, tk.depth, mn, mx, sh.bins, sh.idx, sh.dec);
+    decide_warp(p, p.idx_a, p.idx_a, tk.begin, tk.end - tk.begin, tk.depth, mn, mx, sh.bins, sh.idx, sh.dec);
     const Decision d = sh.dec;
     __syncwarp();
     SubTask l, r;
@@ -1405,7 +1431,7 @@ __device__ void emit_segment(const SahParams& p, const Level& lv, SahShared& sh,
 
 // Scan and emission of a level of few tasks by one block.
 constexpr uint32_t kFewTasks = 4u * kLargeBlock;
-__device__ void scan_emit_block(const SahParams& p, const Level& lv, SahShared& sh) {
+__device__ void scan_emit_block(const SahParams& p, const Level& lv, SahShared& sh, bool advance) {
   uint64_t carry = 0;
   for (uint32_t base = 0; base < lv.L; base += kLargeBlock) {
     const uint32_t t = base + threadIdx.x;
@@ -1424,9 +1450,14 @@ __device__ void scan_emit_block(const SahParams& p, const Level& lv, SahShared& 
   }
   if (threadIdx.x == 0) {
     const uint32_t nl = (uint32_t)(carry >> 32), ns = (uint32_t)(carry & 0xffffffffu);
-    p.cnt->node_count = lv.node_base + nl + ns;
-    p.cnt->large = nl;
-    p.cnt->sub = lv.sub_base + ns;
+    if (advance) {
+      p.cnt->node_count = lv.node_base + nl + ns;
+      p.cnt->large = nl;
+      p.cnt->sub = lv.sub_base + ns;
+    } else {
+      p.cnt->next_large = nl;
+      p.cnt->next_sub = ns;
+    }
   }
 }
 
@@ -1449,7 +1480,10 @@ __device__ __forceinline__ Level read_level(const SahParams& p, uint32_t level) 
   lv.sub_base = __ldcg(&p.cnt->sub);
   lv.large = p.large[level & 1];
   lv.large_next = p.large[(level + 1) & 1];
+  lv.parity = level & 1;
   lv.next_parity = (level + 1) & 1;
+  lv.src = lv.parity ? p.idx_b : p.idx_a;
+  lv.dst = lv.parity ? p.idx_a : p.idx_b;
   return lv;
 }
 
@@ -1502,13 +1536,12 @@ __global__ void __launch_bounds__(kLargeBlock, 2) k_sah_build(SahParams p) {
       // large partitions (chunks in ticket order)
       large_partition_phase(p, lv, chunks, sh);
       if (!grid_sync(p.bar, G, status)) return;
-      for (uint32_t c = blockIdx.x; c < chunks; c += G) large_copyback_chunk(p, lv, c);
       for (uint32_t c = blockIdx.x * kLargeBlock + threadIdx.x; c < chunks; c += G * kLargeBlock)
         p.chunk_status[c] = 0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) p.cnt->big[level & 1] = 0u;  // the level after the next sets it again
     if (lv.L <= kFewTasks) {
-      if (blockIdx.x == 0) scan_emit_block(p, lv, sh);
+      if (blockIdx.x == 0) scan_emit_block(p, lv, sh, true);
     } else {
       scan_segment(p, lv, sh);
       if (!grid_sync(p.bar, G, status)) return;
@@ -1530,10 +1563,15 @@ __device__ __forceinline__ SahShared& dyn_shared() {
 __global__ void __launch_bounds__(kLargeBlock) k_ph_prep(SahParams p, uint32_t level) {
   SahShared& sh = dyn_shared();
   const Level lv = read_level(p, level);
+  if (lv.L == 0) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.cnt->chunks = 0;
+    return;
+  }
   if (blockIdx.x == 0) large_prep(p, lv, sh, 1u);
   large_bins_init(p, lv);
 }
-__global__ void __launch_bounds__(kLargeBlock) k_ph_bin(SahParams p, uint32_t level) {
+// (three blocks per SM: 80 registers; two or four are 1 and 3 % slower at 4M)
+__global__ void __launch_bounds__(kLargeBlock, 3) k_ph_bin(SahParams p, uint32_t level) {
   SahShared& sh = dyn_shared();
   const Level lv = read_level(p, level);
   const uint32_t chunks = __ldcg(&p.cnt->chunks);
@@ -1550,25 +1588,44 @@ __global__ void __launch_bounds__(kLargeBlock) k_ph_partition(SahParams p, uint3
   const Level lv = read_level(p, level);
   large_partition_phase(p, lv, __ldcg(&p.cnt->chunks), sh);
 }
-__global__ void __launch_bounds__(kLargeBlock) k_ph_copyback_scan(SahParams p, uint32_t level) {
+// Chunk status cleared for the next level, and the numbering of a level: by one
+// more block for few tasks, else by the kernels below.
+__global__ void __launch_bounds__(kLargeBlock) k_ph_number(SahParams p, uint32_t level) {
   SahShared& sh = dyn_shared();
   const Level lv = read_level(p, level);
-  if (lv.L > 0) {
-    const uint32_t chunks = __ldcg(&p.cnt->chunks);
-    for (uint32_t c = blockIdx.x; c < chunks; c += gridDim.x) large_copyback_chunk(p, lv, c);
-    for (uint32_t c = blockIdx.x * kLargeBlock + threadIdx.x; c < chunks; c += gridDim.x * kLargeBlock)
+  const uint32_t chunks = __ldcg(&p.cnt->chunks);
+  if (lv.L == 0) return;
+  if (blockIdx.x + 1u < gridDim.x) {
+    for (uint32_t c = blockIdx.x * kLargeBlock + threadIdx.x; c < chunks; c += (gridDim.x - 1u) * kLargeBlock)
       p.chunk_status[c] = 0;
+  } else if (lv.L <= kFewTasks) {
+    scan_emit_block(p, lv, sh, false);
   }
-  scan_segment(p, lv, sh);
+}
+__global__ void __launch_bounds__(kLargeBlock) k_ph_scan(SahParams p, uint32_t level) {
+  SahShared& sh = dyn_shared();
+  const Level lv = read_level(p, level);
+  if (lv.L > kFewTasks) scan_segment(p, lv, sh);
 }
 __global__ void __launch_bounds__(kLargeBlock) k_ph_emit(SahParams p, uint32_t level) {
   SahShared& sh = dyn_shared();
-  emit_segment(p, read_level(p, level), sh, false);
+  const Level lv = read_level(p, level);
+  if (lv.L > kFewTasks) emit_segment(p, lv, sh, false);
 }
-// Counters of the next level (after every block of k_ph_emit read them).
-__global__ void k_ph_advance(SahParams p, uint32_t level, uint32_t blocks) {
+// Counters of the next level (after every block of the kernels before read
+// them).
+__global__ void __launch_bounds__(kLargeBlock) k_ph_advance(SahParams p, uint32_t level, uint32_t blocks) {
   SahShared& sh = dyn_shared();
   const Level lv = read_level(p, level);
+  if (lv.L == 0) return;
+  if (lv.L <= kFewTasks) {
+    if (threadIdx.x == 0) {
+      p.cnt->node_count = lv.node_base + p.cnt->next_large + p.cnt->next_sub;
+      p.cnt->large = p.cnt->next_large;
+      p.cnt->sub = lv.sub_base + p.cnt->next_sub;
+    }
+    return;
+  }
   uint64_t all = 0;
   for (uint32_t b = threadIdx.x; b < blocks; b += kLargeBlock) all += __ldcg(p.scan_sums + b);
   uint64_t tot;
@@ -1804,7 +1861,7 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   int per_sm = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, coop ? (const void*)k_sah_build
                                                                          : (const void*)k_ph_partition,
-                                                         kLargeBlock, coop ? 0 : kShSmall)))
+                                                         kLargeBlock, coop ? 0 : kShChunk)))
     return fail(cuda_rc(e));
   if (per_sm < 1) return fail(DeviceError);
   const uint32_t grid = (uint32_t)sm_count() * (coop && n <= 65536u ? 1u : (uint32_t)per_sm);
@@ -1883,19 +1940,27 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
       if ((e = cudaLaunchCooperativeKernel((void*)k_sah_build, dim3(grid), dim3(kLargeBlock), args, 0, s)))
         return fail(cuda_rc(e));
     } else {
+      // The kernels read a level's counts on the device and do nothing past
+      // the last one, so the host looks at them every fourth level only.
       h.large = 1u;
-      const size_t cap = (size_t)grid;
-      auto blocks = [cap](size_t need) { return (unsigned)(need < 1 ? 1 : (need < cap ? need : cap)); };
-      for (uint32_t level = 0; h.large > 0; ++level) {
+      int bin_per_sm = 0;
+      if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bin_per_sm, k_ph_bin, kLargeBlock, kShBins)))
+        return fail(cuda_rc(e));
+      const uint32_t sms = (uint32_t)sm_count(), bin_grid = sms * (uint32_t)(bin_per_sm < 1 ? 1 : bin_per_sm);
+      for (uint32_t level = 0; h.large > 0;) {
         if (level > kMaxDepth + 1) return fail(Error);
-        k_ph_prep<<<blocks(((size_t)h.large * 3 * kBins + kLargeBlock - 1) / kLargeBlock), kLargeBlock, kShSmall,
-                    s>>>(p, level);
-        k_ph_bin<<<grid, kLargeBlock, kShBins, s>>>(p, level);
-        k_ph_decide<<<blocks((h.large + 7) / 8), kLargeBlock, kShBins, s>>>(p, level);
-        k_ph_partition<<<grid, kLargeBlock, kShSmall, s>>>(p, level);
-        k_ph_copyback_scan<<<grid, kLargeBlock, kShSmall, s>>>(p, level);
-        k_ph_emit<<<grid, kLargeBlock, kShSmall, s>>>(p, level);
-        k_ph_advance<<<1, kLargeBlock, kShSmall, s>>>(p, level, grid);
+        for (uint32_t k = 0; k < 4; ++k, ++level) {
+          k_ph_prep<<<sms, kLargeBlock, kShSmall, s>>>(p, level);
+          k_ph_bin<<<bin_grid, kLargeBlock, kShBins, s>>>(p, level);
+          k_ph_decide<<<sms * 2u, kLargeBlock, kShBins, s>>>(p, level);
+          k_ph_partition<<<grid, kLargeBlock, kShChunk, s>>>(p, level);
+          k_ph_number<<<9, kLargeBlock, kShSmall, s>>>(p, level);
+          if (large_cap > kFewTasks) {  // else no level has that many tasks
+            k_ph_scan<<<grid, kLargeBlock, kShSmall, s>>>(p, level);
+            k_ph_emit<<<grid, kLargeBlock, kShSmall, s>>>(p, level);
+          }
+          k_ph_advance<<<1, kLargeBlock, kShSmall, s>>>(p, level, grid);
+        }
         if ((e = cudaGetLastError())) return fail(cuda_rc(e));
         if ((e = cudaMemcpyAsync(&h, cnt.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, s)) ||
             (e = cudaStreamSynchronize(s)))

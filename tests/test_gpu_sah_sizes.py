@@ -40,3 +40,16 @@ def test_sah_sizes(n, ppl, kind):
     assert canonical(nodes, idx) == canonical(on, oi)
     assert np.array_equal(np.sort(idx), np.arange(len(tris)))
     assert np.array_equal(u32(rb.Mbvh.construct(g).quad_nodes()), u32(oracle.mbvh(nodes)))
+
+
+@pytest.mark.parametrize("n,kind", [(1048577, "soup"), (1300003, "equal"), (1100000, "sphere")])
+def test_sah_above_the_cooperative_size(n, kind):
+    """Builds of more than 2^20 primitives launch the phases of a level one by
+    one, the indices changing sides at every level."""
+    tris = _scene(n, kind)
+    g = gpu_build(tris, "sah")
+    on, oi = oracle_build(tris, "sah")
+    nodes, idx = g.nodes(), g.indices()
+    assert len(nodes) == len(on)
+    assert np.array_equal(np.sort(idx), np.arange(len(tris)))
+    assert np.array_equal(u32(oracle.mbvh(nodes)), u32(oracle.mbvh(on)))
