@@ -17,10 +17,11 @@ namespace {
 
 constexpr int kBlock = 256;  // threads per tile == number of digits
 // Keys per thread: what a tile costs is the latency of ranking them one after
-// another and of the look-back, so few keys take small tiles, one per SM or
-// more as long as there are enough. LOCB builds, 4 keys against 15 per thread:
-// 6,400 triangles 464 / 488 us, 20k 529 / 543, 150k 733 / 761; 1M 1,477 / 1,454.
-inline int items_for(size_t n) { return n <= 160000 ? 4 : 15; }
+// another and of the look-back, so few keys take small tiles. LOCB builds: 4
+// keys against 15 per thread, 6,400 triangles 464 / 488 us, 20k 529 / 543;
+// 8 against 15, 1M triangles 1,453 / 1,482, 4M 3,909 / 3,949. Per pass: 200k
+// pairs 15 -> 10 us, 4.2M 53 -> 42.
+inline int items_for(size_t n) { return n <= 160000 ? 4 : 8; }
 inline size_t tile_for(size_t n) { return (size_t)kBlock * items_for(n); }
 // Earlier tiles that a look-back reads at a time.
 constexpr int kLook = 4;
@@ -84,8 +85,10 @@ __global__ void __launch_bounds__(kBlock) k_hist_scan(uint32_t* __restrict__ his
   h[threadIdx.x] = incl - v;
 }
 
+// Digits are recomputed from the keys and ranks kept in 16 bits: four blocks
+// fit an SM (with 15 keys per thread and all of it held it was two).
 template <int kItems>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, 4)
     k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, size_t n, int shift,
                const uint32_t* __restrict__ digit_offsets, uint32_t* __restrict__ lookback,
@@ -111,26 +114,28 @@ __global__ void __launch_bounds__(kBlock)
   const size_t tile_base = tile * kTile;
   const size_t warp_base = tile_base + (size_t)warp * (kItems * 32);
 
-  uint32_t key[kItems], val[kItems], rank[kItems];
-  uint32_t dig[kItems];
+  uint32_t key[kItems], val[kItems];
+  uint16_t rank[kItems];  // below 32 kItems
+  const uint32_t in_warp = warp_base >= n ? 0u : (n - warp_base < (size_t)(kItems * 32) ? (uint32_t)(n - warp_base)
+                                                                                   : (uint32_t)(kItems * 32));
+  auto valid = [&](int k) { return (uint32_t)(k * 32 + lane) < in_warp; };
+  auto digit = [&](int k) { return (key[k] >> shift) & 0xffu; };
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
-    size_t idx = warp_base + (size_t)k * 32 + lane;
-    bool valid = idx < n;
-    key[k] = valid ? __ldg(keys_in + idx) : 0xffffffffu;
-    val[k] = valid ? __ldg(vals_in + idx) : 0u;
-    dig[k] = valid ? ((key[k] >> shift) & 0xffu) : (uint32_t)kRadix;
+    key[k] = valid(k) ? __ldg(keys_in + warp_base + k * 32 + lane) : 0u;
+    val[k] = valid(k) ? __ldg(vals_in + warp_base + k * 32 + lane) : 0u;
   }
   const uint32_t lt_mask = (1u << lane) - 1u;
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
-    uint32_t d = dig[k];
-    uint32_t peers = __match_any_sync(0xffffffffu, d);
+    const bool v = valid(k);
+    const uint32_t d = v ? digit(k) : (uint32_t)kRadix;
+    const uint32_t peers = __match_any_sync(0xffffffffu, d);
     uint32_t base = 0;
-    if (d < (uint32_t)kRadix) base = s_whist[warp][d];
-    rank[k] = base + __popc(peers & lt_mask);
+    if (v) base = s_whist[warp][d];
+    rank[k] = (uint16_t)(base + __popc(peers & lt_mask));
     __syncwarp();
-    if (d < (uint32_t)kRadix && (__ffs(peers) - 1) == lane) s_whist[warp][d] = base + __popc(peers);
+    if (v && (__ffs(peers) - 1) == lane) s_whist[warp][d] = base + __popc(peers);
     __syncwarp();
   }
   __syncthreads();
@@ -190,8 +195,8 @@ __global__ void __launch_bounds__(kBlock)
 
 #pragma unroll
   for (int k = 0; k < kItems; ++k) {
-    if (dig[k] < (uint32_t)kRadix) {
-      uint32_t pos = s_local_off[dig[k]] + s_whist[warp][dig[k]] + rank[k];
+    if (valid(k)) {
+      const uint32_t dk = digit(k), pos = s_local_off[dk] + s_whist[warp][dk] + rank[k];
       s_keys[pos] = key[k];
       s_vals[pos] = val[k];
     }
@@ -236,8 +241,7 @@ cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, size_t n, int bits,
   if (hblocks > cap) hblocks = cap;
   k_histogram<<<hblocks, kBlock, 0, s>>>(keys, n, passes, t.hist);
   k_hist_scan<<<passes, kBlock, 0, s>>>(t.hist);
-  const int items = items_for(n);
-  auto sweep = items == 4 ? k_onesweep<4> : k_onesweep<15>;
+  auto sweep = items_for(n) == 4 ? k_onesweep<4> : k_onesweep<8>;
   uint32_t *kin = keys, *vin = vals, *kout = t.keys_alt, *vout = t.vals_alt;
   for (int p = 0; p < passes; ++p) {
     sweep<<<(unsigned)tiles, kBlock, 0, s>>>(kin, vin, kout, vout, n, 8 * p, t.hist + p * kRadix,
