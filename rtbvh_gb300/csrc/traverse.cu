@@ -313,8 +313,17 @@ constexpr uint32_t kFewWarpsPerScheduler = 3;
 // 246 / 226 (200k soup, LOCB), 301 / 224 (300k clustered, SAH); 16,384: 111 /
 // 98, 264 / 255, 315 / 245; 32,768: 102 / 78, 273 / 298, 317 / 261. Any hit
 // (300k clustered): 4,096 rays 194 / 132, 65,536: 281 / 235, 131,072: 301 /
-// 319. Rays handed on by the compact walk come from binned-SAH trees.
-constexpr uint32_t kFewClosest = 20480, kFewAny = 65536, kFewDeferred = 32768;
+// 319. Rays handed on by the compact walk come from binned-SAH trees; up to
+// kFewDeferred of them take four lanes. So do more, up to kFewDeferredMost,
+// where they are a small part of their launch: that part is the rays with the
+// longest walks, so the longest chain counts and not the throughput. One lane
+// against four, in us: 4M rays of which 68k are handed on 5,607 / 4,580 (2M
+// clustered), 4.2M of which 83k 1,882 / 1,677 (200k sphere), 16M of which 270k
+// 14,770 / 13,970; 1/4 to 1/32 of the launch as the line: all the same. Where
+// whole launches are handed on (scenes beyond the compact walk's range) one
+// lane per ray is the better from about 131k rays, and 1.4 times at 262k.
+constexpr uint32_t kFewClosest = 20480, kFewAny = 65536;
+constexpr uint32_t kFewDeferred = 32768, kFewDeferredMost = 524288, kFewDeferredPart = 16;
 __device__ __host__ __forceinline__ uint32_t few_warps(uint32_t rays, uint32_t sms) {
   const uint32_t spread = sms * 4u * kFewWarpsPerScheduler;
   const uint32_t least = (rays + 7u) / 8u;
@@ -600,7 +609,8 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int
   const uint32_t ray_count = a.ray_count_dev ? *a.ray_count_dev : (uint32_t)a.ray_count;
   if (FEW) {
     __shared__ int32_t s_stack[kBlock / 4][kStack];
-    if (ray_count <= kFewDeferred) {
+    if (ray_count <= kFewDeferred ||
+        (ray_count <= kFewDeferredMost && ray_count <= a.ray_count / kFewDeferredPart)) {
       const uint32_t launched = gridDim.x * (kBlock / 32u), wanted = few_warps(ray_count, a.sms);
       walk_mbvh4<ANY_HIT, CULL>(a, ray_count, wanted < launched ? wanted : launched, s_stack);
       return;

@@ -54,6 +54,29 @@ def test_small_launches_equal_large_ones(name, kind, scale, mode):
     assert (rb.hit_prims(want) >= 0).any()
 
 
+@pytest.mark.parametrize("step,count", [(35, 700001), (20, 700001), (35, 500001), (35, 8000003), (35, 10000019)])
+def test_handed_on_rays_of_large_launches(step, count):
+    """Rays that the compact walk hands on (about 3 % and every step-th), on
+    both sides of the lines between four lanes and one: 1/16 of the launch,
+    32,768 rays, 524,288 rays. The exact walk is theirs, bit for bit."""
+    tris = scene("sphere")
+    m = rb.Mbvh.construct(gpu_build(tris, "sah"))
+    rays, _ = _rays(tris, 500001, 6)
+    rays[::97, :3] *= np.float32(1e-4)  # back within range
+    rays[:, :3] = np.clip(rays[:, :3], -100, 100)
+    r = to_cuda(rays)[torch.arange(count, device="cuda") % 500001]
+    r[::step, :3] += 300.0 * r[::step, 3:]  # beyond it
+    got, work = m.intersect(r, walk_stats=True)
+    handed = work[:, 2] > 0
+    n = int(handed.sum())
+    assert (n <= count // 16) == (step == 35) and (n > 32768) == (count > 600000) and (n > 524288) == (count > 9000000)
+    want = m.intersect(r, exact_nodes=True)[0]
+    assert torch.equal(got[handed].view(torch.int32), want[handed].view(torch.int32))
+    # the others may take another of two triangles at the same t
+    assert torch.equal(got[:, 0].view(torch.int32), want[:, 0].view(torch.int32))
+    assert m.status() == rb.ResultCode.Ok
+
+
 def test_small_batch_of_meshes():
     sizes = [1, 2, 300, 5000, 3]
     off = np.concatenate([[0], np.cumsum(sizes)])
