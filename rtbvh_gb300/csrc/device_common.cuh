@@ -114,6 +114,37 @@ __device__ __forceinline__ float ordered_to_float(uint32_t k) {
   return __uint_as_float(k ^ ((uint32_t)((int32_t)~k >> 31) | 0x80000000u));
 }
 
+// A box folded as six ordered keys under max, the minima complemented, so that
+// zeroed memory is the empty box. Min and max are exact: no order matters.
+struct KeyBox {
+  uint32_t k[6];
+  __device__ __forceinline__ KeyBox(const float mn[3], const float mx[3]) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      k[a] = ~float_to_ordered(mn[a]);
+      k[3 + a] = float_to_ordered(mx[a]);
+    }
+  }
+  // over the whole warp, on every lane
+  __device__ __forceinline__ void fold_warp() {
+#pragma unroll
+    for (int a = 0; a < 6; ++a) k[a] = __reduce_max_sync(0xffffffffu, k[a]);
+  }
+};
+
+// Aabb::union_of_list and its 1e-4 offset (Aabb::with_offset) of folded keys.
+__device__ __forceinline__ DAabb world_box(const uint32_t k[6]) {
+  DAabb w;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    w.min[a] = rs_min(1e34f, ordered_to_float(~k[a])) - 0.0001f;
+    w.max[a] = rs_max(-1e34f, ordered_to_float(k[3 + a])) + 0.0001f;
+  }
+  w.count = 0;
+  w.left_first = 0;
+  return w;
+}
+
 // Aabb::half_area (src/aabb.rs:342-346), no FMA.
 __device__ __forceinline__ float half_area(float mnx, float mny, float mnz, float mxx, float mxy, float mxz) {
   float d0 = mxx - mnx, d1 = mxy - mny, d2 = mxz - mnz;

@@ -59,7 +59,9 @@ cudaError_t launch_point_prep(const float* centers, size_t stride_floats, size_t
 cudaError_t launch_pack_centers(const float* centers, size_t stride_floats, size_t n, float4* centers4,
                                 cudaStream_t s);
 // Aabb::union_of_list (src/aabb.rs:124-131) into *world (one DAabb).
-cudaError_t launch_world_bounds(const DAabb* aabbs, size_t n, DAabb* world, uint32_t* acc6, cudaStream_t s);
+// acc: kBoundsWords words of scratch
+constexpr size_t kBoundsWords = 7;
+cudaError_t launch_world_bounds(const DAabb* aabbs, size_t n, DAabb* world, uint32_t* acc, cudaStream_t s);
 // MortonEncoder::encode of every centre against `world` (src/morton.rs:36-61);
 // vals[i] = i.
 cudaError_t launch_morton(const float4* centers, size_t n, const DAabb* world, uint32_t* keys, uint32_t* vals,

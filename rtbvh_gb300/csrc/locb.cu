@@ -946,7 +946,7 @@ ResultCode build_locb(const DAabb* aabbs, const float4* centers, size_t n_, cuda
   };
   Scratch<DAabb> world;
   Scratch<uint32_t> acc, status;
-  if ((e = world.alloc(1, s)) || (e = acc.alloc(8, s)) || (e = status.alloc(4, s))) return fail(cuda_rc(e));
+  if ((e = world.alloc(1, s)) || (e = acc.alloc(kBoundsWords, s)) || (e = status.alloc(4, s))) return fail(cuda_rc(e));
   if ((e = cudaMemsetAsync(status.ptr, 0, 16, s))) return fail(cuda_rc(e));
   if ((e = launch_world_bounds(aabbs, n, world.ptr, acc.ptr, s))) return fail(cuda_rc(e));
   if (n <= 2) {

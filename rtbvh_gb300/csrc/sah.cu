@@ -1890,7 +1890,7 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   Scratch<uint64_t> scan_vals, scan_sums;
   Scratch<Counters> cnt;
   Scratch<GridBarrier> bar;
-  if ((e = world.alloc(1, s)) || (e = acc.alloc(8, s)) || (e = idx_b.alloc(n, s)) ||
+  if ((e = world.alloc(1, s)) || (e = acc.alloc(kBoundsWords, s)) || (e = idx_b.alloc(n, s)) ||
       (e = bins.alloc((size_t)large_cap * kTaskBinWords, s)) || (e = chunk_base.alloc(large_cap + 1, s)) ||
       (e = chunk_status.alloc(chunk_cap, s)) || (e = large0.alloc(large_cap, s)) || (e = large1.alloc(large_cap, s)) ||
       (e = subs.alloc(sub_cap, s)) || (e = dec.alloc(large_cap, s)) || (e = tbox.alloc((size_t)large_cap * 6, s)) ||

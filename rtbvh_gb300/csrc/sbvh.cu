@@ -1383,7 +1383,7 @@ ResultCode build_spatial_sah(const DAabb* aabbs, const float4* centers, const fl
   Scratch<SbRef> r0, r1, r2, scr;
   Scratch<unsigned long long> k0, k1;
   Scratch<float> fbuf;
-  Scratch<uint32_t> perm, hk, hv, ready, child, arrive, ic, lr, ib, lb, acc6, rstat;
+  Scratch<uint32_t> perm, hk, hv, ready, child, arrive, ic, lr, ib, lb, acc, rstat;
   Scratch<uint8_t> cls;
   Scratch<SbTask> tasks;
   Scratch<SbCtl> ctl;
@@ -1396,10 +1396,10 @@ ResultCode build_spatial_sah(const DAabb* aabbs, const float4* centers, const fl
       (e = tasks.alloc(task_cap, s)) || (e = ready.alloc(task_cap, s)) || (e = child.alloc(task_cap, s)) ||
       (e = arrive.alloc(task_cap, s)) || (e = ic.alloc(task_cap, s)) || (e = lr.alloc(task_cap, s)) ||
       (e = ib.alloc(task_cap, s)) || (e = lb.alloc(task_cap, s)) || (e = ctl.alloc(1, s)) ||
-      (e = world.alloc(1, s)) || (e = acc6.alloc(6, s)) || (e = rstat.alloc(1, s)) ||
+      (e = world.alloc(1, s)) || (e = acc.alloc(kBoundsWords, s)) || (e = rstat.alloc(1, s)) ||
       (e = cudaMemsetAsync(rstat.ptr, 0, 4, s)))
     return cuda_rc(e);
-  if ((e = launch_world_bounds(aabbs, n, world.ptr, acc6.ptr, s))) return cuda_rc(e);
+  if ((e = launch_world_bounds(aabbs, n, world.ptr, acc.ptr, s))) return cuda_rc(e);
   SbArgs A;
   A.refs[0] = r0.ptr;
   A.refs[1] = r1.ptr;
