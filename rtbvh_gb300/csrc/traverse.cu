@@ -290,7 +290,6 @@ __device__ __forceinline__ uint32_t subtree_mask(const DTBox* box, const RayStat
 // with a lane per ray: the slots go through the same sorting network, lane by
 // lane, and where the leaves of one node are tested side by side, a hit counts
 // if no leaf before it in the walk's order has a nearer one.
-// The stack is the four lanes' in shared memory.
 struct FourLanes {
   uint32_t first;  // lane 0 of the four
   uint32_t l;      // this lane of the four
@@ -407,13 +406,16 @@ struct LaneQuad {
   }
 };
 
-// k_trace_mbvh's walk, four lanes per ray, for ray_count rays; s_stack: the
-// block's stacks. The next node is popped and asked for before the leaves are
-// tested.
-template <bool ANY_HIT, int CULL>
-__device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warps, int32_t (*s_stack)[kStack]) {
+// k_trace_mbvh's walk, four lanes per ray, for ray_count rays. The next node
+// is popped and asked for before the leaves are tested. The four lanes share
+// one stack in `shared`, or, without it, each keeps the whole of it: as a
+// branch of k_trace_mbvh the shared stacks took L1 from the other branch (1M
+// rays beyond the compact walk's range over a 200k soup 3,770 -> 3,830 us).
+template <bool ANY_HIT, int CULL, bool SHARED>
+__device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warps, int32_t* shared) {
   const FourLanes q;
-  int32_t* stack = s_stack[threadIdx.x >> 2];
+  int32_t own[SHARED ? 1 : kStack];
+  int32_t* const stack = SHARED ? shared : own;
   const uint32_t warp = blockIdx.x * (kBlock / 32u) + (threadIdx.x >> 5);
   RayState ray;
   float hu = 0.0f, hv = 0.0f;
@@ -503,7 +505,7 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
     const uint32_t inners = q.ballot(inner);
     const int n = __popc(inners);
     const int32_t nearest = q.from(child, inners ? (uint32_t)__ffs(inners) - 1u : 0u);
-    bool done = false;
+    bool done = false, push = false;
     int32_t next = -1;
     if (n > 0) {
       next = nearest;
@@ -512,12 +514,23 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
         prim = -2;
         done = true;
       } else {
-        // farther slots below nearer ones
+        push = true;
+      }
+    }
+    // farther slots below nearer ones
+    if (SHARED) {
+      if (push) {
         if (inner && (inners & ((1u << q.l) - 1u))) stack[sp + 1 + __popc(inners >> (q.l + 1u))] = child;
         sp += n - 1;
       }
+      __syncwarp();
+    } else {
+#pragma unroll
+      for (uint32_t k = 3; k > 0; --k) {
+        const int32_t c = q.from(child, k);
+        if (push && ((inners >> k) & 1u) && (inners & ((1u << k) - 1u))) stack[++sp] = c;
+      }
     }
-    __syncwarp();
     if (active && !done) {
       current = next;
       if (next < 0 && sp >= 0) current = stack[sp--];
@@ -566,7 +579,7 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
 template <bool ANY_HIT, int CULL>
 __global__ void __launch_bounds__(kBlock) k_trace_mbvh4(TraceArgs a, uint32_t warps) {
   __shared__ int32_t s_stack[kBlock / 4][kStack];
-  walk_mbvh4<ANY_HIT, CULL>(a, (uint32_t)a.ray_count, warps, s_stack);
+  walk_mbvh4<ANY_HIT, CULL, true>(a, (uint32_t)a.ray_count, warps, s_stack[threadIdx.x >> 2]);
 }
 
 // Persistent MBVH traversal over the exact quad nodes with per-lane ray
@@ -588,9 +601,13 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh4(TraceArgs a, uint32_t wa
 //   4.2M shadow rays over 1M clustered triangles: 10.74 ms without the skip,
 //   3.80 ms with it.
 // FEW: a launch whose ray count is read from the device walks with four lanes
-// per ray when that is at most kFewDeferred.
+// per ray when that is at most kFewDeferred. The launch bounds keep that
+// branch from taking registers from the other one: 8 blocks per SM, 7 with
+// subtree boxes (8 spill there). Without them 68 and 78 registers, and launches
+// handed on whole were 5 to 10 % slower (1M rays, 1M clustered triangles:
+// 6,190 us for 5,770; 200k sphere, SAH: 4,260 for 3,880).
 template <bool ANY_HIT, bool STATS, int CULL = kCullNone, bool FEW = false>
-__global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int* work) {
+__global__ void __launch_bounds__(kBlock, FEW ? (CULL ? 7 : 8) : 0) k_trace_mbvh(TraceArgs a, unsigned int* work) {
   RayState ray;
   float hu = 0.0f, hv = 0.0f;
   int32_t prim = -1;
@@ -608,11 +625,10 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh(TraceArgs a, unsigned int
   uint32_t batch = a.ray_batch ? a.ray_batch : kPoolBatch;
   const uint32_t ray_count = a.ray_count_dev ? *a.ray_count_dev : (uint32_t)a.ray_count;
   if (FEW) {
-    __shared__ int32_t s_stack[kBlock / 4][kStack];
     if (ray_count <= kFewDeferred ||
         (ray_count <= kFewDeferredMost && ray_count <= a.ray_count / kFewDeferredPart)) {
       const uint32_t launched = gridDim.x * (kBlock / 32u), wanted = few_warps(ray_count, a.sms);
-      walk_mbvh4<ANY_HIT, CULL>(a, ray_count, wanted < launched ? wanted : launched, s_stack);
+      walk_mbvh4<ANY_HIT, CULL, false>(a, ray_count, wanted < launched ? wanted : launched, nullptr);
       return;
     }
   }
