@@ -206,17 +206,19 @@ struct WarpPool {
   uint32_t next = 0, end = 0;  // warp-uniform (ray counts < 2^32 - 2^25)
   bool exhausted = false;      // warp-uniform
   // Calls start(k) on every lane that is not active, for the next unclaimed
-  // ray positions k; start decides whether the lane becomes active. A single
-  // idle lane waits for a second one (unless no lane is active), so that the
-  // ray set-up, which only the refilled lanes execute, runs for two or more
-  // lanes at a time.
-  template <class Start>
+  // ray positions k; start decides whether the lane becomes active. Idle lanes
+  // wait until there are IDLE of them (unless no lane is active), so that the
+  // ray set-up, which only the refilled lanes execute, runs for that many
+  // lanes at a time. Any hit, 4.2M shadow rays over 1M triangles with 2, 4, 6,
+  // 8 lanes: 3,620, 3,596, 3,598, 3,660 us; closest hits over the exact nodes,
+  // 1M rays over 1M triangles with 2 and 4: 4,294, 4,343.
+  template <int IDLE, class Start>
   __device__ __forceinline__ void refill(bool active, uint32_t batch, uint32_t ray_count, unsigned int* work,
                                          Start&& start) {
     const int lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint32_t need = __ballot_sync(0xffffffffu, !active);
-    if (!need || (__popc(need) < 2 && need != 0xffffffffu)) return;
+    if (!need || (__popc(need) < IDLE && need != 0xffffffffu)) return;
     // first from what is left in the pool ...
     const uint32_t avail = end - next;
     if (avail) {
@@ -606,8 +608,11 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh4(TraceArgs a, uint32_t wa
 // subtree boxes (8 spill there). Without them 68 and 78 registers, and launches
 // handed on whole were 5 to 10 % slower (1M rays, 1M clustered triangles:
 // 6,190 us for 5,770; 200k sphere, SAH: 4,260 for 3,880).
+// Any hit, leaves in one loop and at least 7 blocks per SM asked for (64
+// registers either way, but another allocation; 9 spill: 5,080 us): those
+// shadow rays 3,817 -> 3,596 us, over the binned-SAH tree 4,358 -> 4,076.
 template <bool ANY_HIT, bool STATS, int CULL = kCullNone, bool FEW = false>
-__global__ void __launch_bounds__(kBlock, FEW ? (CULL ? 7 : 8) : 0) k_trace_mbvh(TraceArgs a, unsigned int* work) {
+__global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 7 : FEW ? (CULL ? 7 : 8) : 0) k_trace_mbvh(TraceArgs a, unsigned int* work) {
   RayState ray;
   float hu = 0.0f, hv = 0.0f;
   int32_t prim = -1;
@@ -674,7 +679,7 @@ __global__ void __launch_bounds__(kBlock, FEW ? (CULL ? 7 : 8) : 0) k_trace_mbvh
     }
   };
   for (;;) {
-    if (!pool.exhausted) pool.refill(active, batch, ray_count, work, start_ray);
+    if (!pool.exhausted) pool.refill<ANY_HIT ? 4 : 2>(active, batch, ray_count, work, start_ray);
     if (!__any_sync(0xffffffffu, active)) {
       if (pool.exhausted) break;
       continue;
@@ -697,6 +702,45 @@ __global__ void __launch_bounds__(kBlock, FEW ? (CULL ? 7 : 8) : 0) k_trace_mbvh
     else quad_intersect<false>(a.mnodes + current, ray, mask, ids, children, counts);
     if (CULL == kCullSubtree && cull) mask &= subtree_mask(a.tboxes + current, ray);
     if (STATS) ++visits;
+    if (ANY_HIT && !STATS && sp + 4 < kStack) {
+      // An accepted triangle ends the walk whatever the node pushed, so the
+      // pushes go first and the leaves' triangles follow in one loop, in their
+      // order; slot by slot, every slot was a loop of its own for the few
+      // lanes with a leaf there.
+      uint32_t leaves = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t id = (ids >> (2 * (3 - i))) & 3u;
+        const int32_t count = sel4(counts, id), lf = sel4(children, id);
+        if ((mask >> id) & 1u) {
+          if (count > -1) {
+            leaves |= 1u << i;
+          } else if (lf > -1) {
+            if (next >= 0) stack[++sp] = next;
+            next = lf;
+          }
+        }
+      }
+      int32_t j = 0;
+#pragma unroll 1
+      while (leaves) {
+        const uint32_t id = (ids >> (2 * (4 - __ffs(leaves)))) & 3u;
+        const int32_t count = sel4(counts, id), lf = sel4(children, id);
+        if (lf < 0 || (uint32_t)lf + (uint32_t)count > a.prim_count) {
+          atomicOr(a.status, kStatusBadIndex);
+          done = true;
+          break;
+        }
+        if (j < count && mt_test(a.tris + kTriFloat4 * (size_t)(lf + j), ray, hu, hv, prim)) {
+          done = true;
+          break;
+        }
+        if (++j >= count) {
+          leaves &= leaves - 1u;
+          j = 0;
+        }
+      }
+    } else
 #pragma unroll 1
     for (int i = 0; i < 4; ++i) {
       const uint32_t id = (ids >> (2 * (3 - i))) & 3u;
@@ -990,7 +1034,7 @@ __global__ void __launch_bounds__(kBlock, 9) k_trace_compact(TraceArgs a, unsign
     // incoherent rays +1 %; eight: incoherent +3 %.
     uint32_t amask = __ballot_sync(0xffffffffu, active);
     if (!pool.exhausted && __popc(amask) <= 28) {
-      pool.refill(active, batch, ray_count, work, start_ray);
+      pool.refill<2>(active, batch, ray_count, work, start_ray);
       amask = __ballot_sync(0xffffffffu, active);
     }
     if (!amask) {
