@@ -114,23 +114,33 @@ __device__ __forceinline__ uint32_t sibling_of(uint32_t x, uint32_t w) { return 
 // the next level is read meanwhile. Counts of 200k sphere
 // triangles 62 -> 22 us, of 1M 111 -> 39 us (before: parent, arrival counter,
 // node and both counts one after another); refit walk of 200k 80 -> 53 us.
+// Two leaves of a pair in one warp meet by shuffles, without the atomics (and
+// with TRIS their fences): 4M clustered triangles (SAH) 558 -> 521 us, 64 meshes
+// 187 -> 57. Blocks of 128 and 16 of them per SM (32 registers): a block stays
+// until its longest walk ends, mostly with a few lanes, so walks in flight are
+// what counts; the 4M build with 256 threads and 38 registers 8,336 us, 256 x 8
+// 8,104, 128 x 16 8,072, 64 x 32 8,088.
 // With TRIS, the same walk also computes every node's traversal box `tb`
 // from the triangles: a leaf's is the union of its triangles' vertex boxes
 // grown by 1e-4, an interior node's the union of its children's (the union
 // of boxes grown by 1e-4 is the union grown by 1e-4); count/left_first are
 // copied from `nodes`.
+constexpr int kCountBlock = 128, kCountBlocks = 16;
 template <bool TRIS>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kCountBlock, kCountBlocks)
     k_counts_bottom_up(const DAabb* __restrict__ nodes, uint32_t node_count, const uint32_t* __restrict__ parent,
                        uint64_t* __restrict__ cnt, MbvhTriangles tri, uint32_t* __restrict__ status) {
-  uint32_t c = blockIdx.x * kBlock + threadIdx.x;
-  if (c >= node_count) return;
-  uint32_t w = __ldg(parent + c);
-  DAabb box;
-  if (TRIS) {
-    const DAabb nd = load_aabb(nodes + c);
-    if (nd.count < 0) return;  // walks start at leaves
-    box = nd;
+  const uint32_t c = blockIdx.x * kCountBlock + threadIdx.x, lane = threadIdx.x & 31u;
+  uint32_t w = kNone;
+  bool leaf = false;  // walks start at leaves
+  DAabb box = {};
+  if (c < node_count) {
+    w = __ldg(parent + c);
+    if (TRIS) box = load_aabb(nodes + c);
+    leaf = (TRIS ? box.count : __ldg(&nodes[c].count)) >= 0;
+  }
+  if (TRIS && leaf) {
+    const DAabb nd = box;
     for (int a = 0; a < 3; ++a) { box.min[a] = 1e34f; box.max[a] = -1e34f; }
     if (nd.left_first >= 0) {
       for (int a = 0; a < 3; ++a) { box.min[a] = 1e34f - 0.0001f; box.max[a] = -1e34f + 0.0001f; }
@@ -146,10 +156,37 @@ __global__ void __launch_bounds__(kBlock)
       }
     }
     store_aabb(tri.tb + c, box);
-  } else if (__ldg(&nodes[c].count) < 0) {
-    return;
   }
   uint32_t x = c, e = 0, o = 0;
+  // two leaves of one pair: nothing else arrives at their parent
+  const uint32_t other = (w & 1u) ? lane - 1u : lane + 1u;
+  const uint32_t pair_w = __shfl_sync(0xffffffffu, leaf ? w : kNone, (int)(other & 31u));
+  const bool pair = leaf && w != kNone && other < 32u && pair_w == (w ^ 1u);
+  if (TRIS) {
+    for (int a = 0; a < 3; ++a) {
+      const float mn = __shfl_sync(0xffffffffu, box.min[a], (int)(other & 31u));
+      const float mx = __shfl_sync(0xffffffffu, box.max[a], (int)(other & 31u));
+      if (pair) {
+        box.min[a] = rs_min(box.min[a], mn);
+        box.max[a] = rs_max(box.max[a], mx);
+      }
+    }
+  }
+  if (!leaf || (pair && (w & 1u))) return;
+  if (pair) {
+    x = parent_of(w);
+    uint64_t sum = 2u * kArrived + 1u;
+    if (TRIS) {
+      const DAabb pn = load_aabb(nodes + x);
+      box.count = pn.count;
+      box.left_first = pn.left_first;
+      store_aabb(tri.tb + x, box);
+      if (!box_contains(pn, box)) sum |= kBadBox;
+    }
+    cnt[x] = sum;
+    e = 1;
+    w = __ldg(parent + x);
+  }
   for (uint32_t steps = 0; steps < node_count; ++steps) {
     if (w == kNone) break;
     const uint32_t p = parent_of(w);
@@ -1079,10 +1116,11 @@ cudaError_t launch_counts(const DAabb* nodes, uint32_t node_count, const Collaps
   if ((e = cudaMemsetAsync(w.parent, 0xff, (size_t)node_count * 4, s))) return e;
   const unsigned blocks = (node_count + kBlock - 1) / kBlock;
   k_parents<<<blocks, kBlock, 0, s>>>(nodes, node_count, w.parent, nullptr, w.cnt, w.known, status);
+  const unsigned count_blocks = (node_count + kCountBlock - 1) / kCountBlock;
   if (tri)
-    k_counts_bottom_up<true><<<blocks, kBlock, 0, s>>>(nodes, node_count, w.parent, w.cnt, *tri, status);
+    k_counts_bottom_up<true><<<count_blocks, kCountBlock, 0, s>>>(nodes, node_count, w.parent, w.cnt, *tri, status);
   else
-    k_counts_bottom_up<false><<<blocks, kBlock, 0, s>>>(nodes, node_count, w.parent, w.cnt, MbvhTriangles(),
+    k_counts_bottom_up<false><<<count_blocks, kCountBlock, 0, s>>>(nodes, node_count, w.parent, w.cnt, MbvhTriangles(),
                                                         status);
   return cudaGetLastError();
 }
