@@ -20,7 +20,7 @@
 //
 // After the last level, k_sub_build builds every listed subtree depth first,
 // one warp per subtree (bins in shared memory, the warp-parallel decision,
-// ballot partition); what is left, subtrees of at most kSmall primitives, is
+// ballot partition), large ones in two launches (kMid); what is left, subtrees of at most kSmall primitives, is
 // built by k_sub_small, one lane per primitive and several subtrees per warp.
 // Neither has grid-wide phases. The node pair of a split at primitive position
 // m goes to scratch slots 2(m-1), 2(m-1)+1 -- split positions are distinct
@@ -84,6 +84,7 @@ struct Counters {
   uint32_t sub_splits;  // splits inside the subtrees (the scan's total)
   uint32_t tiny;        // entries of the small-subtree list
   uint32_t tiny_head;   // next ones a warp of k_sub_small takes
+  uint32_t mid, mid_head;  // the same for the list of k_sub_build's second launch
 };
 
 struct BinMap {
@@ -362,6 +363,8 @@ struct SahParams {
   Task* subs;           // subtree tasks (at most sub_max primitives), all levels
   void* tiny;           // SubTask list: subtrees of at most kSmall primitives (empty entries have end 0)
   uint32_t small_cap;   // its capacity
+  void* mid;            // SubTask list: subtrees of at most kMid primitives (NULL: built in one go)
+  uint32_t mid_cap;
   Decision* dec;        // large tasks of the level
   float* tbox;          // 6 floats per large task (box with first offset)
   uint32_t* bins;       // kTaskBinWords per large task
@@ -1000,57 +1003,71 @@ __device__ __forceinline__ void first_offset(const SubTask& tk, float mn[3], flo
   }
 }
 
-// Entries of the small-subtree list that a warp reserves at a time: one atomic
-// per so many subtrees; what is left over when the warp ends is marked empty.
-constexpr uint32_t kListChunk = 32;
-struct SmallList {
+// A list of subtrees that warps append to, each reserving CHUNK entries at a
+// time: one atomic per so many subtrees. What is left over when the warp ends
+// is marked empty.
+template <uint32_t CHUNK>
+struct SubList {
+  SubTask* entries;
+  uint32_t cap;
+  uint32_t* count;
   uint32_t next = 0, end = 0;
+  __device__ __forceinline__ SubList(void* list, uint32_t capacity, uint32_t* counter)
+      : entries(reinterpret_cast<SubTask*>(list)), cap(capacity), count(counter) {}
   // by one lane of the warp
   __device__ __forceinline__ void add(const SahParams& p, const SubTask& t) {
     if (next == end) {
-      next = atomicAdd(&p.cnt->tiny, kListChunk);
-      end = next + kListChunk;
+      next = atomicAdd(count, CHUNK);
+      end = next + CHUNK;
     }
-    if (next < p.small_cap) reinterpret_cast<SubTask*>(p.tiny)[next] = t;
+    if (next < cap) entries[next] = t;
     else atomicOr(&p.cnt->status, kStatusBadIndex);
     ++next;
   }
-  __device__ __forceinline__ void finish(const SahParams& p) {
-    for (; next < end && next < p.small_cap; ++next) {
+  __device__ __forceinline__ void finish() {
+    for (; next < end && next < cap; ++next) {
       SubTask t = {};
-      reinterpret_cast<SubTask*>(p.tiny)[next] = t;
+      entries[next] = t;
     }
   }
 };
+constexpr uint32_t kListChunk = 32, kMidChunk = 4;
+using SmallList = SubList<kListChunk>;
+using MidList = SubList<kMidChunk>;
 
-// One subtree by one warp, depth first: tasks of more than kSmall primitives
-// by the whole warp; smaller ones are listed for k_sub_small. Every write goes
-// to a place fixed by the task's primitive range, so the order in which tasks
-// run does not matter.
-__device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& sh, SmallList& list) {
+// Builds with subtrees of more than kMidFrom primitives build them in two
+// launches: the first splits every subtree until its parts are at most kMid,
+// the second builds the parts. In one, a warp that has a whole subtree of up
+// to 1,024 primitives is busy for a third of the launch, and there are fewer
+// than three of them for each. 4M clustered triangles in one launch 8,077 us;
+// kMid 512: 8,047, 256: 7,871, 128: 7,828, 64: 7,871; 700k 2,345 in one, 2,285
+// in two, 520k 2,028 and 1,960, 400k 1,824 and 1,772, but 300k 1,504 and 1,500,
+// 270k 1,452 and 1,471. Five or six blocks per SM (102 or 80 registers) and
+// less shared memory in the second launch: no faster.
+constexpr uint32_t kMid = 128, kMidFrom = 160;
+
+// One subtree (index array of its level in idx_a) by one warp, depth first:
+// tasks of more than kSmall primitives by the whole warp; smaller ones are
+// listed for k_sub_small and, with SPLIT, those of up to kMid for the second
+// launch. Every write goes to a place fixed by the task's primitive range, so
+// the order in which tasks run does not matter.
+template <bool SPLIT>
+__device__ void sub_warp_tree(const SahParams& p, const SubTask& root, SubShared& sh, SmallList& list, MidList& mids) {
   const int lane = threadIdx.x & 31;
   int sp = -1;  // warp-uniform
-  const uint32_t rws = root.end - root.begin;
-  // a subtree that hangs below an even level has its indices in idx_b
-  if (root.depth & 1u)
-    for (uint32_t i = root.begin + lane; i < root.end; i += 32) p.idx_a[i] = __ldcg(p.idx_b + i);
-  __syncwarp();
-  if (lane == 0) {
-    const DAabb rb = load_aabb_cg(p.nodes + root.node);
-    SubTask t;
-    t.loc = root.node;
-    t.begin = root.begin;
-    t.end = root.end;
-    t.depth = root.depth;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      t.box[k] = rb.min[k];
-      t.box[3 + k] = rb.max[k];
+  // true where the task goes onto the stack; by all lanes, with the same task
+  auto keep = [&](uint32_t size, const SubTask& t) {
+    if (size <= kSmall) {
+      if (lane == 0) list.add(p, t);
+    } else if (SPLIT && size <= kMid) {
+      if (lane == 0) mids.add(p, t);
+    } else {
+      if (lane == 0) sh.stack[sp + 1] = t;
+      return true;
     }
-    if (rws <= kSmall) list.add(p, t);
-    else sh.stack[0] = t;
-  }
-  if (rws > kSmall) sp = 0;
+    return false;
+  };
+  if (keep(root.end - root.begin, root)) sp = 0;
   __syncwarp();
   while (sp >= 0) {
     const SubTask tk = sh.stack[sp--];
@@ -1068,21 +1085,31 @@ __device__ void sub_warp_tree(const SahParams& p, const Task& root, SubShared& s
         return;
       }
       // right child first onto the stack: the left one is taken next
-      if (nr <= kSmall) {
-        if (lane == 0) list.add(p, r);
-      } else {
-        if (lane == 0) sh.stack[sp + 1] = r;
-        ++sp;
-      }
-      if (nl <= kSmall) {
-        if (lane == 0) list.add(p, l);
-      } else {
-        if (lane == 0) sh.stack[sp + 1] = l;
-        ++sp;
-      }
+      if (keep(nr, r)) ++sp;
+      if (keep(nl, l)) ++sp;
     }
     __syncwarp();
   }
+}
+
+// The listed subtree t of the breadth-first part, with its indices in idx_a.
+__device__ __forceinline__ SubTask sub_root(const SahParams& p, const Task& root) {
+  // a subtree that hangs below an even level has its indices in idx_b
+  if (root.depth & 1u)
+    for (uint32_t i = root.begin + (threadIdx.x & 31u); i < root.end; i += 32) p.idx_a[i] = __ldcg(p.idx_b + i);
+  __syncwarp();
+  const DAabb rb = load_aabb_cg(p.nodes + root.node);
+  SubTask t;
+  t.loc = root.node;
+  t.begin = root.begin;
+  t.end = root.end;
+  t.depth = root.depth;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    t.box[k] = rb.min[k];
+    t.box[3 + k] = rb.max[k];
+  }
+  return t;
 }
 
 // ------------------------------------------------------------------ subtrees of at most kSmall primitives
@@ -1639,20 +1666,34 @@ __global__ void __launch_bounds__(kLargeBlock) k_ph_advance(SahParams p, uint32_
 }
 
 // ---- subtrees and their placement
+enum SubPass { kSubWhole, kSubSplit, kSubRest };
+template <int PASS>
 __global__ void __launch_bounds__(kSubBlock) k_sub_build(SahParams p) {
   extern __shared__ __align__(16) unsigned char sub_dyn[];
   SubShared& sh = reinterpret_cast<SubShared*>(sub_dyn)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
-  const uint32_t S = __ldcg(&p.cnt->sub);
-  SmallList list;  // lane 0's
+  const uint32_t S = PASS == kSubRest ? min(__ldcg(&p.cnt->mid), p.mid_cap) : __ldcg(&p.cnt->sub);
+  uint32_t* const head = PASS == kSubRest ? &p.cnt->mid_head : &p.cnt->sub_head;
+  SmallList list(p.tiny, p.small_cap, &p.cnt->tiny);  // lane 0's
+  MidList mids(p.mid, p.mid_cap, &p.cnt->mid);
   for (;;) {
     uint32_t t = 0;
-    if (lane == 0) t = atomicAdd(&p.cnt->sub_head, 1u);
+    if (lane == 0) t = atomicAdd(head, 1u);
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t >= S) break;
-    sub_warp_tree(p, ld_task(p.subs + t), sh, list);
+    SubTask root;
+    if (PASS == kSubRest) {
+      root = reinterpret_cast<const SubTask*>(p.mid)[t];
+      if (root.end == 0u) continue;
+    } else {
+      root = sub_root(p, ld_task(p.subs + t));
+    }
+    sub_warp_tree<PASS == kSubSplit>(p, root, sh, list, mids);
   }
-  if (lane == 0) list.finish(p);
+  if (lane == 0) {
+    list.finish();
+    if (PASS == kSubSplit) mids.finish();
+  }
 }
 
 // The listed subtrees of at most kSmall primitives: a warp takes 32 entries at a
@@ -1825,6 +1866,8 @@ __global__ void k_sah_init(SahParams p, const DAabb* world) {
     p.cnt->sub_splits = 0;
     p.cnt->tiny = 0;
     p.cnt->tiny_head = 0;
+    p.cnt->mid = 0;
+    p.cnt->mid_head = 0;
   }
 }
 
@@ -1873,18 +1916,21 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   const uint32_t tiles = (n + kScanTile - 1) / kScanTile;
   int sub_per_sm = 0;
   const size_t sub_smem = (kSubBlock / 32) * sizeof(SubShared);
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sub_per_sm, k_sub_build, kSubBlock, sub_smem)))
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sub_per_sm, k_sub_build<kSubWhole>, kSubBlock, sub_smem)))
     return fail(cuda_rc(e));
   if (sub_per_sm < 1) return fail(DeviceError);
   uint32_t sub_grid = (uint32_t)sm_count() * (uint32_t)sub_per_sm;
   const uint32_t want = (n / (sub_max > 8u ? 8u : sub_max) + kSubBlock / 32) / (kSubBlock / 32) + 1u;
   if (want < sub_grid) sub_grid = want;
   // listed subtrees hold a primitive or more; every warp may leave a chunk
-  const uint32_t small_cap = n + sub_grid * (kSubBlock / 32) * kListChunk;
+  const bool two_launches = sub_max > kMidFrom;
+  const uint32_t sub_warps = sub_grid * (kSubBlock / 32);
+  const uint32_t small_cap = n + sub_warps * kListChunk * (two_launches ? 2u : 1u);
+  const uint32_t mid_cap = two_launches ? n / (kSmall + 1u) + sub_warps * kMidChunk : 0u;
   Scratch<DAabb> world, tnodes;
   Scratch<uint32_t> acc, idx_b, bins, chunk_base, chunk_status, sflag, srank, tile_off;
   Scratch<Task> large0, large1, subs;
-  Scratch<SubTask> tiny;
+  Scratch<SubTask> tiny, mid;
   Scratch<Decision> dec;
   Scratch<float> tbox;
   Scratch<uint64_t> scan_vals, scan_sums;
@@ -1896,7 +1942,8 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
       (e = subs.alloc(sub_cap, s)) || (e = dec.alloc(large_cap, s)) || (e = tbox.alloc((size_t)large_cap * 6, s)) ||
       (e = scan_vals.alloc(large_cap, s)) || (e = scan_sums.alloc(grid, s)) || (e = cnt.alloc(1, s)) ||
       (e = bar.alloc(1, s)) || (e = tnodes.alloc(2 * (size_t)n, s)) || (e = sflag.alloc(n, s)) ||
-      (e = srank.alloc(n, s)) || (e = tile_off.alloc(tiles + 1, s)) || (e = tiny.alloc(small_cap, s)))
+      (e = srank.alloc(n, s)) || (e = tile_off.alloc(tiles + 1, s)) || (e = tiny.alloc(small_cap, s)) ||
+      (two_launches && (e = mid.alloc(mid_cap, s))))
     return fail(cuda_rc(e));
   if ((e = cudaMemsetAsync(chunk_status.ptr, 0, (size_t)chunk_cap * 4, s)) ||
       (e = cudaMemsetAsync(bar.ptr, 0, sizeof(GridBarrier), s)) ||
@@ -1918,6 +1965,8 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   p.subs = subs.ptr;
   p.tiny = tiny.ptr;
   p.small_cap = small_cap;
+  p.mid = mid.ptr;
+  p.mid_cap = mid_cap;
   p.dec = dec.ptr;
   p.tbox = tbox.ptr;
   p.bins = bins.ptr;
@@ -1975,7 +2024,12 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   // kernels read the subtree count and the breadth-first node count on the
   // device)
   {
-    k_sub_build<<<sub_grid, kSubBlock, sub_smem, s>>>(p);
+    if (two_launches) {
+      k_sub_build<kSubSplit><<<sub_grid, kSubBlock, sub_smem, s>>>(p);
+      k_sub_build<kSubRest><<<sub_grid, kSubBlock, sub_smem, s>>>(p);
+    } else {
+      k_sub_build<kSubWhole><<<sub_grid, kSubBlock, sub_smem, s>>>(p);
+    }
     int small_per_sm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&small_per_sm, k_sub_small, kSubBlock, 0)))
       return fail(cuda_rc(e));

@@ -53,3 +53,14 @@ def test_sah_above_the_cooperative_size(n, kind):
     assert len(nodes) == len(on)
     assert np.array_equal(np.sort(idx), np.arange(len(tris)))
     assert np.array_equal(u32(oracle.mbvh(nodes)), u32(oracle.mbvh(on)))
+
+
+@pytest.mark.parametrize("n,kind", [(329727, "soup"), (329728, "soup"), (330001, "equal"), (340007, "sphere")])
+def test_sah_subtrees_in_two_launches(n, kind):
+    """From 329,728 primitives subtrees have more than 160 and are split first."""
+    tris = _scene(n, kind)
+    g = gpu_build(tris, "sah")
+    on, oi = oracle_build(tris, "sah", 1)
+    nodes, idx = g.nodes(), g.indices()
+    assert len(nodes) == len(on)
+    assert canonical(nodes, idx) == canonical(on, oi)
