@@ -47,6 +47,43 @@ struct Scratch {
   Scratch& operator=(const Scratch&) = delete;
 };
 
+// Several scratch arrays in one allocation (each on a 256-byte boundary). An
+// allocation and its free cost the host 3 us, and small builds wait for the
+// host: binned SAH took 20 of them, LOCB 11. SAH build
+// of 6,400 triangles 633 -> 605 us, LOCB build of 64 341 -> 320.
+struct ScratchPack {
+  template <class T>
+  void add(T** p, size_t n) {
+    arrays[count++] = {reinterpret_cast<void**>(p), bytes};
+    bytes += (n * sizeof(T) + 255) & ~(size_t)255;
+  }
+  cudaError_t alloc(cudaStream_t s) {
+    stream = s;
+    const cudaError_t e = pool_alloc(reinterpret_cast<void**>(&base), bytes, s);
+    if (e) return e;
+    for (int i = 0; i < count; ++i) *arrays[i].p = base + arrays[i].offset;
+    return cudaSuccess;
+  }
+  ~ScratchPack() {
+    if (base) pool_free(base, stream);
+  }
+  ScratchPack() = default;
+  ScratchPack(const ScratchPack&) = delete;
+  ScratchPack& operator=(const ScratchPack&) = delete;
+
+ private:
+  struct Array {
+    void** p;
+    size_t offset;
+  };
+  static constexpr int kMost = 24;
+  Array arrays[kMost];
+  int count = 0;
+  size_t bytes = 0;
+  char* base = nullptr;
+  cudaStream_t stream = nullptr;
+};
+
 // ------------------------------------------------------------------ prep
 // Triangle::aabb / Triangle::center (shared/src/lib.rs:27-39) of n triangles
 // (9 floats each). centers are written as float4 (w = 0).

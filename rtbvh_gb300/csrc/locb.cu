@@ -944,36 +944,6 @@ ResultCode build_locb(const DAabb* aabbs, const float4* centers, size_t n_, cuda
     pool_free(indices, s);
     return rc;
   };
-  Scratch<DAabb> world;
-  Scratch<uint32_t> acc, status;
-  if ((e = world.alloc(1, s)) || (e = acc.alloc(kBoundsWords, s)) || (e = status.alloc(4, s))) return fail(cuda_rc(e));
-  if ((e = cudaMemsetAsync(status.ptr, 0, 16, s))) return fail(cuda_rc(e));
-  if ((e = launch_world_bounds(aabbs, n, world.ptr, acc.ptr, s))) return fail(cuda_rc(e));
-  if (n <= 2) {
-    k_locb_single<<<1, 32, 0, s>>>(world.ptr, n, nodes, indices);
-    if ((e = cudaGetLastError()) || (e = cudaStreamSynchronize(s))) return fail(cuda_rc(e));
-    out->nodes = nodes;
-    out->indices = indices;
-    out->node_count = 1;
-    return Ok;
-  }
-  Scratch<uint32_t> keys;
-  Scratch<char> sort_temp;
-  const size_t sort_bytes = radix_sort_temp_bytes(n);
-  if ((e = keys.alloc(n, s)) || (e = sort_temp.alloc(sort_bytes, s))) return fail(cuda_rc(e));
-  if ((e = launch_morton(centers, n, world.ptr, keys.ptr, indices, s))) return fail(cuda_rc(e));
-  if ((e = radix_sort_pairs(keys.ptr, indices, n, 30, sort_temp.ptr, sort_bytes, status.ptr, s)))
-    return fail(cuda_rc(e));
-
-  Scratch<DAabb> lvl0, lvl1;
-  Scratch<uint32_t> nb, blocksum, info;
-  Scratch<GridBarrier> bar;
-  if ((e = lvl0.alloc(node_count, s)) || (e = lvl1.alloc(node_count, s)) || (e = nb.alloc(node_count, s)) ||
-      (e = info.alloc(4, s)) || (e = bar.alloc(1, s)))
-    return fail(cuda_rc(e));
-  k_locb_leaves<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(aabbs, indices, n, lvl0.ptr);
-  if ((e = cudaGetLastError())) return fail(cuda_rc(e));
-
   int dev = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_locb_levels, kBlock, 0);
@@ -986,19 +956,47 @@ ResultCode build_locb(const DAabb* aabbs, const float4* centers, size_t n_, cuda
   const unsigned useful = (unsigned)((n + kBlock - 1) / kBlock);
   if (grid > useful) grid = useful;
   if (grid < 1) grid = 1;
-  if ((e = blocksum.alloc(grid, s)) || (e = cudaMemsetAsync(bar.ptr, 0, sizeof(GridBarrier), s)))
-    return fail(cuda_rc(e));
+  ScratchPack scratch;
+  DAabb *world, *lvl0 = nullptr, *lvl1 = nullptr;
+  uint32_t *acc, *status, *keys = nullptr, *nb = nullptr, *blocksum = nullptr;
+  char* sort_temp = nullptr;
+  constexpr size_t kBarWords = (sizeof(GridBarrier) + 3) / 4;
+  const size_t sort_bytes = radix_sort_temp_bytes(n);
+  scratch.add(&world, 1);
+  scratch.add(&acc, kBoundsWords);
+  scratch.add(&status, 8 + kBarWords);  // status, info, barrier
+  if (n > 2) {
+    scratch.add(&keys, n);
+    scratch.add(&sort_temp, sort_bytes);
+    scratch.add(&lvl0, node_count);
+    scratch.add(&lvl1, node_count);
+    scratch.add(&nb, node_count);
+    scratch.add(&blocksum, grid);
+  }
+  if ((e = scratch.alloc(s)) || (e = cudaMemsetAsync(status, 0, (8 + kBarWords) * 4, s))) return fail(cuda_rc(e));
+  if ((e = launch_world_bounds(aabbs, n, world, acc, s))) return fail(cuda_rc(e));
+  if (n <= 2) {
+    k_locb_single<<<1, 32, 0, s>>>(world, n, nodes, indices);
+    if ((e = cudaGetLastError()) || (e = cudaStreamSynchronize(s))) return fail(cuda_rc(e));
+    out->nodes = nodes;
+    out->indices = indices;
+    out->node_count = 1;
+    return Ok;
+  }
+  if ((e = launch_morton(centers, n, world, keys, indices, s))) return fail(cuda_rc(e));
+  if ((e = radix_sort_pairs(keys, indices, n, 30, sort_temp, sort_bytes, status, s))) return fail(cuda_rc(e));
+  k_locb_leaves<<<(n + kBlock - 1) / kBlock, kBlock, 0, s>>>(aabbs, indices, n, lvl0);
+  if ((e = cudaGetLastError())) return fail(cuda_rc(e));
 
-  if ((e = cudaMemsetAsync(info.ptr, 0, 4 * sizeof(uint32_t), s))) return fail(cuda_rc(e));
   LocbParams p;
-  p.lvl[0] = lvl0.ptr;
-  p.lvl[1] = lvl1.ptr;
+  p.lvl[0] = lvl0;
+  p.lvl[1] = lvl1;
   p.final_nodes = nodes;
-  p.nb = nb.ptr;
-  p.blocksum = blocksum.ptr;
-  p.bar = bar.ptr;
-  p.status = status.ptr;
-  p.info = info.ptr;
+  p.nb = nb;
+  p.blocksum = blocksum;
+  p.bar = reinterpret_cast<GridBarrier*>(status + 8);
+  p.status = status;
+  p.info = status + 4;
   p.n = n;
   const unsigned blocks = cluster_size();
   p.stop = blocks * kClusterCap;
@@ -1010,7 +1008,7 @@ ResultCode build_locb(const DAabb* aabbs, const float4* centers, size_t n_, cuda
   }
   if ((e = launch_cluster(k_locb_cluster, 1, blocks, s, p, wide, n - 1u, node_count))) return fail(cuda_rc(e));
   uint32_t h_status = 0;
-  if ((e = cudaMemcpyAsync(&h_status, status.ptr, 4, cudaMemcpyDeviceToHost, s)) ||
+  if ((e = cudaMemcpyAsync(&h_status, status, 4, cudaMemcpyDeviceToHost, s)) ||
       (e = cudaStreamSynchronize(s)))
     return fail(cuda_rc(e));
   if (h_status & kStatusTimeout) return fail(Timeout);

@@ -1196,11 +1196,14 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
   const bool check_nested = req.wide && !tri;
   const uint32_t* check_indices = req.wide ? req.check_indices : nullptr;
   cudaError_t e;
-  Scratch<uint32_t> words, seen;
+  Scratch<uint32_t> seen;
+  ScratchPack scratch;
   // result words: 0 status, 1 check (not nested, duplicate leaf slots), 2
   // primitives in leaves, 3 escaped triangles, 4 quad nodes, 5 traversal nodes
-  Scratch<uint32_t> res;
-  if ((e = words.alloc(collapse_scratch_words(node_count), s)) || (e = res.alloc(8, s))) return cuda_rc(e);
+  uint32_t *words, *res;
+  scratch.add(&words, collapse_scratch_words(node_count));
+  scratch.add(&res, 8);
+  if ((e = scratch.alloc(s))) return cuda_rc(e);
   auto drop = [&](ResultCode rc) {
     pool_free(out->mnodes, s);
     pool_free(out->tboxes, s);
@@ -1213,11 +1216,11 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
   if (tri && (e = device_alloc(&out->tboxes, m_cap, s))) return drop(cuda_rc(e));
   if (req.wide && ((e = device_alloc(&out->wnodes, m_cap, s)) || (e = device_alloc(&out->wq, m_cap, s))))
     return drop(cuda_rc(e));
-  if ((e = cudaMemsetAsync(res.ptr, 0, 32, s))) return drop(cuda_rc(e));
-  const CollapseScratch w(words.ptr, node_count);
-  if ((e = launch_counts(nodes, node_count, w, tri, res.ptr, s))) return drop(cuda_rc(e));
+  if ((e = cudaMemsetAsync(res, 0, 32, s))) return drop(cuda_rc(e));
+  const CollapseScratch w(words, node_count);
+  if ((e = launch_counts(nodes, node_count, w, tri, res, s))) return drop(cuda_rc(e));
   const unsigned blocks = (node_count + kBlock - 1) / kBlock;
-  k_root_place<<<1, 32, 0, s>>>(w.cnt, nodes, w.known, m_cap, res.ptr + 4, res.ptr + 5, res.ptr);
+  k_root_place<<<1, 32, 0, s>>>(w.cnt, nodes, w.known, m_cap, res + 4, res + 5, res);
   CollapseParams p = {};
   p.nodes = nodes;
   p.node_count = node_count;
@@ -1227,10 +1230,10 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
   p.quads = w.quads;
   p.mnodes = out->mnodes;
   p.m_total = m_cap;
-  p.m_count = res.ptr + 4;
-  p.status = res.ptr;
+  p.m_count = res + 4;
+  p.status = res;
   if (tri) p.tri = *tri;
-  p.escaped = res.ptr + 3;
+  p.escaped = res + 3;
   p.tboxes = out->tboxes;
   if (!req.wide) {
     if ((e = launch_nodes(p, tri != nullptr, nullptr, s))) return drop(cuda_rc(e));
@@ -1239,7 +1242,7 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
       if ((e = seen.alloc(req.index_count, s)) || (e = cudaMemsetAsync(seen.ptr, 0, (size_t)req.index_count * 4, s)))
         return drop(cuda_rc(e));
       k_check_leaves<<<blocks, kBlock, 0, s>>>(nodes, node_count, check_indices, req.index_count, seen.ptr,
-                                               res.ptr + 2, res.ptr + 1);
+                                               res + 2, res + 1);
     }
     WideParams q = {};
     q.nodes = tri ? tri->tb : nodes;
@@ -1252,15 +1255,15 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
     q.wnodes = out->wnodes;
     q.wq = out->wq;
     q.capacity = m_cap;
-    q.walloc = res.ptr + 5;
-    q.status = res.ptr;
-    q.check = res.ptr + 1;
+    q.walloc = res + 5;
+    q.status = res;
+    q.check = res + 1;
     q.check_nested = check_nested;
     q.expect_seen = check_indices ? req.index_count : kNone;
     if ((e = launch_nodes(p, tri != nullptr, &q, s))) return drop(cuda_rc(e));
   }
   uint32_t h[6];
-  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(h, res.ptr, 24, cudaMemcpyDeviceToHost, s)) ||
+  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(h, res, 24, cudaMemcpyDeviceToHost, s)) ||
       (e = cudaStreamSynchronize(s)))
     return drop(cuda_rc(e));
   if (h[0] != 0) return drop((h[0] & kStatusTimeout) ? Timeout : Error);

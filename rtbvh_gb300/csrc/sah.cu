@@ -1927,60 +1927,71 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   const uint32_t sub_warps = sub_grid * (kSubBlock / 32);
   const uint32_t small_cap = n + sub_warps * kListChunk * (two_launches ? 2u : 1u);
   const uint32_t mid_cap = two_launches ? n / (kSmall + 1u) + sub_warps * kMidChunk : 0u;
-  Scratch<DAabb> world, tnodes;
-  Scratch<uint32_t> acc, idx_b, bins, chunk_base, chunk_status, sflag, srank, tile_off;
-  Scratch<Task> large0, large1, subs;
-  Scratch<SubTask> tiny, mid;
-  Scratch<Decision> dec;
-  Scratch<float> tbox;
-  Scratch<uint64_t> scan_vals, scan_sums;
-  Scratch<Counters> cnt;
-  Scratch<GridBarrier> bar;
-  if ((e = world.alloc(1, s)) || (e = acc.alloc(kBoundsWords, s)) || (e = idx_b.alloc(n, s)) ||
-      (e = bins.alloc((size_t)large_cap * kTaskBinWords, s)) || (e = chunk_base.alloc(large_cap + 1, s)) ||
-      (e = chunk_status.alloc(chunk_cap, s)) || (e = large0.alloc(large_cap, s)) || (e = large1.alloc(large_cap, s)) ||
-      (e = subs.alloc(sub_cap, s)) || (e = dec.alloc(large_cap, s)) || (e = tbox.alloc((size_t)large_cap * 6, s)) ||
-      (e = scan_vals.alloc(large_cap, s)) || (e = scan_sums.alloc(grid, s)) || (e = cnt.alloc(1, s)) ||
-      (e = bar.alloc(1, s)) || (e = tnodes.alloc(2 * (size_t)n, s)) || (e = sflag.alloc(n, s)) ||
-      (e = srank.alloc(n, s)) || (e = tile_off.alloc(tiles + 1, s)) || (e = tiny.alloc(small_cap, s)) ||
-      (two_launches && (e = mid.alloc(mid_cap, s))))
-    return fail(cuda_rc(e));
-  if ((e = cudaMemsetAsync(chunk_status.ptr, 0, (size_t)chunk_cap * 4, s)) ||
-      (e = cudaMemsetAsync(bar.ptr, 0, sizeof(GridBarrier), s)) ||
-      (e = cudaMemsetAsync(sflag.ptr, 0, (size_t)n * 4, s)))
-    return fail(cuda_rc(e));
-  if ((e = launch_world_bounds(aabbs, n, world.ptr, acc.ptr, s))) return fail(cuda_rc(e));
+  constexpr size_t kBarWords = (sizeof(GridBarrier) + 3) / 4;
+  const size_t zero_words = kBarWords + chunk_cap + n;
+  ScratchPack scratch;
+  DAabb *world, *tnodes;
+  uint32_t *acc, *idx_b, *bins, *chunk_base, *zeros, *srank, *tile_off;
+  Task *large0, *large1, *subs;
+  SubTask *tiny, *mid;
+  Decision* dec;
+  float* tbox;
+  uint64_t *scan_vals, *scan_sums;
+  Counters* cnt;
+  scratch.add(&world, 1);
+  scratch.add(&acc, kBoundsWords);
+  scratch.add(&idx_b, n);
+  scratch.add(&bins, (size_t)large_cap * kTaskBinWords);
+  scratch.add(&chunk_base, large_cap + 1);
+  scratch.add(&zeros, zero_words);  // barrier, chunk status, split flags
+  scratch.add(&large0, large_cap);
+  scratch.add(&large1, large_cap);
+  scratch.add(&subs, sub_cap);
+  scratch.add(&dec, large_cap);
+  scratch.add(&tbox, (size_t)large_cap * 6);
+  scratch.add(&scan_vals, large_cap);
+  scratch.add(&scan_sums, grid);
+  scratch.add(&cnt, 1);
+  scratch.add(&tnodes, 2 * (size_t)n);
+  scratch.add(&srank, n);
+  scratch.add(&tile_off, tiles + 1);
+  scratch.add(&tiny, small_cap);
+  scratch.add(&mid, mid_cap);
+  if ((e = scratch.alloc(s)) || (e = cudaMemsetAsync(zeros, 0, zero_words * 4, s))) return fail(cuda_rc(e));
+  uint32_t* const chunk_status = zeros + kBarWords;
+  uint32_t* const sflag = chunk_status + chunk_cap;
+  if ((e = launch_world_bounds(aabbs, n, world, acc, s))) return fail(cuda_rc(e));
 
   SahParams p;
   p.aabbs = aabbs;
   p.centers = centers;
   p.nodes = nodes;
   p.idx_a = indices;
-  p.idx_b = idx_b.ptr;
+  p.idx_b = idx_b;
   p.n = n;
   p.sub_max = sub_max;
   p.max_leaf = prims_per_leaf == 0 ? 1u : (uint32_t)(prims_per_leaf > 0xffffffffu ? 0xffffffffu : prims_per_leaf);
-  p.large[0] = large0.ptr;
-  p.large[1] = large1.ptr;
-  p.subs = subs.ptr;
-  p.tiny = tiny.ptr;
+  p.large[0] = large0;
+  p.large[1] = large1;
+  p.subs = subs;
+  p.tiny = tiny;
   p.small_cap = small_cap;
-  p.mid = mid.ptr;
+  p.mid = mid;
   p.mid_cap = mid_cap;
-  p.dec = dec.ptr;
-  p.tbox = tbox.ptr;
-  p.bins = bins.ptr;
-  p.chunk_base = chunk_base.ptr;
-  p.chunk_status = chunk_status.ptr;
-  p.scan_vals = scan_vals.ptr;
-  p.scan_sums = scan_sums.ptr;
-  p.tnodes = tnodes.ptr;
-  p.sflag = sflag.ptr;
-  p.srank = srank.ptr;
-  p.tile_off = tile_off.ptr;
-  p.cnt = cnt.ptr;
-  p.bar = bar.ptr;
-  k_sah_init<<<(n + 255) / 256, 256, 0, s>>>(p, world.ptr);
+  p.dec = dec;
+  p.tbox = tbox;
+  p.bins = bins;
+  p.chunk_base = chunk_base;
+  p.chunk_status = chunk_status;
+  p.scan_vals = scan_vals;
+  p.scan_sums = scan_sums;
+  p.tnodes = tnodes;
+  p.sflag = sflag;
+  p.srank = srank;
+  p.tile_off = tile_off;
+  p.cnt = cnt;
+  p.bar = reinterpret_cast<GridBarrier*>(zeros);
+  k_sah_init<<<(n + 255) / 256, 256, 0, s>>>(p, world);
   Counters h{};
   if (n > sub_max) {
     if (coop) {
@@ -2011,7 +2022,7 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
           k_ph_advance<<<1, kLargeBlock, kShSmall, s>>>(p, level, grid);
         }
         if ((e = cudaGetLastError())) return fail(cuda_rc(e));
-        if ((e = cudaMemcpyAsync(&h, cnt.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, s)) ||
+        if ((e = cudaMemcpyAsync(&h, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s)) ||
             (e = cudaStreamSynchronize(s)))
           return fail(cuda_rc(e));
         if (h.status) break;
@@ -2036,15 +2047,15 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
     const uint32_t small_grid = (uint32_t)sm_count() * (uint32_t)(small_per_sm < 1 ? 1 : small_per_sm);
     const uint32_t small_want = (small_cap / 32u + kSubBlock / 32) / (kSubBlock / 32);
     k_sub_small<<<small_want < small_grid ? small_want : small_grid, kSubBlock, 0, s>>>(p);
-    k_tile_sums<<<tiles, 1024, 0, s>>>(sflag.ptr, n, tile_off.ptr);
-    k_tile_scan<<<1, 1024, 0, s>>>(tile_off.ptr, tiles, cnt.ptr);
-    k_rank<<<tiles, 1024, 0, s>>>(sflag.ptr, n, tile_off.ptr, srank.ptr);
+    k_tile_sums<<<tiles, 1024, 0, s>>>(sflag, n, tile_off);
+    k_tile_scan<<<1, 1024, 0, s>>>(tile_off, tiles, cnt);
+    k_rank<<<tiles, 1024, 0, s>>>(sflag, n, tile_off, srank);
     k_relocate<<<(n + kLargeBlock - 1) / kLargeBlock, kLargeBlock, 0, s>>>(p);
     const unsigned fix_blocks = (unsigned)((n + kLargeBlock) / kLargeBlock);
     k_fix_roots<<<fix_blocks < (unsigned)sm_count() * 4u ? fix_blocks : (unsigned)sm_count() * 4u, kLargeBlock, 0,
                   s>>>(p);
     if ((e = cudaGetLastError())) return fail(cuda_rc(e));
-    if ((e = cudaMemcpyAsync(&h, cnt.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, s)) ||
+    if ((e = cudaMemcpyAsync(&h, cnt, sizeof(Counters), cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
       return fail(cuda_rc(e));
     if (h.status) return fail(h.status & kStatusTimeout ? Timeout : Error);
