@@ -702,7 +702,10 @@ __global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 7 : FEW ? (CULL 
     else quad_intersect<false>(a.mnodes + current, ray, mask, ids, children, counts);
     if (CULL == kCullSubtree && cull) mask &= subtree_mask(a.tboxes + current, ray);
     if (STATS) ++visits;
-    if (ANY_HIT && !STATS && sp + 4 < kStack) {
+    if (ANY_HIT && !STATS && mask == 0u) {
+      // nothing to do: most visits of rays that miss (16.8M rays ending short
+      // of the scene 318 -> 265 us)
+    } else if (ANY_HIT && !STATS && sp + 4 < kStack) {
       // An accepted triangle ends the walk whatever the node pushed, so the
       // pushes go first and the leaves' triangles follow in one loop, in their
       // order; slot by slot, every slot was a loop of its own for the few
