@@ -176,7 +176,7 @@ struct Plan {
   size_t sort_bytes = 0;
   // meshes order[0, big_count) get a thread-block cluster each (locb.cu)
   uint32_t big_count = 0;
-  unsigned clusters = 0;
+  unsigned clusters = 0, cluster_blocks = kSegCluster;
   DevBuf<uint32_t> cluster_sums;
   std::vector<uint32_t> sizes_in_order;  // host: primitive count of order[q]
   // launch parameters (RTBatchTuning; 0 = default)
@@ -201,12 +201,27 @@ constexpr uint32_t kMaxClusters = 8192;
 
 // Meshes above `min_prims` primitives (a prefix of the size-ordered mesh
 // list) are clustered by block clusters; meshes of at most 2 primitives
-// always take the single-block path.
+// always take the single-block path. At the default threshold only meshes with
+// more than 1.4 halves of an SM's share of all primitives are: a block keeps an
+// SM to itself, and a level in a cluster of 8 takes more than an eighth of its
+// time in one block, so many meshes are better off with a block or two each.
+// Clustering of meshes of one size, us, with 1 / 2 / 4 / 8 blocks: 700 of 5,000
+// triangles 3,067 / 3,231 / 3,766 / 6,195; 200 of 20,000 4,555 / 3,890 / 3,996
+// / 4,734; 64 of 20,000 2,081 / 1,420 / 1,468 / 1,778; 100 of 50,000 6,338 /
+// 6,166 / 5,213 / 5,986; 8 of 150,000 13,320 / 7,077 / 3,920 / 2,358.
 void set_cluster_min(Plan& p, uint32_t min_prims) {
   p.cluster_min = min_prims < 2u ? 2u : min_prims;
+  const uint64_t blocks2 = 2ull * (uint64_t)sm_count();
+  uint64_t above = p.cluster_min;
+  if (p.cluster_min == kSegClusterMinPrims) above = std::max<uint64_t>(above, p.total_prims * 10ull / (blocks2 * 7ull));
   p.big_count = 0;
-  while (p.big_count < p.mesh_count && p.sizes_in_order[p.big_count] > p.cluster_min) ++p.big_count;
+  while (p.big_count < p.mesh_count && p.sizes_in_order[p.big_count] > above) ++p.big_count;
   p.clusters = std::min<uint32_t>(p.big_count, kMaxClusters);
+  // twice the largest mesh's share of the SMs, to the nearest power of two
+  p.cluster_blocks = 2;
+  while (p.cluster_blocks < kSegCluster &&
+         blocks2 * p.sizes_in_order[0] * 10ull > p.total_prims * (uint64_t)p.cluster_blocks * 14ull)
+    p.cluster_blocks *= 2;
 }
 
 unsigned mesh_blocks(uint32_t mesh_count) {
@@ -234,7 +249,8 @@ cudaError_t run_build(Plan& p, cudaStream_t s) {
   if ((e = cudaMemsetAsync(p.nodes.ptr, 0xff, (size_t)p.node_cap * sizeof(DAabb), s))) return e;
   if ((e = launch_locb_segments(p.aabbs.ptr, p.vals.ptr, p.vals.ptr, p.prim_off.ptr, p.order.ptr, p.worlds.ptr, M, N,
                                 p.lvl0.ptr, p.lvl1.ptr, p.nodes.ptr, p.nb.ptr, p.status.ptr, mesh_blocks(M),
-                                p.big_count, p.cluster_sums.ptr, p.clusters, s, p.side, p.fork, p.join)))
+                                p.big_count, p.cluster_sums.ptr, p.clusters, p.cluster_blocks, s, p.side, p.fork,
+                                p.join)))
     return e;
   // traversal trees for the closest hit only (LOCB trees are nested)
   const bool wide = !(p.flags & (RTBVH_TRACE_ANY_HIT | RTBVH_TRACE_EXACT_NODES));

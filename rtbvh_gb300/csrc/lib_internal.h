@@ -302,22 +302,21 @@ cudaError_t launch_trace_packets(const PacketArgs& a, bool mbvh, cudaStream_t s)
 
 // ------------------------------------------------------------------ many meshes
 // Per-mesh clustering of a concatenated forest (see locb.cu).
-// Meshes order[0, big_count) (the largest, more than kSegClusterMinPrims
-// primitives) are clustered by `clusters` thread-block clusters of
-// kSegCluster blocks; the rest by up to `blocks` single blocks, on `side`
-// (between the events fork and join) when it is given. cluster_sums:
-// kSegCluster words per cluster and a word per mesh. Eight blocks per
-// cluster: 16 are faster for a few large meshes (8 of up to 200k primitives
-// 1.73 against 2.07 ms, build and trace) and slower for many (512 of them 62.8
-// against 60.2 ms), 4 are slower for 64 (9.7 against 8.5 ms).
+// Meshes order[0, big_count) (the largest) are clustered by `clusters`
+// thread-block clusters of cluster_blocks (at most kSegCluster) blocks; the
+// rest by up to `blocks` single blocks, on `side` (between the events fork and
+// join) when it is given. cluster_sums: kSegCluster words per cluster and a
+// word per mesh. Clusters of 16: faster for a few large meshes (8 of up to
+// 200k primitives 1.73 against 2.07 ms, build and trace), slower for many (512
+// of them 62.8 against 60.2 ms).
 constexpr uint32_t kSegCluster = 8;
 constexpr uint32_t kSegClusterMinPrims = 4096;  // default threshold (RTBatchTuning::cluster_min_prims)
 cudaError_t launch_locb_segments(const DAabb* aabbs, const uint32_t* sorted, uint32_t* indices,
                                  const uint32_t* prim_off, const uint32_t* order, const DAabb* worlds,
                                  uint32_t mesh_count, uint32_t total_prims, DAabb* lvl0, DAabb* lvl1,
                                  DAabb* final_nodes, uint32_t* nb, uint32_t* status, unsigned blocks,
-                                 uint32_t big_count, uint32_t* cluster_sums, unsigned clusters, cudaStream_t s,
-                                 cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
+                                 uint32_t big_count, uint32_t* cluster_sums, unsigned clusters, unsigned cluster_blocks,
+                                 cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join);
 // MBVH collapse of a concatenated forest (see mbvh.cu): mesh m's quad nodes
 // at [mbase[m], mbase[m + 1]); with wnodes / wq also the traversal trees of
 // all meshes (LOCB: nested boxes), mesh m's root at qroot[m]. mnodes, wnodes

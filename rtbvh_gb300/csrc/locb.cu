@@ -1027,10 +1027,11 @@ cudaError_t launch_locb_segments(const DAabb* aabbs, const uint32_t* sorted, uin
                                  const uint32_t* prim_off, const uint32_t* order, const DAabb* worlds,
                                  uint32_t mesh_count, uint32_t total_prims, DAabb* lvl0, DAabb* lvl1,
                                  DAabb* final_nodes, uint32_t* nb, uint32_t* status, unsigned blocks,
-                                 uint32_t big_count, uint32_t* cluster_sums, unsigned clusters, cudaStream_t s,
-                                 cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+                                 uint32_t big_count, uint32_t* cluster_sums, unsigned clusters, unsigned cluster_blocks,
+                                 cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
   if (total_prims == 0 || mesh_count == 0) return cudaSuccess;
-  if (big_count > mesh_count || (big_count > 0 && (clusters == 0 || cluster_sums == nullptr)))
+  if (big_count > mesh_count || (big_count > 0 && (clusters == 0 || cluster_blocks == 0 ||
+                                                   cluster_blocks > kSegCluster || cluster_sums == nullptr)))
     return cudaErrorInvalidValue;
   cudaError_t e;
   k_locb_segment_leaves<<<(total_prims + kBlock - 1) / kBlock, kBlock, 0, s>>>(aabbs, sorted, prim_off, mesh_count,
@@ -1056,7 +1057,7 @@ cudaError_t launch_locb_segments(const DAabb* aabbs, const uint32_t* sorted, uin
     small_s = side;
   }
   if (big_count > 0 &&
-      (e = launch_cluster(k_locb_forest, clusters, kSegCluster, s, p, cluster_sums, 0u, big_count)))
+      (e = launch_cluster(k_locb_forest, clusters, cluster_blocks, s, p, cluster_sums, 0u, big_count)))
     return e;
   if (big_count < mesh_count) {
     const unsigned nb_small = std::min<unsigned>(blocks, mesh_count - big_count);
