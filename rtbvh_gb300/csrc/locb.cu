@@ -948,10 +948,12 @@ ResultCode build_locb(const DAabb* aabbs, const float4* centers, size_t n_, cuda
   cudaGetDevice(&dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_locb_levels, kBlock, 0);
   if (per_sm < 1) return fail(DeviceError);
-  // at most 3 blocks per SM: fewer blocks make the grid barriers between
-  // clustering levels cheaper (1.394 against 1.423 ms on 1M triangles at
-  // the occupancy limit; 1 block per SM is slower, 1.74 ms)
-  if (per_sm > 3) per_sm = 3;
+  // Up to a million primitives at most 3 blocks per SM: fewer blocks make the
+  // grid barriers between clustering levels cheaper; above, a level's work
+  // counts for more. 3 against 4 blocks (all that fit), us: 200k 812 / 822, 1M
+  // 1,414 / 1,414, 4M 3,860 / 3,767, 10M 10,921 / 10,481; 2 blocks: 812, 1,444,
+  // 4,116, 12,220.
+  if (per_sm > 3 && n <= 1000000u) per_sm = 3;
   unsigned grid = (unsigned)(sm_count() * per_sm);
   const unsigned useful = (unsigned)((n + kBlock - 1) / kBlock);
   if (grid > useful) grid = useful;

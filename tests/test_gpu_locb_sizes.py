@@ -56,3 +56,13 @@ def test_locb_sizes_in_a_batch(cluster_min):
         wi[~leaf, 7] += base
         got = ints[base:base + len(on)]
         assert np.array_equal(got.view(np.uint32), u32(want)), n
+
+
+@pytest.mark.parametrize("n", [1000000, 1000001])
+def test_locb_at_a_million(n):
+    """More blocks per SM above a million primitives."""
+    tris = _scene(n, "soup")
+    g = gpu_build(tris, "locb")
+    on, oi = oracle_build(tris, "locb")
+    assert np.array_equal(u32(g.nodes()), u32(on))
+    assert np.array_equal(g.indices(), oi)
