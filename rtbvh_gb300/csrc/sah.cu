@@ -51,7 +51,7 @@ constexpr int kChunk = 2048;
 constexpr int kLargeBlock = 256;
 constexpr uint32_t kWarpMax = 1024;  // largest subtree
 constexpr uint32_t kTaskWarp = 64;  // largest task of k_sah_build's lists that one warp does
-constexpr uint32_t kCoopMaxPrims = 1u << 20;      // larger builds launch the phases separately
+constexpr uint32_t kCoopMaxPrims = 1u << 21;      // larger builds launch the phases separately
 constexpr int kBinWords = 8;  // ordered min xyz, ordered max xyz, count, pad
 constexpr int kTaskBinWords = 3 * kBins * kBinWords;
 constexpr uint32_t kFlagAgg = 1u << 30;
@@ -1897,9 +1897,10 @@ ResultCode build_binned_sah(const DAabb* aabbs, const float4* centers, size_t n_
   // covers every SM, with one block each for small builds, whose time is the
   // barriers', and the full resident grid above (builds with both trees, one
   // block against two: 20k triangles 723 / 780 us, 100k 1,217 / 1,176, 400k
-  // 2,047 / 1,887). Large builds launch the phases separately, which lets each phase
-  // run at its own occupancy, and read the level's counts back between
-  // levels.
+  // 2,047 / 1,887). Large builds launch the phases separately, which lets each
+  // phase run at its own occupancy, and read the counts back every fourth
+  // level; cooperative against that, us: 1.2M 3,225 / 3,426, 1.6M 3,815 / 3,956,
+  // 2M 4,470 / 4,507, 3M 7,060 / 6,980, 4M 8,050 / 7,845.
   const bool coop = n <= kCoopMaxPrims;
   int per_sm = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, coop ? (const void*)k_sah_build

@@ -64,3 +64,12 @@ def test_sah_subtrees_in_two_launches(n, kind):
     nodes, idx = g.nodes(), g.indices()
     assert len(nodes) == len(on)
     assert canonical(nodes, idx) == canonical(on, oi)
+
+
+def test_sah_one_launch_above_a_million():
+    tris = _scene(1100003, "sphere")
+    g = gpu_build(tris, "sah")
+    on, oi = oracle_build(tris, "sah", 1)
+    nodes, idx = g.nodes(), g.indices()
+    assert len(nodes) == len(on)
+    assert canonical(nodes, idx) == canonical(on, oi)
