@@ -258,7 +258,7 @@ cudaError_t run_build(Plan& p, cudaStream_t s) {
                                   p.mnodes.ptr, wide ? p.wnodes.ptr : nullptr, wide ? p.qnodes.ptr : nullptr,
                                   p.qroot.ptr, p.status.ptr + 2, p.status.ptr, s)))
     return e;
-  if ((e = launch_gather_triangles(p.vertices, p.vals.ptr, N, p.tris.ptr, s))) return e;
+  if ((e = launch_gather_triangles(p.vertices, p.vals.ptr, N, p.tris.ptr, false, s))) return e;
   return cudaGetLastError();
 }
 

@@ -153,19 +153,44 @@ __global__ void __launch_bounds__(kPrepBlock)
 
 __global__ void __launch_bounds__(kPrepBlock)
     k_gather_triangles(const float* __restrict__ v, const uint32_t* __restrict__ idx, size_t n,
-                       float4* __restrict__ out) {
+                       float4* __restrict__ out, TriEdges* __restrict__ edges) {
   size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+  const bool valid = k < n;
+  if (!valid) k = n - 1;  // the last block's other threads
   uint32_t p = __ldg(idx + k);
   const float* t = v + 9 * (size_t)p;
   float x0 = __ldg(t), y0 = __ldg(t + 1), z0 = __ldg(t + 2);
   float x1 = __ldg(t + 3), y1 = __ldg(t + 4), z1 = __ldg(t + 5);
   float x2 = __ldg(t + 6), y2 = __ldg(t + 7), z2 = __ldg(t + 8);
-  float4* o = out + (size_t)kTriFloat4 * k;
-  o[0] = make_float4(x0, y0, z0, __uint_as_float(p));
-  o[1] = make_float4(x1 - x0, y1 - y0, z1 - z0, 0.0f);
-  o[2] = make_float4(x2 - x0, y2 - y0, z2 - z0, 0.0f);
-  o[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  const float4 e1 = make_float4(x1 - x0, y1 - y0, z1 - z0, 0.0f), e2 = make_float4(x2 - x0, y2 - y0, z2 - z0, 0.0f);
+  if (valid) {
+    float4* o = out + (size_t)kTriFloat4 * k;
+    o[0] = make_float4(x0, y0, z0, __uint_as_float(p));
+    o[1] = e1;
+    o[2] = e2;
+    o[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
+  if (!edges) return;
+  // one atomic per block (one per warp cost a refit of 200k triangles 17 us)
+  const float product = sqrtf(e1.x * e1.x + e1.y * e1.y + e1.z * e1.z) * sqrtf(e2.x * e2.x + e2.y * e2.y + e2.z * e2.z);
+  const bool large = !(product <= kLargeProduct);  // NaN too
+  __shared__ uint32_t s_most;
+  if (threadIdx.x == 0) s_most = 0;
+  __syncthreads();
+  const uint32_t bits = __reduce_max_sync(0xffffffffu, large ? 0u : __float_as_uint(product));
+  const uint32_t larges = __ballot_sync(0xffffffffu, valid && large), lane = threadIdx.x & 31u;
+  if (lane == 0) atomicMax(&s_most, bits);
+  __syncthreads();
+  uint32_t* const most = reinterpret_cast<uint32_t*>(&edges->product);
+  if (threadIdx.x == 0 && s_most > __ldcg(most)) atomicMax(most, s_most);
+  if (!larges) return;
+  uint32_t at = 0;
+  if (lane == 0) {
+    at = __ldcg(&edges->large);
+    if (at <= kLargeTriangles) at = atomicAdd(&edges->large, (uint32_t)__popc(larges));
+  }
+  at = __shfl_sync(0xffffffffu, at, 0) + __popc(larges & ((1u << lane) - 1u));
+  if (valid && large && at < kLargeTriangles) edges->slot[at] = (uint32_t)k;
 }
 
 // Boxes that one block folds alone.
@@ -213,9 +238,12 @@ cudaError_t launch_morton(const float4* centers, size_t n, const DAabb* world, u
 }
 
 cudaError_t launch_gather_triangles(const float* vertices, const uint32_t* indices, size_t n, float4* out,
-                                    cudaStream_t s) {
+                                    bool with_edges, cudaStream_t s) {
+  TriEdges* const edges = with_edges ? tri_edges(out, n) : nullptr;
+  cudaError_t e;
+  if (edges && (e = cudaMemsetAsync(edges, 0, sizeof(TriEdges), s))) return e;
   if (n == 0) return cudaSuccess;
-  k_gather_triangles<<<grid_for(n, kPrepBlock), kPrepBlock, 0, s>>>(vertices, indices, n, out);
+  k_gather_triangles<<<grid_for(n, kPrepBlock), kPrepBlock, 0, s>>>(vertices, indices, n, out, edges);
   return cudaGetLastError();
 }
 

@@ -40,9 +40,10 @@ struct Entry {
   DTBox* d_tboxes = nullptr;      // Mbvh with q_gates: subtree boxes of d_mnodes (from the triangles)
   uint32_t wcount = 0;
   bool quads_cover = false;       // Mbvh: every quad slot box contains its triangles grown by 1e-4
+  bool root_covers = false;       // Mbvh: so does the root's box
   bool q_gates = false;           // Mbvh: escaped triangles are flagged (collapse_entry)
   uint32_t* d_indices = nullptr;
-  float4* d_tris = nullptr;       // 3 per index slot
+  float4* d_tris = nullptr;       // tri_floats4(index slots): leaf-ordered triangles, then a TriEdges
   float* d_vertices = nullptr;    // prim-id order, 9 floats each
   uint32_t* d_status = nullptr;
   uint32_t source_bvh = UINT32_MAX;
@@ -61,6 +62,7 @@ struct Entry {
     wcount = 0;
     q_gates = false;
     quads_cover = false;
+    root_covers = false;
     d_indices = nullptr;
     d_tris = nullptr;
     d_vertices = nullptr;
@@ -122,6 +124,7 @@ ResultCode collapse_entry(Entry& m, cudaStream_t s, DMNode** mnodes, uint32_t* m
   m.wcount = 0;
   m.q_gates = false;
   m.quads_cover = false;
+  m.root_covers = false;
   if (m.bvh_node_count == 0) {  // Mbvh::default()
     *mnodes = nullptr;
     *mcount = 0;
@@ -157,6 +160,8 @@ ResultCode collapse_entry(Entry& m, cudaStream_t s, DMNode** mnodes, uint32_t* m
   m.wcount = out.wcount;
   m.d_tboxes = out.tboxes;
   m.quads_cover = tris && (from_triangles ? out.escaped == 0 : m.boxes_cover);
+  // a root leaf's one slot has the root's box
+  m.root_covers = m.quads_cover ? !out.bad_root : from_triangles && !out.bad_root && m.bvh_node_count > 1;
   m.q_gates = out.escaped != 0 && m.wcount != 0;
   if (!m.q_gates) {  // no ray is handed on for an escape: the subtree boxes would go unused
     pool_free(m.d_tboxes, s);
@@ -246,8 +251,8 @@ ResultCode store_bvh(const BuildOutput& out, uint32_t slots, size_t n, uint32_t 
   if (d_vertices) {
     if ((err = device_alloc(&e->d_vertices, 9 * n, s)) ||
         (err = cudaMemcpyAsync(e->d_vertices, d_vertices, 36 * n, cudaMemcpyDeviceToDevice, s)) ||
-        (err = device_alloc(&e->d_tris, (size_t)kTriFloat4 * slots, s)) ||
-        (err = launch_gather_triangles(e->d_vertices, e->d_indices, slots, e->d_tris, s))) {
+        (err = device_alloc(&e->d_tris, tri_floats4(slots), s)) ||
+        (err = launch_gather_triangles(e->d_vertices, e->d_indices, slots, e->d_tris, true, s))) {
       e->release();
       return cuda_rc(err);
     }
@@ -798,9 +803,8 @@ ResultCode rtbvh_gpu_create_mbvh(RTBvh bvh, uint32_t flags, rtbvh_stream_t strea
     return cuda_rc(err);
   }
   if (d_tris) {
-    if ((err = device_alloc(&e->d_tris, (size_t)kTriFloat4 * prim_count, s)) ||
-        (err = cudaMemcpyAsync(e->d_tris, d_tris, 16 * (size_t)kTriFloat4 * prim_count, cudaMemcpyDeviceToDevice,
-                               s)) ||
+    if ((err = device_alloc(&e->d_tris, tri_floats4(prim_count), s)) ||
+        (err = cudaMemcpyAsync(e->d_tris, d_tris, 16 * tri_floats4(prim_count), cudaMemcpyDeviceToDevice, s)) ||
         (err = device_alloc(&e->d_vertices, 9 * (size_t)vertex_count, s)) ||
         (err = cudaMemcpyAsync(e->d_vertices, d_vertices, 36 * (size_t)vertex_count, cudaMemcpyDeviceToDevice,
                                s))) {
@@ -847,9 +851,9 @@ ResultCode rtbvh_gpu_set_triangles(uint32_t structure_id, int is_mbvh, const flo
   e->vertex_count = (uint32_t)prim_count;
   e->vertex_lower_bound = false;
   if (!e->d_vertices && (err = device_alloc(&e->d_vertices, 9 * (size_t)prim_count, s))) return cuda_rc(err);
-  if (!e->d_tris && (err = device_alloc(&e->d_tris, (size_t)kTriFloat4 * e->prim_count, s))) return cuda_rc(err);
+  if (!e->d_tris && (err = device_alloc(&e->d_tris, tri_floats4(e->prim_count), s))) return cuda_rc(err);
   if ((err = cudaMemcpyAsync(e->d_vertices, vertices, 36 * (size_t)prim_count, cudaMemcpyDeviceToDevice, s)) ||
-      (err = launch_gather_triangles(e->d_vertices, e->d_indices, e->prim_count, e->d_tris, s)))
+      (err = launch_gather_triangles(e->d_vertices, e->d_indices, e->prim_count, e->d_tris, true, s)))
     return cuda_rc(err);
   // the boxes promise nothing about these triangles: an Mbvh's traversal
   // tree is rebuilt from them (gated where the boxes miss them)
@@ -889,6 +893,8 @@ static ResultCode trace_common(uint32_t id, bool mbvh, const float* rays, const 
       a.q_gates = e->q_gates;
       a.tboxes = e->q_gates ? e->d_tboxes : nullptr;
       a.quads_cover = e->quads_cover;
+      a.root_covers = e->root_covers;
+      a.edges = e->d_tris ? tri_edges(e->d_tris, e->prim_count) : nullptr;
     }
     if (walk_stats && (a.qnodes == nullptr || a.q_count == 0)) return InvalidArgument;
     a.nodes = e->d_nodes;
@@ -1156,9 +1162,9 @@ static ResultCode recollapse(Entry* m, const float* vertices, cudaStream_t s) {
   m->q_gates = false;
   if (vertices) {
     if (!m->d_vertices && (err = device_alloc(&m->d_vertices, 9 * n, s))) return cuda_rc(err);
-    if (!m->d_tris && (err = device_alloc(&m->d_tris, (size_t)kTriFloat4 * slots, s))) return cuda_rc(err);
+    if (!m->d_tris && (err = device_alloc(&m->d_tris, tri_floats4(slots), s))) return cuda_rc(err);
     if ((err = cudaMemcpyAsync(m->d_vertices, vertices, 36 * n, cudaMemcpyDeviceToDevice, s)) ||
-        (err = launch_gather_triangles(m->d_vertices, m->d_indices, slots, m->d_tris, s)))
+        (err = launch_gather_triangles(m->d_vertices, m->d_indices, slots, m->d_tris, true, s)))
       return cuda_rc(err);
   }
   // recollapse follows a refit: from triangles, every box now contains
@@ -1229,7 +1235,7 @@ ResultCode rtbvh_gpu_refit(uint32_t bvh_id, const float* vertices, const RTAabb*
     boxes = d_a.ptr;
     if (b->d_vertices) {
       if ((err = cudaMemcpyAsync(b->d_vertices, vertices, 36 * n, cudaMemcpyDeviceToDevice, s)) ||
-          (err = launch_gather_triangles(b->d_vertices, b->d_indices, b->prim_count, b->d_tris, s)))
+          (err = launch_gather_triangles(b->d_vertices, b->d_indices, b->prim_count, b->d_tris, true, s)))
         return cuda_rc(err);
     }
   }

@@ -477,9 +477,10 @@ __global__ void __launch_bounds__(kBlock) k_quads(CollapseParams p) {
 }
 
 // The root's place, and the number of quad nodes for the host. A root whose
-// count did not come up (no tree) is an error.
+// count did not come up (no tree) is an error. *bad_root: the root is interior
+// and its box misses triangles (kBadBox).
 __global__ void k_root_place(const uint64_t* cnt, const DAabb* nodes, uint2* known, uint32_t m_cap, uint32_t* m_total,
-                             uint32_t* walloc, uint32_t* status) {
+                             uint32_t* walloc, uint32_t* bad_root, uint32_t* status) {
   if (threadIdx.x == 0) {
     *walloc = 1u;  // traversal node 0 is the root's
     const uint64_t c = *cnt;
@@ -487,6 +488,7 @@ __global__ void k_root_place(const uint64_t* cnt, const DAabb* nodes, uint2* kno
     if (!counted(c) || t == 0u || t > m_cap) atomicOr(status, kStatusBadIndex);
     else *known = make_uint2(0u, kNone);
     *m_total = t;
+    *bad_root = (c & kBadBox) ? 1u : 0u;
   }
 }
 
@@ -1199,7 +1201,8 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
   Scratch<uint32_t> seen;
   ScratchPack scratch;
   // result words: 0 status, 1 check (not nested, duplicate leaf slots), 2
-  // primitives in leaves, 3 escaped triangles, 4 quad nodes, 5 traversal nodes
+  // primitives in leaves, 3 escaped triangles, 4 quad nodes, 5 traversal nodes,
+  // 6 the root's box misses triangles
   uint32_t *words, *res;
   scratch.add(&words, collapse_scratch_words(node_count));
   scratch.add(&res, 8);
@@ -1220,7 +1223,7 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
   const CollapseScratch w(words, node_count);
   if ((e = launch_counts(nodes, node_count, w, tri, res, s))) return drop(cuda_rc(e));
   const unsigned blocks = (node_count + kBlock - 1) / kBlock;
-  k_root_place<<<1, 32, 0, s>>>(w.cnt, nodes, w.known, m_cap, res + 4, res + 5, res);
+  k_root_place<<<1, 32, 0, s>>>(w.cnt, nodes, w.known, m_cap, res + 4, res + 5, res + 6, res);
   CollapseParams p = {};
   p.nodes = nodes;
   p.node_count = node_count;
@@ -1262,13 +1265,14 @@ ResultCode build_mbvh(const DAabb* nodes, uint32_t node_count, cudaStream_t s, c
     q.expect_seen = check_indices ? req.index_count : kNone;
     if ((e = launch_nodes(p, tri != nullptr, &q, s))) return drop(cuda_rc(e));
   }
-  uint32_t h[6];
-  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(h, res, 24, cudaMemcpyDeviceToHost, s)) ||
+  uint32_t h[7];
+  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(h, res, sizeof(h), cudaMemcpyDeviceToHost, s)) ||
       (e = cudaStreamSynchronize(s)))
     return drop(cuda_rc(e));
   if (h[0] != 0) return drop((h[0] & kStatusTimeout) ? Timeout : Error);
   out->mcount = h[4];
   out->escaped = h[3];
+  out->bad_root = h[6] != 0;
   if (req.wide && (h[1] || (check_indices && h[2] != req.index_count))) {
     // no traversal tree: closest hit reads the exact nodes
     pool_free(out->wnodes, s);

@@ -100,6 +100,20 @@ __device__ __forceinline__ bool mt_test(const float4* tri, RayState& r, float& h
   return false;
 }
 
+// Margins on the slab values of the three axes for walks that skip slots (see
+// kTestError), infinite where none may be skipped.
+struct SlabMargin {
+  float x, y, z;
+  __device__ __forceinline__ void set(const RayState& r, float distance) {
+    x = distance * fabsf(r.ix);
+    y = distance * fabsf(r.iy);
+    z = distance * fabsf(r.iz);
+  }
+  __device__ __forceinline__ void set_none() { x = y = z = __int_as_float(0x7f800000); }
+  // Whether a box with these exit values reaches the origin.
+  __device__ __forceinline__ bool reaches(float tx, float ty, float tz) const { return tx >= -x && ty >= -y && tz >= -z; }
+};
+
 // MbvhNode::intersect: mask bit i set when slot i is hit; ids packed as
 // 2-bit fields, ascending by t_min after the 5-compare network.
 //
@@ -110,11 +124,11 @@ __device__ __forceinline__ bool mt_test(const float4* tri, RayState& r, float& h
 // comparison can see. So the fast form takes every decision the exact form
 // takes. Rays with a zero or non-finite component use the exact form.
 //
-// BEHIND (FAST only): slots whose exit t is below exit_min are left out of
-// the mask (0: boxes wholly behind the origin; -inf: none).
+// BEHIND (FAST only): slots that lie behind the origin by the margin are left
+// out of the mask.
 template <bool FAST, bool BEHIND = false>
 __device__ __forceinline__ void quad_intersect(const DMNode* node, const RayState& r, uint32_t& mask, uint32_t& ids,
-                                               int4& children, int4& counts, float exit_min = 0.0f) {
+                                               int4& children, int4& counts, const SlabMargin& behind = {}) {
   const float* q = reinterpret_cast<const float*>(node);
   float vx[8], vy[8], vz[8], vc[8];
   ld8(q, vx);
@@ -138,9 +152,12 @@ __device__ __forceinline__ void quad_intersect(const DMNode* node, const RayStat
     const float ty0 = (a_mny[i] - r.oy) * r.iy, ty1 = (a_mxy[i] - r.oy) * r.iy;
     const float tz0 = (a_mnz[i] - r.oz) * r.iz, tz1 = (a_mxz[i] - r.oz) * r.iz;
     float tn, tx;
+    bool reaches = true;
     if (FAST) {
+      const float txx = fmaxf(tx0, tx1), tyx = fmaxf(ty0, ty1), tzx = fmaxf(tz0, tz1);
       tn = fmaxf(fminf(tx0, tx1), fmaxf(fminf(ty0, ty1), fminf(tz0, tz1)));
-      tx = fminf(fmaxf(tx0, tx1), fminf(fmaxf(ty0, ty1), fmaxf(tz0, tz1)));
+      tx = fminf(txx, fminf(tyx, tzx));
+      if (BEHIND) reaches = behind.reaches(txx, tyx, tzx);
     } else {
       const float txn = sse_min(tx0, tx1), txx = sse_max(tx0, tx1);
       const float tyn = sse_min(ty0, ty1), tyx = sse_max(ty0, ty1);
@@ -149,7 +166,7 @@ __device__ __forceinline__ void quad_intersect(const DMNode* node, const RayStat
       tx = sse_min(txx, sse_min(tyx, tzx));
     }
     tmin[i] = tn;
-    if ((tx >= tn) && (tn < r.t) && (!BEHIND || tx >= exit_min)) m |= 1u << i;
+    if ((tx >= tn) && (tn < r.t) && reaches) m |= 1u << i;
   }
   uint32_t i0 = 0, i1 = 1, i2 = 2, i3 = 3;
   float t0 = tmin[0], t1 = tmin[1], t2 = tmin[2], t3 = tmin[3], tt;
@@ -261,11 +278,26 @@ __device__ __forceinline__ uint32_t ray_mesh(const TraceArgs& a, uint32_t r) {
   return lo;
 }
 
+// Whether a ray with the bound t may have a hit in a box with these entry and
+// exit values of the axes.
+template <bool ANY_HIT>
+__device__ __forceinline__ bool enters(float nx, float ny, float nz, float fx, float fy, float fz, float t,
+                                       const SlabMargin& m) {
+  if (!ANY_HIT) {
+    const float tn = fmaxf(nx, fmaxf(ny, nz)), tx = fminf(fx, fminf(fy, fz));
+    return tx >= tn && tx >= 0.0f && tn < t;
+  }
+  const float tn = fmaxf(nx - m.x, fmaxf(ny - m.y, nz - m.z)), tx = fminf(fx + m.x, fminf(fy + m.y, fz + m.z));
+  return tx >= tn && tx >= 0.0f && tn < t;
+}
+
 // Hit mask of a quad node's subtree boxes (DTBox): slot i is set when the
 // ray can enter its box at some t in [0, r.t). Finite rays within the
 // compact walk's range only (the rounding argument of kCompactRange: a box
-// that holds a triangle hit at t > 1e-4 passes).
-__device__ __forceinline__ uint32_t subtree_mask(const DTBox* box, const RayState& r) {
+// that holds a triangle hit at t > 1e-4 passes), any hit with a margin
+// (kTestError).
+template <bool ANY_HIT>
+__device__ __forceinline__ uint32_t subtree_mask(const DTBox* box, const RayState& r, const SlabMargin& margin) {
   const float* q = reinterpret_cast<const float*>(box);
   float vx[8], vy[8], vz[8];
   ld8(q, vx);
@@ -277,9 +309,9 @@ __device__ __forceinline__ uint32_t subtree_mask(const DTBox* box, const RayStat
     const float tx0 = (vx[i] - r.ox) * r.ix, tx1 = (vx[4 + i] - r.ox) * r.ix;
     const float ty0 = (vy[i] - r.oy) * r.iy, ty1 = (vy[4 + i] - r.oy) * r.iy;
     const float tz0 = (vz[i] - r.oz) * r.iz, tz1 = (vz[4 + i] - r.oz) * r.iz;
-    const float tn = fmaxf(fminf(tx0, tx1), fmaxf(fminf(ty0, ty1), fminf(tz0, tz1)));
-    const float tx = fminf(fmaxf(tx0, tx1), fminf(fmaxf(ty0, ty1), fmaxf(tz0, tz1)));
-    if (tx >= tn && tx >= 0.0f && tn < r.t) m |= 1u << i;
+    if (enters<ANY_HIT>(fminf(tx0, tx1), fminf(ty0, ty1), fminf(tz0, tz1), fmaxf(tx0, tx1), fmaxf(ty0, ty1),
+                        fmaxf(tz0, tz1), r.t, margin))
+      m |= 1u << i;
   }
   return m;
 }
@@ -357,9 +389,64 @@ __device__ __forceinline__ int first_nearest(const FourLanes& q, float t, float 
 
 constexpr int kCullNone = 0, kCullSubtree = 1, kCullBehind = 2;  // see k_trace_mbvh
 
-// Whether slots may be skipped for this ray.
-template <int CULL>
-__device__ __forceinline__ bool cull_ray(const TraceArgs& a, const RayState& ray) {
+// How far the float triangle test may be off, for any-hit walks that skip
+// slots. In exact arithmetic, with s = o - v0 and an accepted (t, u, v),
+//   det (o + t d - v0 - u e1 - v e2) = dDet s + dT d - dU e1 - dV e2
+// where dDet .. dV are the rounding errors of the determinant and of the
+// numerators of t, u and v. The roundings of mt_test (2^-24 each) add up to at
+// most 5.9, 7.3, 6.9 and 7.3 times 2^-24 |e1| |e2| |d| |s| for the four terms,
+// and an accepted |det| is at least 1e-5: the point o + t d lies within
+//   0.17 |e1| |e2| |d| |s|  (27.4 * 2^-24 / 1e-5)
+// of the triangle, and 1.6e-6 |s| more for the roundings of t d and of the edges
+// themselves (no edge is longer than 2 |s| with s the farthest corner). A ray
+// nearly in a triangle's plane gets that far: t is noise there. Over the
+// each direction component that distance, less what the boxes' own growth
+// takes up, is a margin on the axis's slab values. |s| is at most the distance
+// of the root box's farthest corner, |e1| |e2| the largest of the tree's
+// triangles but for the few large ones of TriEdges. Those are tested with the
+// ray first: one that such a triangle accepts outside its own box skips nothing,
+// and scenes with more of them skip nothing at all.
+// 4.2M shadow rays over 1M clustered triangles, us: 3,790; 3,600 without the
+// margins (and with other hits on such rays); 4,300 with the largest margin of
+// the axes for all three, which needs one comparison instead of three, where
+// directions with a small component skip little; 4,610 with each slot's
+// squared diagonal for |e1| |e2|; 5,490 with each slot's farthest corner for |s|.
+constexpr float kTestError = 0.17f, kTestErrorRest = 1.6e-6f;
+constexpr float kBoxSlack = 5e-5f;  // of the 1e-4 that boxes are grown by, what the slab test's rounding leaves
+
+// Whether one of the large triangles accepts this ray outside its own box.
+__device__ __forceinline__ bool large_noise(const TraceArgs& a, uint32_t large, const RayState& ray,
+                                            const SlabMargin& margin) {
+#pragma unroll 1
+  for (uint32_t k = 0; k < large; ++k) {
+    const uint32_t slot = __ldg(a.edges->slot + k);
+    if (slot >= a.prim_count) return true;
+    const float4* tri = a.tris + kTriFloat4 * (size_t)slot;
+    RayState r = ray;
+    float u, v;
+    int32_t p;
+    if (!mt_test(tri, r, u, v, p)) continue;
+    // slab values of its box, which lies inside every box on the way to it
+    const float4 v0 = __ldg(tri), e1 = __ldg(tri + 1), e2 = __ldg(tri + 2);
+    float n[3], f[3];
+    auto slab = [&](int k, float x, float ax, float bx, float o, float i) {
+      const float t0 = (fminf(x, fminf(x + ax, x + bx)) - o) * i, t1 = (fmaxf(x, fmaxf(x + ax, x + bx)) - o) * i;
+      n[k] = fminf(t0, t1);
+      f[k] = fmaxf(t0, t1);
+    };
+    slab(0, v0.x, e1.x, e2.x, ray.ox, ray.ix);
+    slab(1, v0.y, e1.y, e2.y, ray.oy, ray.iy);
+    slab(2, v0.z, e1.z, e2.z, ray.oz, ray.iz);
+    if (!enters<true>(n[0], n[1], n[2], f[0], f[1], f[2], ray.t, margin)) return true;
+  }
+  return false;
+}
+
+// Whether slots may be skipped for this ray, and (any hit) the margin, infinite
+// where they may not.
+template <bool ANY_HIT, int CULL>
+__device__ __forceinline__ bool cull_ray(const TraceArgs& a, const RayState& ray, SlabMargin& margin) {
+  margin.set_none();
   const DAabb root = load_aabb(a.nodes);
   // |x| <= bound is false for NaN and infinities
   bool cull = fabsf(ray.ox) <= kCompactRange && fabsf(ray.oy) <= kCompactRange && fabsf(ray.oz) <= kCompactRange &&
@@ -374,8 +461,27 @@ __device__ __forceinline__ bool cull_ray(const TraceArgs& a, const RayState& ray
   } else {
     // the margin argument needs the boxes within the range too
     for (int k = 0; k < 3; ++k) cull = cull && root.min[k] >= -kCompactRange && root.max[k] <= kCompactRange;
+    // rays that enter the scene from outside have nothing behind them
+    const float tn = fmaxf(fminf((root.min[0] - ray.ox) * ray.ix, (root.max[0] - ray.ox) * ray.ix),
+                           fmaxf(fminf((root.min[1] - ray.oy) * ray.iy, (root.max[1] - ray.oy) * ray.iy),
+                                 fminf((root.min[2] - ray.oz) * ray.iz, (root.max[2] - ray.oz) * ray.iz)));
+    cull = cull && tn < 0.0f;
   }
-  return cull;
+  if (!ANY_HIT || !cull) return cull;
+  const uint32_t large = __ldg(&a.edges->large);
+  const float x = fmaxf(fabsf(ray.ox - root.min[0]), fabsf(ray.ox - root.max[0]));
+  const float y = fmaxf(fabsf(ray.oy - root.min[1]), fabsf(ray.oy - root.max[1]));
+  const float z = fmaxf(fabsf(ray.oz - root.min[2]), fabsf(ray.oz - root.max[2]));
+  const float far = sqrtf(x * x + y * y + z * z);
+  const float len = sqrtf(ray.dx * ray.dx + ray.dy * ray.dy + ray.dz * ray.dz);
+  const float off = far * (kTestError * __ldg(&a.edges->product) * len + kTestErrorRest);
+  if (!(off <= 1.0e18f) || large > kLargeTriangles) return false;
+  margin.set(ray, fmaxf(0.0f, off - kBoxSlack));
+  if (large && large_noise(a, large, ray, margin)) {
+    margin.set_none();
+    return false;
+  }
+  return true;
 }
 
 // Start of ray r's walk over the quad nodes: the root (of its mesh); false:
@@ -424,6 +530,8 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
   int32_t prim = -1, current = -1;  // the node whose slots are in `slot`
   int sp = -1;
   bool active = false, fast = true, cull = false;
+  SlabMargin margin;
+  margin.set_none();
   uint32_t r = 0;
   LaneQuad slot;
   auto fetch = [&]() {
@@ -440,7 +548,7 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
       i += 8u * (size_t)warps;
       ray = load_ray(a.rays, r, a.t_max);
       fast = finite_ray(ray);
-      if (CULL != kCullNone && a.node_count > 0) cull = cull_ray<CULL>(a, ray);
+      if (CULL != kCullNone && a.node_count > 0) cull = cull_ray<ANY_HIT, CULL>(a, ray, margin);
       hu = hv = 0.0f;
       prim = -1;
       sp = -1;
@@ -463,23 +571,24 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
       child = slot.child;
       count = slot.count;
       float tx;
+      bool reaches = true;
       if (fast) {
+        const float txx = fmaxf(tx0, tx1), tyx = fmaxf(ty0, ty1), tzx = fmaxf(tz0, tz1);
         t = fmaxf(fminf(tx0, tx1), fmaxf(fminf(ty0, ty1), fminf(tz0, tz1)));
-        tx = fminf(fmaxf(tx0, tx1), fminf(fmaxf(ty0, ty1), fmaxf(tz0, tz1)));
+        tx = fminf(txx, fminf(tyx, tzx));
+        if (CULL == kCullBehind) reaches = margin.reaches(txx, tyx, tzx);
       } else {
         t = sse_max(sse_min(tx0, tx1), sse_max(sse_min(ty0, ty1), sse_min(tz0, tz1)));
         tx = sse_min(sse_max(tx0, tx1), sse_min(sse_max(ty0, ty1), sse_max(tz0, tz1)));
       }
-      hit = (tx >= t) && (t < ray.t);
-      if (CULL == kCullBehind && cull) hit = hit && tx >= 0.0f;
+      hit = (tx >= t) && (t < ray.t) && reaches;
       if (CULL == kCullSubtree && cull && hit) {
         const float* b = reinterpret_cast<const float*>(a.tboxes + current) + q.l;
         const float bx0 = (__ldg(b) - ray.ox) * ray.ix, bx1 = (__ldg(b + 4) - ray.ox) * ray.ix;
         const float by0 = (__ldg(b + 8) - ray.oy) * ray.iy, by1 = (__ldg(b + 12) - ray.oy) * ray.iy;
         const float bz0 = (__ldg(b + 16) - ray.oz) * ray.iz, bz1 = (__ldg(b + 20) - ray.oz) * ray.iz;
-        const float bn = fmaxf(fminf(bx0, bx1), fmaxf(fminf(by0, by1), fminf(bz0, bz1)));
-        const float bf = fminf(fmaxf(bx0, bx1), fminf(fmaxf(by0, by1), fmaxf(bz0, bz1)));
-        hit = bf >= bn && bf >= 0.0f && bn < ray.t;
+        hit = enters<ANY_HIT>(fminf(bx0, bx1), fminf(by0, by1), fminf(bz0, bz1), fmaxf(bx0, bx1), fmaxf(by0, by1),
+                              fmaxf(bz0, bz1), ray.t, margin);
       }
     }
     const uint32_t hits = q.ballot(hit);
@@ -596,23 +705,31 @@ __global__ void __launch_bounds__(kBlock) k_trace_mbvh4(TraceArgs a, uint32_t wa
 //  kCullSubtree (binned-SAH trees with a.tboxes): slots whose subtree box
 //   (from the triangles) the ray cannot enter below its current t.
 //  kCullBehind (any hit over a tree whose slot boxes contain their triangles
-//   with the 1e-4 margin, a.quads_cover): slots wholly behind the origin, by
-//   the exit t the slab test has anyway. What bounds such a walk is the
+//   grown by 1e-4, a.quads_cover): slots behind the origin, by the exit
+//   values the slab test has anyway. What bounds such a walk is the
 //   number of boxes visited: the slab test has no lower bound on t, so a
 //   shadow ray that leaves a surface walks the whole scene behind it too.
-//   4.2M shadow rays over 1M clustered triangles: 10.74 ms without the skip,
-//   3.80 ms with it.
+//   4.2M shadow rays over 1M clustered triangles: 9,155 us without the skip,
+//   3,790 with it. Rays that enter the scene from outside have nothing
+//   behind them: warps with only such rays leave the comparisons out (1M
+//   rays into a 200k soup, us: 2,230 with them, 2,165 without; 2,100 without
+//   any of this).
+//  Any hit leaves both a margin for the rounding of the triangle test
+//   (kTestError), so that the hit is the reference's on grazing rays too.
+//   Closest hit leaves none, like the compact walk: a hit that the triangle
+//   test reports by rounding, outside the triangle's boxes, can be missed there.
 // FEW: a launch whose ray count is read from the device walks with four lanes
 // per ray when that is at most kFewDeferred. The launch bounds keep that
 // branch from taking registers from the other one: 8 blocks per SM, 7 with
 // subtree boxes (8 spill there). Without them 68 and 78 registers, and launches
 // handed on whole were 5 to 10 % slower (1M rays, 1M clustered triangles:
 // 6,190 us for 5,770; 200k sphere, SAH: 4,260 for 3,880).
-// Any hit, leaves in one loop and at least 7 blocks per SM asked for (64
-// registers either way, but another allocation; 9 spill: 5,080 us): those
-// shadow rays 3,817 -> 3,596 us, over the binned-SAH tree 4,358 -> 4,076.
+// Any hit, leaves in one loop and 8 blocks per SM asked for (64 registers; 7
+// take 72 and 4,040 us, 9 spill: 5,080 without the margins): those shadow rays
+// 3,790 us, over the binned-SAH tree 4,240 (9,145 without the skip).
 template <bool ANY_HIT, bool STATS, int CULL = kCullNone, bool FEW = false>
-__global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 7 : FEW ? (CULL ? 7 : 8) : 0) k_trace_mbvh(TraceArgs a, unsigned int* work) {
+__global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 8 : FEW ? (CULL ? 7 : 8) : 0)
+    k_trace_mbvh(TraceArgs a, unsigned int* work) {
   RayState ray;
   float hu = 0.0f, hv = 0.0f;
   int32_t prim = -1;
@@ -626,6 +743,9 @@ __global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 7 : FEW ? (CULL 
   int32_t next = -1;
   uint32_t r = 0;
   bool active = false, fast = true, cull = false;
+  bool culls = false;  // warp-uniform: some ray of the warp skips slots
+  SlabMargin margin;
+  margin.set_none();
   WarpPool pool;
   uint32_t batch = a.ray_batch ? a.ray_batch : kPoolBatch;
   const uint32_t ray_count = a.ray_count_dev ? *a.ray_count_dev : (uint32_t)a.ray_count;
@@ -647,7 +767,7 @@ __global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 7 : FEW ? (CULL 
     r = a.order ? __ldg(a.order + rr) : rr;
     ray = load_ray(a.rays, r, a.t_max);
     fast = finite_ray(ray);
-    if (CULL != kCullNone && a.node_count > 0) cull = cull_ray<CULL>(a, ray);
+    if (CULL != kCullNone && a.node_count > 0) cull = cull_ray<ANY_HIT, CULL>(a, ray, margin);
     hu = hv = 0.0f;
     prim = -1;
     visits = tests = max_depth = 0;
@@ -679,7 +799,10 @@ __global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 7 : FEW ? (CULL 
     }
   };
   for (;;) {
-    if (!pool.exhausted) pool.refill<ANY_HIT ? 4 : 2>(active, batch, ray_count, work, start_ray);
+    if (!pool.exhausted) {
+      pool.refill<ANY_HIT ? 4 : 2>(active, batch, ray_count, work, start_ray);
+      if (CULL == kCullBehind) culls = __any_sync(0xffffffffu, active && cull);
+    }
     if (!__any_sync(0xffffffffu, active)) {
       if (pool.exhausted) break;
       continue;
@@ -696,11 +819,11 @@ __global__ void __launch_bounds__(kBlock, (ANY_HIT && !STATS) ? 7 : FEW ? (CULL 
     uint32_t mask, ids;
     int4 children, counts;
     bool done = false;
-    if (fast)
-      quad_intersect<true, CULL == kCullBehind>(a.mnodes + current, ray, mask, ids, children, counts,
-                                                cull ? 0.0f : -__int_as_float(0x7f800000));
+    if (CULL == kCullBehind && fast && culls)
+      quad_intersect<true, true>(a.mnodes + current, ray, mask, ids, children, counts, margin);
+    else if (fast) quad_intersect<true>(a.mnodes + current, ray, mask, ids, children, counts);
     else quad_intersect<false>(a.mnodes + current, ray, mask, ids, children, counts);
-    if (CULL == kCullSubtree && cull) mask &= subtree_mask(a.tboxes + current, ray);
+    if (CULL == kCullSubtree && cull) mask &= subtree_mask<ANY_HIT>(a.tboxes + current, ray, margin);
     if (STATS) ++visits;
     if (ANY_HIT && !STATS && mask == 0u) {
       // nothing to do: most visits of rays that miss (16.8M rays ending short
@@ -1734,12 +1857,14 @@ cudaError_t launch_any(const TraceArgs& a0, cudaStream_t s) {
   }
   const bool st = a.stats != nullptr;
   if (a.any_hit && MBVH && !st) {
+    const bool behind = a.root_covers && a.edges && a.quads_cover;
+    const bool subtree = a.root_covers && a.edges && !behind && a.tboxes;
     if (few) {
-      e = a.quads_cover ? launch_few<true, kCullBehind>(a, s)
-                        : (a.tboxes ? launch_few<true, kCullSubtree>(a, s) : launch_few<true, kCullNone>(a, s));
+      e = behind ? launch_few<true, kCullBehind>(a, s)
+                 : (subtree ? launch_few<true, kCullSubtree>(a, s) : launch_few<true, kCullNone>(a, s));
     } else {
-      auto kern = a.quads_cover ? k_trace_mbvh<true, false, kCullBehind>
-                                : (a.tboxes ? k_trace_mbvh<true, false, kCullSubtree> : k_trace_mbvh<true, false>);
+      auto kern = behind ? k_trace_mbvh<true, false, kCullBehind>
+                         : (subtree ? k_trace_mbvh<true, false, kCullSubtree> : k_trace_mbvh<true, false>);
       kern<<<persistent_grid(kern, a), kBlock, 0, s>>>(a, work.ptr);
       e = cudaGetLastError();
     }
