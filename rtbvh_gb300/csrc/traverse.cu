@@ -612,18 +612,22 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
     child = q.from(child, id);
     count = q.from(count, id);
     hit = (hits >> id) & 1u;
-    const bool inner = hit && count <= -1 && child > -1, leaf = hit && count > -1;
+    const bool inner = hit && count <= -1 && child > -1;
+    bool leaf = hit && count > -1;
     const uint32_t inners = q.ballot(inner);
     const int n = __popc(inners);
     const int32_t nearest = q.from(child, inners ? (uint32_t)__ffs(inners) - 1u : 0u);
-    bool done = false, push = false;
+    bool done = false, push = false, overflow = false;
     int32_t next = -1;
     if (n > 0) {
       next = nearest;
       if (sp + n - 1 >= kStack) {
-        if (q.l == 0u) atomicOr(a.status, kStatusStackOverflow);
-        prim = -2;
-        done = true;
+        // the walk ends at the slot whose push does not fit: the first interior
+        // one needs none, then kStack - 1 - sp fit
+        uint32_t rest = inners;
+        for (int fit = kStack - sp; fit > 0; --fit) rest &= ~(0x80000000u >> __clz(rest));
+        leaf = leaf && q.l > 31u - (uint32_t)__clz(rest);
+        done = overflow = true;
       } else {
         push = true;
       }
@@ -663,7 +667,10 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
         }
       }
       const uint32_t founds = q.ballot(found);
-      if (q.ballot(bad)) done = true;
+      if (q.ballot(bad)) {
+        done = true;
+        overflow = false;
+      }
       float best, before;
       int w = first_nearest<true>(q, ray.t, entry, best, before);
       if (ANY_HIT) w = founds ? 31 - __clz(founds) : -1;  // the first leaf in the walk's order
@@ -671,13 +678,20 @@ __device__ void walk_mbvh4(const TraceArgs& a, uint32_t ray_count, uint32_t warp
       const float wt = q.from(ray.t, src), wu = q.from(u, src), wv = q.from(v, src);
       const int32_t wp = q.from(p, src);
       ray.t = entry;
-      if (w >= 0 && prim != -2) {
+      if (w >= 0) {
         ray.t = wt;
         hu = wu;
         hv = wv;
         prim = wp;
-        if (ANY_HIT) done = true;
+        if (ANY_HIT) {
+          done = true;
+          overflow = false;
+        }
       }
+    }
+    if (overflow) {
+      if (q.l == 0u) atomicOr(a.status, kStatusStackOverflow);
+      prim = -2;
     }
     if (active && (done || current < 0)) {
       if (q.l == 0u) a.hits[r] = make_float4(ray.t, hu, hv, __int_as_float(prim));
