@@ -1644,6 +1644,7 @@ __global__ void __launch_bounds__(kLargeBlock) k_ph_emit(SahParams p, uint32_t l
 __global__ void __launch_bounds__(kLargeBlock) k_ph_advance(SahParams p, uint32_t level, uint32_t blocks) {
   SahShared& sh = dyn_shared();
   const Level lv = read_level(p, level);
+  __syncthreads();  // thread 0 overwrites below what every warp has to read here
   if (lv.L == 0) return;
   if (lv.L <= kFewTasks) {
     if (threadIdx.x == 0) {
