@@ -30,3 +30,10 @@ def test_levels_of_few_and_of_many_tasks():
     the grid; here levels of 512, 1,013, 1,652, 942 and 127 tasks follow one
     another, so the form changes both ways."""
     _check(3300001, "soup")
+
+
+@pytest.mark.parametrize("n,kind", [(2097152, "soup"), (2097153, "soup"), (2200003, "equal"), (2200001, "sphere")])
+def test_both_sides_of_the_cooperative_size(n, kind):
+    """The last size of one launch and the first of separate phases, and equal
+    and clustered primitives above it."""
+    _check(n, kind)
