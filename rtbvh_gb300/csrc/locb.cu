@@ -24,9 +24,9 @@
 // output is bit-identical to the reference's node array.
 #include <algorithm>
 #include <cstdio>
-#include <mutex>
 
 #include "lib_internal.h"
+#include "per_device.h"
 
 namespace rtbvh {
 
@@ -897,15 +897,23 @@ cudaError_t launch_cluster(K kern, unsigned clusters, unsigned blocks, cudaStrea
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
-// Blocks of the largest cluster the device can hold (16 where it is allowed,
-// else the portable 8); sets the kernels' attributes on first use.
-unsigned cluster_size() {
-  static std::once_flag once;
-  static unsigned size = 8;
-  std::call_once(once, [] {
+// Blocks of the largest cluster the current device can hold (16 where it is
+// allowed, else the portable 8); sets the kernels' attributes on its first use.
+cudaError_t cluster_size(unsigned* blocks) {
+  static PerDevice<unsigned> sizes;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e) return e;
+  return sizes.get(dev, blocks, [](unsigned* size) {
     for (auto k : {reinterpret_cast<const void*>(k_locb_cluster), reinterpret_cast<const void*>(k_locb_forest)}) {
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterShared));
-      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      cudaError_t err =
+          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ClusterShared));
+      if (err) return err;
+    }
+    *size = 8;
+    if (cudaFuncSetAttribute(k_locb_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      return cudaSuccess;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kClusterMax);
@@ -918,10 +926,10 @@ unsigned cluster_size() {
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_locb_cluster, &cfg) == cudaSuccess && n > 0) size = kClusterMax;
+    if (cudaOccupancyMaxActiveClusters(&n, k_locb_cluster, &cfg) == cudaSuccess && n > 0) *size = kClusterMax;
     else cudaGetLastError();
+    return cudaSuccess;
   });
-  return size;
 }
 
 }  // namespace
@@ -1000,7 +1008,8 @@ ResultCode build_locb(const DAabb* aabbs, const float4* centers, size_t n_, cuda
   p.status = status;
   p.info = status + 4;
   p.n = n;
-  const unsigned blocks = cluster_size();
+  unsigned blocks = 0;
+  if ((e = cluster_size(&blocks))) return fail(cuda_rc(e));
   p.stop = blocks * kClusterCap;
   const bool wide = n > p.stop;  // larger levels in the cooperative launch
   if (wide) {
@@ -1051,7 +1060,8 @@ cudaError_t launch_locb_segments(const DAabb* aabbs, const uint32_t* sorted, uin
   p.mesh_count = mesh_count;
   // small meshes (one block each) on the side stream, concurrently with the
   // clusters of the large ones; the two sets of meshes share no memory
-  cluster_size();  // sets the kernel's attributes
+  unsigned largest = 0;
+  if ((e = cluster_size(&largest))) return e;  // sets the kernel's attributes
   const bool fork_side = side != nullptr && big_count > 0 && big_count < mesh_count;
   cudaStream_t small_s = s;
   if (fork_side) {
