@@ -201,27 +201,30 @@ constexpr uint32_t kMaxClusters = 8192;
 
 // Meshes above `min_prims` primitives (a prefix of the size-ordered mesh
 // list) are clustered by block clusters; meshes of at most 2 primitives
-// always take the single-block path. At the default threshold only meshes with
-// more than 1.4 halves of an SM's share of all primitives are: a block keeps an
-// SM to itself, and a level in a cluster of 8 takes more than an eighth of its
-// time in one block, so many meshes are better off with a block or two each.
-// Clustering of meshes of one size, us, with 1 / 2 / 4 / 8 blocks: 700 of 5,000
-// triangles 3,067 / 3,231 / 3,766 / 6,195; 200 of 20,000 4,555 / 3,890 / 3,996
-// / 4,734; 64 of 20,000 2,081 / 1,420 / 1,468 / 1,778; 100 of 50,000 6,338 /
-// 6,166 / 5,213 / 5,986; 8 of 150,000 13,320 / 7,077 / 3,920 / 2,358.
+// always take the single-block path.
 void set_cluster_min(Plan& p, uint32_t min_prims) {
   p.cluster_min = min_prims < 2u ? 2u : min_prims;
   const uint64_t blocks2 = 2ull * (uint64_t)sm_count();
-  uint64_t above = p.cluster_min;
-  if (p.cluster_min == kSegClusterMinPrims) above = std::max<uint64_t>(above, p.total_prims * 10ull / (blocks2 * 7ull));
   p.big_count = 0;
-  while (p.big_count < p.mesh_count && p.sizes_in_order[p.big_count] > above) ++p.big_count;
+  while (p.big_count < p.mesh_count && p.sizes_in_order[p.big_count] > p.cluster_min) ++p.big_count;
   p.clusters = std::min<uint32_t>(p.big_count, kMaxClusters);
   // twice the largest mesh's share of the SMs, to the nearest power of two
   p.cluster_blocks = 2;
   while (p.cluster_blocks < kSegCluster &&
          blocks2 * p.sizes_in_order[0] * 10ull > p.total_prims * (uint64_t)p.cluster_blocks * 14ull)
     p.cluster_blocks *= 2;
+}
+
+// The default threshold: kSegClusterMinPrims, and in batches of many meshes
+// 1.4 halves of an SM's share of all primitives. A block keeps an SM to itself,
+// and a level in a cluster of 8 takes more than an eighth of its
+// time in one block, so many meshes are better off with a block or two each.
+// Clustering of meshes of one size, us, with 1 / 2 / 4 / 8 blocks: 700 of 5,000
+// triangles 3,067 / 3,231 / 3,766 / 6,195; 200 of 20,000 4,555 / 3,890 / 3,996
+// / 4,734; 64 of 20,000 2,081 / 1,420 / 1,468 / 1,778; 100 of 50,000 6,338 /
+// 6,166 / 5,213 / 5,986; 8 of 150,000 13,320 / 7,077 / 3,920 / 2,358.
+uint32_t default_cluster_min(const Plan& p) {
+  return (uint32_t)std::max<uint64_t>(kSegClusterMinPrims, p.total_prims * 10ull / (14ull * (uint64_t)sm_count()));
 }
 
 unsigned mesh_blocks(uint32_t mesh_count) {
@@ -393,7 +396,7 @@ ResultCode rtbvh_gpu_batch_create(const float* vertices, const uint32_t* prim_of
   p->sort_bytes = radix_sort_temp_bytes(N);
   p->sizes_in_order.resize(mesh_count);
   for (uint32_t q = 0; q < mesh_count; ++q) p->sizes_in_order[q] = prim_offsets[order[q] + 1] - prim_offsets[order[q]];
-  set_cluster_min(*p, kSegClusterMinPrims);
+  set_cluster_min(*p, default_cluster_min(*p));
   cudaError_t e;
   if ((e = p->cluster_sums.alloc((size_t)kSegCluster * std::min<uint32_t>(mesh_count, kMaxClusters) + mesh_count)) ||
       (e = cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking)) ||
@@ -485,7 +488,7 @@ ResultCode rtbvh_gpu_batch_set_tuning(RTBatch batch, const RTBatchTuning* t, rtb
   p->trace_blocks_per_sm = t->trace_blocks_per_sm;
   p->trace_ray_batch = t->trace_ray_batch;
   p->trace_stack = t->trace_stack;
-  set_cluster_min(*p, t->cluster_min_prims ? t->cluster_min_prims : kSegClusterMinPrims);
+  set_cluster_min(*p, t->cluster_min_prims ? t->cluster_min_prims : default_cluster_min(*p));
   return cuda_rc(capture(*p));
 }
 
@@ -496,10 +499,11 @@ ResultCode rtbvh_gpu_batch_tune(RTBatch batch, rtbvh_stream_t stream, RTBatchTun
   cudaError_t e;
   if ((e = cudaStreamSynchronize(s))) return cuda_rc(e);
   // 1. clustering threshold, timed on the build alone
-  static const uint32_t kClusterMin[] = {2048u, 4096u, 8192u, 16384u, 65536u};
+  const uint32_t kClusterMin[] = {default_cluster_min(*p), 2048u, 4096u, 8192u, 16384u, 65536u};
   uint32_t best_c = p->cluster_min;
   float best = 3.4e38f;
-  for (uint32_t c : kClusterMin) {
+  for (const uint32_t& c : kClusterMin) {
+    if (&c != kClusterMin && c == kClusterMin[0]) continue;
     set_cluster_min(*p, c);
     float ms;
     if ((e = time_ms([&] { return run_build(*p, s); }, s, 2, &ms))) return cuda_rc(e);
