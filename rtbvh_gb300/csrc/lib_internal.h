@@ -335,7 +335,7 @@ cudaError_t launch_trace_packets(const PacketArgs& a, bool mbvh, cudaStream_t s)
 // 200k primitives 1.73 against 2.07 ms, build and trace), slower for many (512
 // of them 62.8 against 60.2 ms).
 constexpr uint32_t kSegCluster = 8;
-constexpr uint32_t kSegClusterMinPrims = 4096;  // default threshold (RTBatchTuning::cluster_min_prims)
+constexpr uint32_t kSegClusterMinPrims = 4096;  // least default of RTBatchTuning::cluster_min_prims
 cudaError_t launch_locb_segments(const DAabb* aabbs, const uint32_t* sorted, uint32_t* indices,
                                  const uint32_t* prim_off, const uint32_t* order, const DAabb* worlds,
                                  uint32_t mesh_count, uint32_t total_prims, DAabb* lvl0, DAabb* lvl1,

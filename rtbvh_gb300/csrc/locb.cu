@@ -18,7 +18,8 @@
 // (k_locb_levels); from there on one thread-block cluster keeps the whole
 // level in its blocks' shared memory (cluster_levels): halos are read from and
 // parents written to the neighbours' shared memory, and the barriers are the
-// cluster's. The last 128 nodes are one block's.
+// cluster's. Levels of at most 256 nodes (kClusterAlone) are one block's, of at
+// most 32 one warp's (warp_levels).
 // Many meshes: the same two forms with a cluster per mesh (k_locb_forest).
 // Node positions follow the reference exactly (locb.rs:178-215), so the
 // output is bit-identical to the reference's node array.

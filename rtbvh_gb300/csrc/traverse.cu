@@ -25,7 +25,10 @@
 // quad nodes (DQNode, two 256-bit loads) when they exist: the boxes contain
 // the exact ones, so the nearest triangle and its t/u/v are unchanged, and
 // only the winner among triangles hit at exactly the same t can differ from
-// the reference's visit order. This halves the node bytes and the L1 fill
+// the reference's visit order. (All of this for hits that lie in their
+// triangles' boxes: nearly in a triangle's plane the test's t can be noise, see
+// kTestError, and which such hits a walk finds depends on its boxes and order.)
+// This halves the node bytes and the L1 fill
 // traffic. Any hit, statistics and rays with a zero, non-finite or huge
 // component use the exact nodes.
 #include <cstdlib>
@@ -185,7 +188,9 @@ __device__ __forceinline__ void quad_intersect(const DMNode* node, const RayStat
 // 128 and the smallest normal binade above, the same line q * 2^-133. One
 // instruction, where an offset in the mantissa needed a subtraction as well.
 // The factor goes into the step (kStepBias), so that the slab products come
-// out times kKeyScale, a power of two: nothing rounds differently. The walk is
+// out times kKeyScale, a power of two, and round as before down to keys of
+// 2^-54; nearer the origin they are denormal and lose bits, which can reorder
+// visits at such distances (the boxes' margin is 1e-4). The walk is
 // bound by its issue rate; 24 subtractions fewer of about 250 instructions per
 // node, with counts decoded only for tested leaves and the pushes counted at
 // once: 16.8M incoherent rays over 1M triangles 16.07 -> 14.13 ms, 4.2M camera
@@ -962,8 +967,9 @@ __device__ __forceinline__ void sort_slots(float (&key)[4], int32_t (&ch)[4]) {
 // t > 1e-4 (the triangle test's lower bound) lies inside its boxes with that
 // margin, and the box's computed exit t stays above 0 (the slab rounding is
 // below the margin, see kCompactRange). The cull removes no box that holds
-// a hit; it saves the walks of rays that start inside the scene (secondary
-// rays) through the boxes behind them.
+// such a hit (one that the test reports by rounding, outside its triangle's
+// box, can go with it, see kTestError); it saves the walks of rays that start
+// inside the scene (secondary rays) through the boxes behind them.
 __device__ __forceinline__ void slot_key(float tn, float tx, float t, int32_t child, bool inner, int i, float& key,
                                          uint32_t& leaves) {
   const bool hit = tx >= tn && tx >= 0.0f && tn < t && child >= 0;
